@@ -33,8 +33,10 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -93,7 +95,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -134,7 +136,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_0 = 0;
           float o34_0 = 0;
           float o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -172,7 +174,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g0_32 = 0;
             float g0_33 = 0;
             float g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -1470,7 +1472,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_1 = 0;
           float o34_1 = 0;
           float o35_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g1_0 = 0;
@@ -1508,7 +1510,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g1_32 = 0;
             float g1_33 = 0;
             float g1_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -2892,7 +2894,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_2 = 0;
           float o34_2 = 0;
           float o35_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g2_0 = 0;
@@ -2930,7 +2932,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g2_32 = 0;
             float g2_33 = 0;
             float g2_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -4304,7 +4306,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_3 = 0;
           float o34_3 = 0;
           float o35_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g3_0 = 0;
@@ -4342,7 +4344,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g3_32 = 0;
             float g3_33 = 0;
             float g3_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -5712,7 +5714,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_4 = 0;
           float o34_4 = 0;
           float o35_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g4_0 = 0;
@@ -5750,7 +5752,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g4_32 = 0;
             float g4_33 = 0;
             float g4_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -7134,7 +7136,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_5 = 0;
           float o34_5 = 0;
           float o35_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g5_0 = 0;
@@ -7172,7 +7174,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g5_32 = 0;
             float g5_33 = 0;
             float g5_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -8658,7 +8660,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_6 = 0;
           float o34_6 = 0;
           float o35_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g6_0 = 0;
@@ -8696,7 +8698,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g6_32 = 0;
             float g6_33 = 0;
             float g6_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -10213,7 +10215,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_7 = 0;
           float o34_7 = 0;
           float o35_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g7_0 = 0;
@@ -10251,7 +10253,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g7_32 = 0;
             float g7_33 = 0;
             float g7_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -11764,7 +11766,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_8 = 0;
           float o34_8 = 0;
           float o35_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g8_0 = 0;
@@ -11802,7 +11804,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g8_32 = 0;
             float g8_33 = 0;
             float g8_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -13176,7 +13178,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_9 = 0;
           float o34_9 = 0;
           float o35_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g9_0 = 0;
@@ -13214,7 +13216,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g9_32 = 0;
             float g9_33 = 0;
             float g9_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -14731,7 +14733,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_10 = 0;
           float o34_10 = 0;
           float o35_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g10_0 = 0;
@@ -14769,7 +14771,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g10_32 = 0;
             float g10_33 = 0;
             float g10_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -16225,7 +16227,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_11 = 0;
           float o34_11 = 0;
           float o35_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g11_0 = 0;
@@ -16263,7 +16265,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g11_32 = 0;
             float g11_33 = 0;
             float g11_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -17762,7 +17764,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_12 = 0;
           float o34_12 = 0;
           float o35_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g12_0 = 0;
@@ -17800,7 +17802,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g12_32 = 0;
             float g12_33 = 0;
             float g12_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -19170,7 +19172,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_13 = 0;
           float o34_13 = 0;
           float o35_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g13_0 = 0;
@@ -19208,7 +19210,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g13_32 = 0;
             float g13_33 = 0;
             float g13_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -20721,7 +20723,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_14 = 0;
           float o34_14 = 0;
           float o35_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g14_0 = 0;
@@ -20759,7 +20761,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g14_32 = 0;
             float g14_33 = 0;
             float g14_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -22258,7 +22260,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_15 = 0;
           float o34_15 = 0;
           float o35_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g15_0 = 0;
@@ -22296,7 +22298,7 @@ jk_DD_LL_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g15_32 = 0;
             float g15_33 = 0;
             float g15_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;

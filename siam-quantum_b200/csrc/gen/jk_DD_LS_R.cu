@@ -32,8 +32,10 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -97,7 +99,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -138,7 +140,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_0 = 0;
           double o34_0 = 0;
           double o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -176,7 +178,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_32 = 0;
             double g0_33 = 0;
             double g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 12 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1553,7 +1555,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_1 = 0;
           double o34_1 = 0;
           double o35_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -1591,7 +1593,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_32 = 0;
             double g1_33 = 0;
             double g1_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 12 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3054,7 +3056,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_2 = 0;
           double o34_2 = 0;
           double o35_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -3092,7 +3094,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_32 = 0;
             double g2_33 = 0;
             double g2_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 12 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4545,7 +4547,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_3 = 0;
           double o34_3 = 0;
           double o35_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -4583,7 +4585,7 @@ jk_DD_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_32 = 0;
             double g3_33 = 0;
             double g3_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 12 * kS;
               const double q = kj[0];
               const double pq = p + q;

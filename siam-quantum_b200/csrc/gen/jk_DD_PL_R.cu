@@ -32,8 +32,10 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -97,7 +99,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -138,7 +140,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_0 = 0;
           double o34_0 = 0;
           double o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -176,7 +178,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_32 = 0;
             double g0_33 = 0;
             double g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1640,7 +1642,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_1 = 0;
           double o34_1 = 0;
           double o35_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -1678,7 +1680,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_32 = 0;
             double g1_33 = 0;
             double g1_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3243,7 +3245,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_2 = 0;
           double o34_2 = 0;
           double o35_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -3281,7 +3283,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_32 = 0;
             double g2_33 = 0;
             double g2_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4877,7 +4879,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_3 = 0;
           double o34_3 = 0;
           double o35_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -4915,7 +4917,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_32 = 0;
             double g3_33 = 0;
             double g3_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6507,7 +6509,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_4 = 0;
           double o34_4 = 0;
           double o35_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -6545,7 +6547,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_32 = 0;
             double g4_33 = 0;
             double g4_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7998,7 +8000,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_5 = 0;
           double o34_5 = 0;
           double o35_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -8036,7 +8038,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_32 = 0;
             double g5_33 = 0;
             double g5_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9632,7 +9634,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_6 = 0;
           double o34_6 = 0;
           double o35_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -9670,7 +9672,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_32 = 0;
             double g6_33 = 0;
             double g6_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11205,7 +11207,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_7 = 0;
           double o34_7 = 0;
           double o35_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -11243,7 +11245,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_32 = 0;
             double g7_33 = 0;
             double g7_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -12821,7 +12823,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_8 = 0;
           double o34_8 = 0;
           double o35_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -12859,7 +12861,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_32 = 0;
             double g8_33 = 0;
             double g8_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -14308,7 +14310,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_9 = 0;
           double o34_9 = 0;
           double o35_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -14346,7 +14348,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_32 = 0;
             double g9_33 = 0;
             double g9_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -15938,7 +15940,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_10 = 0;
           double o34_10 = 0;
           double o35_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -15976,7 +15978,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_32 = 0;
             double g10_33 = 0;
             double g10_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -17554,7 +17556,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_11 = 0;
           double o34_11 = 0;
           double o35_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -17592,7 +17594,7 @@ jk_DD_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_32 = 0;
             double g11_33 = 0;
             double g11_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -33,8 +33,10 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -93,7 +95,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -135,7 +137,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_0 = 0;
           float o34_0 = 0;
           float o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -173,7 +175,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g0_32 = 0;
             float g0_33 = 0;
             float g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -1606,7 +1608,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_1 = 0;
           float o34_1 = 0;
           float o35_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g1_0 = 0;
@@ -1644,7 +1646,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g1_32 = 0;
             float g1_33 = 0;
             float g1_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -3178,7 +3180,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_2 = 0;
           float o34_2 = 0;
           float o35_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g2_0 = 0;
@@ -3216,7 +3218,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g2_32 = 0;
             float g2_33 = 0;
             float g2_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -4781,7 +4783,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_3 = 0;
           float o34_3 = 0;
           float o35_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g3_0 = 0;
@@ -4819,7 +4821,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g3_32 = 0;
             float g3_33 = 0;
             float g3_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -6380,7 +6382,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_4 = 0;
           float o34_4 = 0;
           float o35_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g4_0 = 0;
@@ -6418,7 +6420,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g4_32 = 0;
             float g4_33 = 0;
             float g4_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -7840,7 +7842,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_5 = 0;
           float o34_5 = 0;
           float o35_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g5_0 = 0;
@@ -7878,7 +7880,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g5_32 = 0;
             float g5_33 = 0;
             float g5_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -9443,7 +9445,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_6 = 0;
           float o34_6 = 0;
           float o35_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g6_0 = 0;
@@ -9481,7 +9483,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g6_32 = 0;
             float g6_33 = 0;
             float g6_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -10985,7 +10987,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_7 = 0;
           float o34_7 = 0;
           float o35_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g7_0 = 0;
@@ -11023,7 +11025,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g7_32 = 0;
             float g7_33 = 0;
             float g7_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -12570,7 +12572,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_8 = 0;
           float o34_8 = 0;
           float o35_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g8_0 = 0;
@@ -12608,7 +12610,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g8_32 = 0;
             float g8_33 = 0;
             float g8_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -14026,7 +14028,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_9 = 0;
           float o34_9 = 0;
           float o35_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g9_0 = 0;
@@ -14064,7 +14066,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g9_32 = 0;
             float g9_33 = 0;
             float g9_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -15625,7 +15627,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_10 = 0;
           float o34_10 = 0;
           float o35_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g10_0 = 0;
@@ -15663,7 +15665,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g10_32 = 0;
             float g10_33 = 0;
             float g10_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -17210,7 +17212,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_11 = 0;
           float o34_11 = 0;
           float o35_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g11_0 = 0;
@@ -17248,7 +17250,7 @@ jk_DD_PL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g11_32 = 0;
             float g11_33 = 0;
             float g11_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const float q = kj[0];
               const float pq = p + q;

@@ -32,8 +32,10 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -97,7 +99,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -138,7 +140,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_0 = 0;
           double o34_0 = 0;
           double o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -176,7 +178,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_32 = 0;
             double g0_33 = 0;
             double g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1742,7 +1744,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_1 = 0;
           double o34_1 = 0;
           double o35_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -1780,7 +1782,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_32 = 0;
             double g1_33 = 0;
             double g1_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3376,7 +3378,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_2 = 0;
           double o34_2 = 0;
           double o35_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -3414,7 +3416,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_32 = 0;
             double g2_33 = 0;
             double g2_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5006,7 +5008,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_3 = 0;
           double o34_3 = 0;
           double o35_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -5044,7 +5046,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_32 = 0;
             double g3_33 = 0;
             double g3_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6640,7 +6642,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_4 = 0;
           double o34_4 = 0;
           double o35_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -6678,7 +6680,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_32 = 0;
             double g4_33 = 0;
             double g4_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8213,7 +8215,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_5 = 0;
           double o34_5 = 0;
           double o35_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -8251,7 +8253,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_32 = 0;
             double g5_33 = 0;
             double g5_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9829,7 +9831,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_6 = 0;
           double o34_6 = 0;
           double o35_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -9867,7 +9869,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_32 = 0;
             double g6_33 = 0;
             double g6_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11459,7 +11461,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_7 = 0;
           double o34_7 = 0;
           double o35_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -11497,7 +11499,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_32 = 0;
             double g7_33 = 0;
             double g7_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13075,7 +13077,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o33_8 = 0;
           double o34_8 = 0;
           double o35_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 341;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -13113,7 +13115,7 @@ jk_DD_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_32 = 0;
             double g8_33 = 0;
             double g8_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;

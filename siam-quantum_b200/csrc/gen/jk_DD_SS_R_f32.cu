@@ -33,8 +33,10 @@ jk_DD_SS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 341; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -93,7 +95,7 @@ jk_DD_SS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -134,7 +136,7 @@ jk_DD_SS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o33_0 = 0;
           float o34_0 = 0;
           float o35_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 341;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -172,7 +174,7 @@ jk_DD_SS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g0_32 = 0;
             float g0_33 = 0;
             float g0_34 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 6 * kS;
               const float q = kj[0];
               const float pq = p + q;

@@ -32,8 +32,10 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -85,7 +87,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -114,7 +116,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_0 = 0;
           double o22_0 = 0;
           double o23_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -137,7 +139,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -888,7 +890,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_1 = 0;
           double o22_1 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -911,7 +913,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1733,7 +1735,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_2 = 0;
           double o22_2 = 0;
           double o23_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1756,7 +1758,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2626,7 +2628,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_3 = 0;
           double o22_3 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2649,7 +2651,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3516,7 +3518,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_4 = 0;
           double o22_4 = 0;
           double o23_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3539,7 +3541,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4271,7 +4273,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_5 = 0;
           double o22_5 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -4294,7 +4296,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5148,7 +5150,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_6 = 0;
           double o22_6 = 0;
           double o23_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -5171,7 +5173,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5957,7 +5959,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_7 = 0;
           double o22_7 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5980,7 +5982,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6820,7 +6822,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_8 = 0;
           double o22_8 = 0;
           double o23_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -6843,7 +6845,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7566,7 +7568,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_9 = 0;
           double o22_9 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -7589,7 +7591,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8434,7 +8436,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_10 = 0;
           double o22_10 = 0;
           double o23_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -8457,7 +8459,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9290,7 +9292,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_11 = 0;
           double o22_11 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -9313,7 +9315,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10081,7 +10083,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_12 = 0;
           double o22_12 = 0;
           double o23_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -10104,7 +10106,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g12_17 = 0;
             double g12_18 = 0;
             double g12_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10873,7 +10875,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_13 = 0;
           double o22_13 = 0;
           double o23_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g13_0 = 0;
@@ -10896,7 +10898,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11766,7 +11768,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_14 = 0;
           double o22_14 = 0;
           double o23_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -11789,7 +11791,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -12643,7 +12645,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_15 = 0;
           double o22_15 = 0;
           double o23_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -12666,7 +12668,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13571,7 +13573,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_16 = 0;
           double o22_16 = 0;
           double o23_16 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g16_0 = 0;
@@ -13594,7 +13596,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g16_17 = 0;
             double g16_18 = 0;
             double g16_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -14360,7 +14362,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_17 = 0;
           double o22_17 = 0;
           double o23_17 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g17_0 = 0;
@@ -14383,7 +14385,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g17_17 = 0;
             double g17_18 = 0;
             double g17_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -15250,7 +15252,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_18 = 0;
           double o22_18 = 0;
           double o23_18 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g18_0 = 0;
@@ -15273,7 +15275,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g18_17 = 0;
             double g18_18 = 0;
             double g18_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -16178,7 +16180,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_19 = 0;
           double o22_19 = 0;
           double o23_19 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g19_0 = 0;
@@ -16201,7 +16203,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g19_17 = 0;
             double g19_18 = 0;
             double g19_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -17046,7 +17048,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_20 = 0;
           double o22_20 = 0;
           double o23_20 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g20_0 = 0;
@@ -17069,7 +17071,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g20_17 = 0;
             double g20_18 = 0;
             double g20_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -17826,7 +17828,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_21 = 0;
           double o22_21 = 0;
           double o23_21 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g21_0 = 0;
@@ -17849,7 +17851,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g21_17 = 0;
             double g21_18 = 0;
             double g21_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -18754,7 +18756,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_22 = 0;
           double o22_22 = 0;
           double o23_22 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g22_0 = 0;
@@ -18777,7 +18779,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g22_17 = 0;
             double g22_18 = 0;
             double g22_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -19617,7 +19619,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_23 = 0;
           double o22_23 = 0;
           double o23_23 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g23_0 = 0;
@@ -19640,7 +19642,7 @@ jk_DL_DL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g23_17 = 0;
             double g23_18 = 0;
             double g23_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -80,7 +82,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -134,7 +136,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_1 = 0;
           double o23_0 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -177,7 +179,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1243,7 +1245,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_3 = 0;
           double o23_2 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1286,7 +1288,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2480,7 +2482,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_5 = 0;
           double o23_4 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -2523,7 +2525,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3620,7 +3622,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_7 = 0;
           double o23_6 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -3663,7 +3665,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4779,7 +4781,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_9 = 0;
           double o23_8 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -4822,7 +4824,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5910,7 +5912,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_11 = 0;
           double o23_10 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -5953,7 +5955,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7057,7 +7059,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_13 = 0;
           double o23_12 = 0;
           double o23_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -7100,7 +7102,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8234,7 +8236,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_15 = 0;
           double o23_14 = 0;
           double o23_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -8277,7 +8279,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9504,7 +9506,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_17 = 0;
           double o23_16 = 0;
           double o23_17 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g16_0 = 0;
@@ -9547,7 +9549,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g17_17 = 0;
             double g17_18 = 0;
             double g17_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10678,7 +10680,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_19 = 0;
           double o23_18 = 0;
           double o23_19 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g18_0 = 0;
@@ -10721,7 +10723,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g19_17 = 0;
             double g19_18 = 0;
             double g19_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11944,7 +11946,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_21 = 0;
           double o23_20 = 0;
           double o23_21 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g20_0 = 0;
@@ -11987,7 +11989,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g21_17 = 0;
             double g21_18 = 0;
             double g21_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13156,7 +13158,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o22_23 = 0;
           double o23_22 = 0;
           double o23_23 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g22_0 = 0;
@@ -13199,7 +13201,7 @@ jk_DL_DL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g23_17 = 0;
             double g23_18 = 0;
             double g23_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 134 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -85,7 +87,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -114,7 +116,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_0 = 0;
           double o22_0 = 0;
           double o23_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -137,7 +139,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -960,7 +962,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_1 = 0;
           double o22_1 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -983,7 +985,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1853,7 +1855,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_2 = 0;
           double o22_2 = 0;
           double o23_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1876,7 +1878,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2743,7 +2745,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_3 = 0;
           double o22_3 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2766,7 +2768,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3620,7 +3622,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_4 = 0;
           double o22_4 = 0;
           double o23_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3643,7 +3645,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4429,7 +4431,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_5 = 0;
           double o22_5 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -4452,7 +4454,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5292,7 +5294,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_6 = 0;
           double o22_6 = 0;
           double o23_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -5315,7 +5317,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6160,7 +6162,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_7 = 0;
           double o22_7 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -6183,7 +6185,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7016,7 +7018,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_8 = 0;
           double o22_8 = 0;
           double o23_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -7039,7 +7041,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7807,7 +7809,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_9 = 0;
           double o22_9 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -7830,7 +7832,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8700,7 +8702,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_10 = 0;
           double o22_10 = 0;
           double o23_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -8723,7 +8725,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9577,7 +9579,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_11 = 0;
           double o22_11 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -9600,7 +9602,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10505,7 +10507,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_12 = 0;
           double o22_12 = 0;
           double o23_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -10528,7 +10530,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g12_17 = 0;
             double g12_18 = 0;
             double g12_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11395,7 +11397,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_13 = 0;
           double o22_13 = 0;
           double o23_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g13_0 = 0;
@@ -11418,7 +11420,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -12323,7 +12325,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_14 = 0;
           double o22_14 = 0;
           double o23_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -12346,7 +12348,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13191,7 +13193,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_15 = 0;
           double o22_15 = 0;
           double o23_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -13214,7 +13216,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -14119,7 +14121,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_16 = 0;
           double o22_16 = 0;
           double o23_16 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g16_0 = 0;
@@ -14142,7 +14144,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g16_17 = 0;
             double g16_18 = 0;
             double g16_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -14982,7 +14984,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_17 = 0;
           double o22_17 = 0;
           double o23_17 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g17_0 = 0;
@@ -15005,7 +15007,7 @@ jk_DL_DP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g17_17 = 0;
             double g17_18 = 0;
             double g17_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;

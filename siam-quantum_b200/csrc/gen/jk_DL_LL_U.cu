@@ -32,8 +32,10 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -85,7 +87,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -115,7 +117,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_0 = 0;
           double o22_0 = 0;
           double o23_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -138,7 +140,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -815,7 +817,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_1 = 0;
           double o22_1 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -838,7 +840,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1566,7 +1568,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_2 = 0;
           double o22_2 = 0;
           double o23_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1589,7 +1591,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2311,7 +2313,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_3 = 0;
           double o22_3 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2334,7 +2336,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3053,7 +3055,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_4 = 0;
           double o22_4 = 0;
           double o23_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3076,7 +3078,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3804,7 +3806,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_5 = 0;
           double o22_5 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3827,7 +3829,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4617,7 +4619,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_6 = 0;
           double o22_6 = 0;
           double o23_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4640,7 +4642,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5449,7 +5451,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_7 = 0;
           double o22_7 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5472,7 +5474,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6278,7 +6280,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_8 = 0;
           double o22_8 = 0;
           double o23_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -6301,7 +6303,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7023,7 +7025,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_9 = 0;
           double o22_9 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -7046,7 +7048,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7855,7 +7857,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_10 = 0;
           double o22_10 = 0;
           double o23_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -7878,7 +7880,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8650,7 +8652,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_11 = 0;
           double o22_11 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -8673,7 +8675,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9470,7 +9472,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_12 = 0;
           double o22_12 = 0;
           double o23_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -9493,7 +9495,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g12_17 = 0;
             double g12_18 = 0;
             double g12_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10212,7 +10214,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_13 = 0;
           double o22_13 = 0;
           double o23_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g13_0 = 0;
@@ -10235,7 +10237,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11041,7 +11043,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_14 = 0;
           double o22_14 = 0;
           double o23_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -11064,7 +11066,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11861,7 +11863,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_15 = 0;
           double o22_15 = 0;
           double o23_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -11884,7 +11886,7 @@ jk_DL_LL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;

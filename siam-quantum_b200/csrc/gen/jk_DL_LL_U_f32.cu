@@ -33,8 +33,10 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -81,7 +83,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -135,7 +137,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_1 = 0;
           float o23_0 = 0;
           float o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -178,7 +180,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g1_17 = 0;
             float g1_18 = 0;
             float g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -1068,7 +1070,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_3 = 0;
           float o23_2 = 0;
           float o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g2_0 = 0;
@@ -1111,7 +1113,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g3_17 = 0;
             float g3_18 = 0;
             float g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -2022,7 +2024,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_5 = 0;
           float o23_4 = 0;
           float o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g4_0 = 0;
@@ -2065,7 +2067,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g5_17 = 0;
             float g5_18 = 0;
             float g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -3037,7 +3039,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_7 = 0;
           float o23_6 = 0;
           float o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g6_0 = 0;
@@ -3080,7 +3082,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g7_17 = 0;
             float g7_18 = 0;
             float g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -4125,7 +4127,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_9 = 0;
           float o23_8 = 0;
           float o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g8_0 = 0;
@@ -4168,7 +4170,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g9_17 = 0;
             float g9_18 = 0;
             float g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -5159,7 +5161,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_11 = 0;
           float o23_10 = 0;
           float o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g10_0 = 0;
@@ -5202,7 +5204,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g11_17 = 0;
             float g11_18 = 0;
             float g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -6213,7 +6215,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_13 = 0;
           float o23_12 = 0;
           float o23_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g12_0 = 0;
@@ -6256,7 +6258,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g13_17 = 0;
             float g13_18 = 0;
             float g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -7244,7 +7246,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o22_15 = 0;
           float o23_14 = 0;
           float o23_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 134;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g14_0 = 0;
@@ -7287,7 +7289,7 @@ jk_DL_LL_U_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g15_17 = 0;
             float g15_18 = 0;
             float g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const float q = kj[0];
               const float pq = p + q;

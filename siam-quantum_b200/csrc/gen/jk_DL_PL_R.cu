@@ -32,8 +32,10 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -85,7 +87,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -114,7 +116,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_0 = 0;
           double o22_0 = 0;
           double o23_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -137,7 +139,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -826,7 +828,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_1 = 0;
           double o22_1 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -849,7 +851,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1599,7 +1601,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_2 = 0;
           double o22_2 = 0;
           double o23_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1622,7 +1624,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2391,7 +2393,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_3 = 0;
           double o22_3 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2414,7 +2416,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3180,7 +3182,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_4 = 0;
           double o22_4 = 0;
           double o23_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3203,7 +3205,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3885,7 +3887,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_5 = 0;
           double o22_5 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3908,7 +3910,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4677,7 +4679,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_6 = 0;
           double o22_6 = 0;
           double o23_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4700,7 +4702,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5432,7 +5434,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_7 = 0;
           double o22_7 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5455,7 +5457,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6212,7 +6214,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_8 = 0;
           double o22_8 = 0;
           double o23_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -6235,7 +6237,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6914,7 +6916,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_9 = 0;
           double o22_9 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -6937,7 +6939,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7703,7 +7705,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_10 = 0;
           double o22_10 = 0;
           double o23_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -7726,7 +7728,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8483,7 +8485,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_11 = 0;
           double o22_11 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -8506,7 +8508,7 @@ jk_DL_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 134; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -85,7 +87,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -115,7 +117,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_0 = 0;
           double o22_0 = 0;
           double o23_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -138,7 +140,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -867,7 +869,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_1 = 0;
           double o22_1 = 0;
           double o23_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -890,7 +892,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1680,7 +1682,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_2 = 0;
           double o22_2 = 0;
           double o23_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1703,7 +1705,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2512,7 +2514,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_3 = 0;
           double o22_3 = 0;
           double o23_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2535,7 +2537,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3341,7 +3343,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_4 = 0;
           double o22_4 = 0;
           double o23_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3364,7 +3366,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4086,7 +4088,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_5 = 0;
           double o22_5 = 0;
           double o23_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -4109,7 +4111,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4918,7 +4920,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_6 = 0;
           double o22_6 = 0;
           double o23_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4941,7 +4943,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5713,7 +5715,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_7 = 0;
           double o22_7 = 0;
           double o23_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5736,7 +5738,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6533,7 +6535,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_8 = 0;
           double o22_8 = 0;
           double o23_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -6556,7 +6558,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7275,7 +7277,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_9 = 0;
           double o22_9 = 0;
           double o23_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -7298,7 +7300,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8104,7 +8106,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_10 = 0;
           double o22_10 = 0;
           double o23_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -8127,7 +8129,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8924,7 +8926,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o21_11 = 0;
           double o22_11 = 0;
           double o23_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 134;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -8947,7 +8949,7 @@ jk_DL_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;

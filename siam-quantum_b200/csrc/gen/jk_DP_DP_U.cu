@@ -32,8 +32,10 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -79,7 +81,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -103,7 +105,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_0 = 0;
           double o16_0 = 0;
           double o17_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -126,7 +128,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -888,7 +890,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_1 = 0;
           double o16_1 = 0;
           double o17_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -911,7 +913,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1720,7 +1722,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_2 = 0;
           double o16_2 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1743,7 +1745,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2549,7 +2551,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_3 = 0;
           double o16_3 = 0;
           double o17_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2572,7 +2574,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3365,7 +3367,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_4 = 0;
           double o16_4 = 0;
           double o17_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -3388,7 +3390,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4113,7 +4115,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_5 = 0;
           double o16_5 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -4136,7 +4138,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4915,7 +4917,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_6 = 0;
           double o16_6 = 0;
           double o17_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4938,7 +4940,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5722,7 +5724,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_7 = 0;
           double o16_7 = 0;
           double o17_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5745,7 +5747,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6517,7 +6519,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_8 = 0;
           double o16_8 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -6540,7 +6542,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7247,7 +7249,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_9 = 0;
           double o16_9 = 0;
           double o17_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -7270,7 +7272,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8079,7 +8081,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_10 = 0;
           double o16_10 = 0;
           double o17_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -8102,7 +8104,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8895,7 +8897,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_11 = 0;
           double o16_11 = 0;
           double o17_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -8918,7 +8920,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9762,7 +9764,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_12 = 0;
           double o16_12 = 0;
           double o17_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -9785,7 +9787,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g12_17 = 0;
             double g12_18 = 0;
             double g12_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -10591,7 +10593,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_13 = 0;
           double o16_13 = 0;
           double o17_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g13_0 = 0;
@@ -10614,7 +10616,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -11458,7 +11460,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_14 = 0;
           double o16_14 = 0;
           double o17_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -11481,7 +11483,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -12265,7 +12267,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_15 = 0;
           double o16_15 = 0;
           double o17_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -12288,7 +12290,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13132,7 +13134,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_16 = 0;
           double o16_16 = 0;
           double o17_16 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g16_0 = 0;
@@ -13155,7 +13157,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g16_17 = 0;
             double g16_18 = 0;
             double g16_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -13934,7 +13936,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_17 = 0;
           double o16_17 = 0;
           double o17_17 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g17_0 = 0;
@@ -13957,7 +13959,7 @@ jk_DP_DP_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g17_17 = 0;
             double g17_18 = 0;
             double g17_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 113 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -79,7 +81,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -102,7 +104,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_0 = 0;
           double o16_0 = 0;
           double o17_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -125,7 +127,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -665,7 +667,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_1 = 0;
           double o16_1 = 0;
           double o17_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -688,7 +690,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1279,7 +1281,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_2 = 0;
           double o16_2 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1302,7 +1304,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1887,7 +1889,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_3 = 0;
           double o16_3 = 0;
           double o17_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -1910,7 +1912,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2492,7 +2494,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_4 = 0;
           double o16_4 = 0;
           double o17_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -2515,7 +2517,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3106,7 +3108,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_5 = 0;
           double o16_5 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3129,7 +3131,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3782,7 +3784,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_6 = 0;
           double o16_6 = 0;
           double o17_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -3805,7 +3807,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4477,7 +4479,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_7 = 0;
           double o16_7 = 0;
           double o17_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -4500,7 +4502,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5169,7 +5171,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_8 = 0;
           double o16_8 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -5192,7 +5194,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5777,7 +5779,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_9 = 0;
           double o16_9 = 0;
           double o17_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -5800,7 +5802,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6472,7 +6474,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_10 = 0;
           double o16_10 = 0;
           double o17_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -6495,7 +6497,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7130,7 +7132,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_11 = 0;
           double o16_11 = 0;
           double o17_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -7153,7 +7155,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7813,7 +7815,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_12 = 0;
           double o16_12 = 0;
           double o17_12 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -7836,7 +7838,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g12_17 = 0;
             double g12_18 = 0;
             double g12_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -8418,7 +8420,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_13 = 0;
           double o16_13 = 0;
           double o17_13 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g13_0 = 0;
@@ -8441,7 +8443,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g13_17 = 0;
             double g13_18 = 0;
             double g13_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9110,7 +9112,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_14 = 0;
           double o16_14 = 0;
           double o17_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g14_0 = 0;
@@ -9133,7 +9135,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -9793,7 +9795,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_15 = 0;
           double o16_15 = 0;
           double o17_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -9816,7 +9818,7 @@ jk_DP_LL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -74,7 +76,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -134,7 +136,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o17_0 = 0;
           double o17_1 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -197,7 +199,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1177,7 +1179,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o17_3 = 0;
           double o17_4 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -1240,7 +1242,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2338,7 +2340,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o17_6 = 0;
           double o17_7 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -2401,7 +2403,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3568,7 +3570,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o17_9 = 0;
           double o17_10 = 0;
           double o17_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -3631,7 +3633,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4778,7 +4780,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o17_12 = 0;
           double o17_13 = 0;
           double o17_14 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g12_0 = 0;
@@ -4841,7 +4843,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g14_17 = 0;
             double g14_18 = 0;
             double g14_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5926,7 +5928,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_15 = 0;
           double o16_15 = 0;
           double o17_15 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g15_0 = 0;
@@ -5949,7 +5951,7 @@ jk_DP_LL_U_w(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g15_17 = 0;
             double g15_18 = 0;
             double g15_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 51 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -79,7 +81,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -102,7 +104,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_0 = 0;
           double o16_0 = 0;
           double o17_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -125,7 +127,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -717,7 +719,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_1 = 0;
           double o16_1 = 0;
           double o17_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -740,7 +742,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1393,7 +1395,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_2 = 0;
           double o16_2 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1416,7 +1418,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2088,7 +2090,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_3 = 0;
           double o16_3 = 0;
           double o17_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2111,7 +2113,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2780,7 +2782,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_4 = 0;
           double o16_4 = 0;
           double o17_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -2803,7 +2805,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3388,7 +3390,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_5 = 0;
           double o16_5 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3411,7 +3413,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4083,7 +4085,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_6 = 0;
           double o16_6 = 0;
           double o17_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4106,7 +4108,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4741,7 +4743,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_7 = 0;
           double o16_7 = 0;
           double o17_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -4764,7 +4766,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5424,7 +5426,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_8 = 0;
           double o16_8 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -5447,7 +5449,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6029,7 +6031,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_9 = 0;
           double o16_9 = 0;
           double o17_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -6052,7 +6054,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6721,7 +6723,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_10 = 0;
           double o16_10 = 0;
           double o17_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -6744,7 +6746,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7404,7 +7406,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_11 = 0;
           double o16_11 = 0;
           double o17_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -7427,7 +7429,7 @@ jk_DP_PL_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -79,7 +81,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PB = a.PB + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
@@ -103,7 +105,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_0 = 0;
           double o16_0 = 0;
           double o17_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -126,7 +128,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -754,7 +756,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_1 = 0;
           double o16_1 = 0;
           double o17_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -777,7 +779,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1466,7 +1468,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_2 = 0;
           double o16_2 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1489,7 +1491,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2197,7 +2199,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_3 = 0;
           double o16_3 = 0;
           double o17_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2220,7 +2222,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2925,7 +2927,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_4 = 0;
           double o16_4 = 0;
           double o17_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -2948,7 +2950,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3569,7 +3571,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_5 = 0;
           double o16_5 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3592,7 +3594,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4300,7 +4302,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_6 = 0;
           double o16_6 = 0;
           double o17_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4323,7 +4325,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4994,7 +4996,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_7 = 0;
           double o16_7 = 0;
           double o17_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -5017,7 +5019,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5713,7 +5715,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_8 = 0;
           double o16_8 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -5736,7 +5738,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -6354,7 +6356,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_9 = 0;
           double o16_9 = 0;
           double o17_9 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g9_0 = 0;
@@ -6377,7 +6379,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g9_17 = 0;
             double g9_18 = 0;
             double g9_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7082,7 +7084,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_10 = 0;
           double o16_10 = 0;
           double o17_10 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g10_0 = 0;
@@ -7105,7 +7107,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g10_17 = 0;
             double g10_18 = 0;
             double g10_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -7801,7 +7803,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_11 = 0;
           double o16_11 = 0;
           double o17_11 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g11_0 = 0;
@@ -7824,7 +7826,7 @@ jk_DP_PL_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g11_17 = 0;
             double g11_18 = 0;
             double g11_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 44 * kS;
               const double q = kj[0];
               const double pq = p + q;

@@ -32,8 +32,10 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -79,7 +81,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -102,7 +104,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_0 = 0;
           double o16_0 = 0;
           double o17_0 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -125,7 +127,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g0_17 = 0;
             double g0_18 = 0;
             double g0_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -779,7 +781,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_1 = 0;
           double o16_1 = 0;
           double o17_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g1_0 = 0;
@@ -802,7 +804,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_17 = 0;
             double g1_18 = 0;
             double g1_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1474,7 +1476,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_2 = 0;
           double o16_2 = 0;
           double o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -1497,7 +1499,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_17 = 0;
             double g2_18 = 0;
             double g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2166,7 +2168,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_3 = 0;
           double o16_3 = 0;
           double o17_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g3_0 = 0;
@@ -2189,7 +2191,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_17 = 0;
             double g3_18 = 0;
             double g3_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -2861,7 +2863,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_4 = 0;
           double o16_4 = 0;
           double o17_4 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -2884,7 +2886,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g4_17 = 0;
             double g4_18 = 0;
             double g4_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -3519,7 +3521,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_5 = 0;
           double o16_5 = 0;
           double o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g5_0 = 0;
@@ -3542,7 +3544,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_17 = 0;
             double g5_18 = 0;
             double g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4202,7 +4204,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_6 = 0;
           double o16_6 = 0;
           double o17_6 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g6_0 = 0;
@@ -4225,7 +4227,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g6_17 = 0;
             double g6_18 = 0;
             double g6_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -4894,7 +4896,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_7 = 0;
           double o16_7 = 0;
           double o17_7 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g7_0 = 0;
@@ -4917,7 +4919,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g7_17 = 0;
             double g7_18 = 0;
             double g7_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -5577,7 +5579,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o15_8 = 0;
           double o16_8 = 0;
           double o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 113;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g8_0 = 0;
@@ -5600,7 +5602,7 @@ jk_DP_PP_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g8_17 = 0;
             double g8_18 = 0;
             double g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const double q = kj[0];
               const double pq = p + q;

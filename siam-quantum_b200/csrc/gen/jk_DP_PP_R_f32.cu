@@ -33,8 +33,10 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 113; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -75,7 +77,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -134,7 +136,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o17_0 = 0;
           float o17_1 = 0;
           float o17_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 113;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -197,7 +199,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g2_17 = 0;
             float g2_18 = 0;
             float g2_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -1283,7 +1285,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o17_3 = 0;
           float o17_4 = 0;
           float o17_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 113;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g3_0 = 0;
@@ -1346,7 +1348,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g5_17 = 0;
             float g5_18 = 0;
             float g5_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const float q = kj[0];
               const float pq = p + q;
@@ -2421,7 +2423,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o17_6 = 0;
           float o17_7 = 0;
           float o17_8 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 113;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g6_0 = 0;
@@ -2484,7 +2486,7 @@ jk_DP_PP_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g8_17 = 0;
             float g8_18 = 0;
             float g8_19 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 38 * kS;
               const float q = kj[0];
               const float pq = p + q;

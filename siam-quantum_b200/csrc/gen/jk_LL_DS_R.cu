@@ -32,8 +32,10 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 51; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -77,7 +79,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -114,7 +116,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o14_1 = 0;
           double o15_0 = 0;
           double o15_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 51;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -137,7 +139,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_7 = 0;
             double g1_8 = 0;
             double g1_9 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 26 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -664,7 +666,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o14_3 = 0;
           double o15_2 = 0;
           double o15_3 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 51;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -687,7 +689,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g3_7 = 0;
             double g3_8 = 0;
             double g3_9 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 26 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -1221,7 +1223,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o14_5 = 0;
           double o15_4 = 0;
           double o15_5 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 51;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g4_0 = 0;
@@ -1244,7 +1246,7 @@ jk_LL_DS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g5_7 = 0;
             double g5_8 = 0;
             double g5_9 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 26 * kS;
               const double q = kj[0];
               const double pq = p + q;

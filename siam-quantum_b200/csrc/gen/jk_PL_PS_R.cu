@@ -32,8 +32,10 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 44; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -73,7 +75,7 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = mpq ? 0 : bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -102,7 +104,7 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o10_1 = 0;
           double o11_0 = 0;
           double o11_1 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 44;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g0_0 = 0;
@@ -125,7 +127,7 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g1_7 = 0;
             double g1_8 = 0;
             double g1_9 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 11 * kS;
               const double q = kj[0];
               const double pq = p + q;
@@ -521,7 +523,7 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           double o9_2 = 0;
           double o10_2 = 0;
           double o11_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const double* __restrict__ bi = sbra + i * 44;
             const double p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             double g2_0 = 0;
@@ -534,7 +536,7 @@ jk_PL_PS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             double g2_7 = 0;
             double g2_8 = 0;
             double g2_9 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const double* __restrict__ kj = kprim + (long long)j * 11 * kS;
               const double q = kj[0];
               const double pq = p + q;

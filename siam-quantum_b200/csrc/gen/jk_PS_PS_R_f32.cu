@@ -33,8 +33,10 @@ jk_PS_PS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 11; x += blockDim.x) sbra[x] = a.bra_prims_f[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (bra primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -60,7 +62,7 @@ jk_PS_PS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const float* __restrict__ kprim = a.ket_prims_f + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nbp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gi < nbp ? (unsigned long long)((nbp - gi + si - 1) / si) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
@@ -74,7 +76,7 @@ jk_PS_PS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
           float o2_0 = 0;
           float o2_1 = 0;
           float o2_2 = 0;
-          for (int i = grp; i < nbp; i += isplit) {
+          for (int i = gi; i < nbp; i += si) {
             const float* __restrict__ bi = sbra + i * 11;
             const float p = bi[0], Px = bi[1], Py = bi[2], Pz = bi[3], kpb = bi[4];
             float g0_0 = 0;
@@ -89,7 +91,7 @@ jk_PS_PS_R_f32(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             float g2_1 = 0;
             float g2_2 = 0;
             float g2_3 = 0;
-            for (int j = 0; j < nkp; ++j) {
+            for (int j = gj; j < nkp; j += sj) {
               const float* __restrict__ kj = kprim + (long long)j * 11 * kS;
               const float q = kj[0];
               const float pq = p + q;

@@ -32,8 +32,10 @@ jk_SS_SS_R_s(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 6; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
-      const int isplit = it.isplit;                 // threads sharing one quartet (ket primitives split)
+      // threads sharing one quartet: si strides over the bra primitives x sj over the ket primitives
+      const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
+      const int gj = grp / si, gi = grp - gj * si;
       const int pass = qp_;                   // block of bra functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -57,17 +59,17 @@ jk_SS_SS_R_s(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         const double* __restrict__ kprim = a.ket_prims + kp.poff;
         const int kS = kp.kstride;                   // distance between the fields of one ket record
         const int nbp = bp.nprim, nkp = kp.nprim;
-        nflush = pass == 0 ? (unsigned long long)((nkp - grp + isplit - 1) / isplit) : 0ull;
+        nflush = pass == 0 && gj < nkp ? (unsigned long long)((nkp - gj + sj - 1) / sj) : 0ull;
         const double* __restrict__ PA = a.PA + mr.moff;
         const double* __restrict__ PT = a.PT + mr.moff;
         switch (pass) {
         case 0: {  // bra functions [0]
           double o0_0 = 0;
-          for (int j = grp; j < nkp; j += isplit) {
+          for (int j = gj; j < nkp; j += sj) {
             const double* __restrict__ kj = kprim + (long long)j * 6 * kS;
             const double q = kj[0], Qx = kj[kS], Qy = kj[2 * kS], Qz = kj[3 * kS], kq = kj[4 * kS];
             double g0_0 = 0;
-            for (int i = 0; i < nbp; ++i) {
+            for (int i = gi; i < nbp; i += si) {
               const double* __restrict__ bi = sbra + i * 6;
               const double p = bi[0];
               const double pq = p + q;

@@ -3,9 +3,9 @@
 // Boys function F_m(T) = int_0^1 u^(2m) exp(-T u^2) du  (role of fgamma_set, reference
 // src/fgamma.c:172-206).  Written from the mathematics, not from any library:
 //   T <  BOYS_TMAX : the top order F_M(T) by a 9-term Taylor expansion about the nearest grid
-//                    point T0 (spacing BOYS_H), F_M(T0+d) = sum_k F_{M+k}(T0) (-d)^k / k!,
+//                    point T0 (spacing BOYS_H), F_M(T0-x) = sum_k F_{M+k}(T0) x^k / k!,
 //                    then the stable downward recursion F_m = (2T F_{m+1} + e^-T)/(2m+1), with
-//                    e^-T = e^-T0 e^-d from a tabulated e^-T0 and the Taylor series of e^-d.
+//                    e^-T = e^-T0 e^x from a tabulated e^-T0 and the Taylor series of e^x.
 //   T >= BOYS_TMAX : F_0 = sqrt(pi/T)/2 (the erfc tail is below 1e-17 relative there) and the
 //                    stable upward recursion F_{m+1} = ((2m+1) F_m - e^-T)/(2T).
 // The grid values are computed on the host in extended precision (jk_engine.cu).
@@ -18,10 +18,12 @@
 #define BOYS_NGRID  361      // grid points T0 = 0, 0.1, ..., 36.0
 #define BOYS_MMAX   8        // highest order requested by a kernel ((dd|dd))
 #define BOYS_NTAY   9        // Taylor terms
-// columns m = 0..17 per grid row: a row is 144 bytes (a multiple of 16), so the Taylor values of
-// any order M (columns M..M+8, read from the even column at or below M) come in five 16-byte
-// loads; each lane gathers its own row, one L1 sector per load
+// plain table of F_m(T0), m = 0..17 per grid row (the gradient kernels' table)
 #define BOYS_NCOL   (BOYS_MMAX + BOYS_NTAY + 1)
+// row table of boys<M> / boysf<M>: per order M = 0..8 and grid point, the Taylor coefficients of
+// F_M about T0 and e^-T0 (FP64: 9 + 1 of 16 doubles; FP32: 6 + 1 of 8 floats)
+#define BOYS_ROW    16
+#define BOYS_ROWF   8
 
 #define TWO_PI_2_5  34.986836655249725     // 2 pi^(5/2)
 #define PRIM_CUTOFF 1.0e-15                // reference src/int.h:19
@@ -42,10 +44,11 @@ struct PairRec {
   double schwarz;  // max over the block of the basis-level Schwarz matrix
 };
 
-// A CTA's unit of work: one bra pair and a contiguous range of cnt ket pairs, each ket
-// handled by `isplit` threads (power of two) that split the bra primitives between them.
+// A CTA's unit of work: one bra pair and a contiguous range of cnt ket pairs, each ket handled by
+// si * sj threads: thread (gi, gj) takes the bra primitives gi, gi + si, ... and the ket
+// primitives gj, gj + sj, ... (split = si | sj << 16; si, sj >= 1).
 struct WorkItem {
-  int bra, k0, cnt, isplit;
+  int bra, k0, cnt, split;
   int mol;         // index of the molecule (MolRec) the pairs belong to
 };
 
@@ -73,14 +76,12 @@ struct JKArgs {
   double* Jacc;                // per molecule nbf x nbf, J = Jacc + Jacc^T
   double* KAacc;               // per molecule nbf x nbf, K[PA] = KAacc + KAacc^T
   double* KBacc;
-  const double* boys_tab;      // BOYS_NGRID x BOYS_NCOL
-  const float* boys_tab_f;     // the same table rounded to FP32 (mixed-precision forms)
+  const double* boys_tab;      // row table of boys<M>: (BOYS_MMAX + 1) x BOYS_NGRID x BOYS_ROW
+  const float* boys_tab_f;     // the FP32 row table (mixed-precision forms), rows of BOYS_ROWF
   unsigned long long* counters;// [0] quartets computed, [1] primitive quartets evaluated,
                                // [2] bra-primitive flushes, [3] digestions
   const MolRec* mols;          // per-molecule offsets, sizes and cutoffs (WorkItem::mol)
   int same_class;              // bra and ket pairs come from one class (pair identity possible)
-  int so_off;                  // doubles from the start of dynamic shared memory to the
-                               // accumulator slots of the shared-memory wide form
   const float* bra_prims_f;    // FP32 copies of the primitive records (mixed-precision kernels)
   const float* ket_prims_f;
   // Reference-parity multipole mode (erbank == nullptr: off; narrow FP64 form, isplit 1).
@@ -120,13 +121,19 @@ static __device__ __noinline__ double mpole_value(const double* __restrict__ mp,
   return __dmul_rn(__dmul_rn(m1[0], m2[0]), __dsqrt_rn(__ddiv_rn(1.0, K)));
 }
 
-// F_0..F_M at T.  M is a compile-time order so the recursion unrolls.
+// F_0..F_M at T.  M is a compile-time order so the recursion unrolls.  `tab` is the row table
+// (BOYS_ROW doubles per order and grid point): row (M, g) holds the Taylor coefficients
+// F_{M+k}(T0) / k! of F_M(T0 - x), k < BOYS_NTAY, and e^-T0, so one aligned 128-byte line serves
+// a lane in five 16-byte loads and neither series needs a multiplication per term.  Measured on
+// B200 against rows of plain F_{M+k}(T0) with the 1/k! multiplied in the kernel, e^-T0 in a table of
+// its own and a division and a square root above BOYS_TMAX (C60/6-31G, ms per launch): LL|LL wide
+// 41.0 -> 38.7, LL|LS wide 16.9 -> 15.9, LS|LS swapped 3.3 -> 2.5, LS|SS swapped 0.80 -> 0.58.
 template <int M>
 __device__ __forceinline__ void boys(double T, const double* __restrict__ tab, double* F) {
   if (T < BOYS_TMAX) {
     const int g = __double2int_rn(T * BOYS_INV_H);
-    const double d = T - g * BOYS_H;          // |d| <= BOYS_H/2
-    const double2* r2 = reinterpret_cast<const double2*>(tab + g * BOYS_NCOL + (M & ~1));
+    const double x = fma((double)g, BOYS_H, -T);   // T0 - T, |x| <= BOYS_H/2
+    const double2* r2 = reinterpret_cast<const double2*>(tab + (M * BOYS_NGRID + g) * BOYS_ROW);
     double v[BOYS_NTAY + 1];
 #pragma unroll
     for (int q = 0; q < (BOYS_NTAY + 1) / 2; ++q) {
@@ -134,57 +141,51 @@ __device__ __forceinline__ void boys(double T, const double* __restrict__ tab, d
       v[2 * q] = t.x;
       v[2 * q + 1] = t.y;
     }
-    const double* row = v + (M & 1);          // row[k] = F_{M+k}(T0)
-    // Horner in -d with 1/k! folded in: sum_k row[k] (-d)^k / k!
-    double s = row[BOYS_NTAY - 1];
+    double s = v[BOYS_NTAY - 1];
 #pragma unroll
-    for (int k = BOYS_NTAY - 2; k >= 0; --k) s = fma(s, -d * (1.0 / (double)(k + 1)), row[k]);
+    for (int k = BOYS_NTAY - 2; k >= 0; --k) s = fma(s, x, v[k]);
     F[M] = s;
     if (M > 0) {
-      // e^-T = e^-T0 e^-d: the grid value (stored after the table's rows) times the Taylor
-      // series of e^-d through d^9/9! (|d| <= 0.05: the next term is below 3e-20)
-      const double e0 = __ldg(tab + BOYS_NGRID * BOYS_NCOL + g);
-      double ed = 1.0;
-#pragma unroll
-      for (int k = 9; k >= 1; --k) ed = fma(ed, -d * (1.0 / (double)k), 1.0);
-      const double e = e0 * ed;
+      // e^-T = e^-T0 e^x: the row's e^-T0 times the Taylor series of e^x through x^8/8!
+      // (the next term is below 6e-18)
+      double ed = 1.0 / 40320.0;
+      ed = fma(ed, x, 1.0 / 5040.0);
+      ed = fma(ed, x, 1.0 / 720.0);
+      ed = fma(ed, x, 1.0 / 120.0);
+      ed = fma(ed, x, 1.0 / 24.0);
+      ed = fma(ed, x, 1.0 / 6.0);
+      ed = fma(ed, x, 0.5);
+      ed = fma(ed, x, 1.0);
+      ed = fma(ed, x, 1.0);
+      const double e = v[BOYS_NTAY] * ed;
       const double t2 = T + T;
 #pragma unroll
       for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (2 * m + 1));
     }
   } else {
-    const double it = 1.0 / T;
-    F[0] = 0.88622692545275801365 * sqrt(it);   // sqrt(pi)/2 / sqrt(T)
+    const double rt = rsqrt(T);
+    F[0] = 0.88622692545275801365 * rt;          // sqrt(pi)/2 / sqrt(T)
     if (M > 0) {
-      const double e = exp(-T);
-      const double h = 0.5 * it;
+      // e^-T is below 1e-17 of every (2m+1) F_m, m < 8, for T >= 64
+      const double e = T < 64.0 ? exp(-T) : 0.0;
+      const double h = 0.5 * rt * rt;
 #pragma unroll
-      for (int m = 0; m < M; ++m) F[m + 1] = ((2 * m + 1) * F[m] - e) * h;
+      for (int m = 0; m < M; ++m) F[m + 1] = fma(2 * m + 1, F[m], -e) * h;
     }
   }
 }
 
 // F_0..F_M at T in FP32, for the mixed-precision forms (quartets whose Schwarz bound is below
-// the FP32 threshold): the scheme of boys<M> with the FP32 table and 6 Taylor terms
-// (|d| <= BOYS_H/2: the next term is below 2e-11 of F_M, under FP32 rounding).
+// the FP32 threshold): the scheme of boys<M> with rows of BOYS_ROWF floats, 6 Taylor terms
+// (|x| <= BOYS_H/2: the next term is below 2e-11 of F_M, under FP32 rounding).
 template <int M>
 __device__ __forceinline__ void boysf(float T, const float* __restrict__ tab, float* F) {
   if (T < (float)BOYS_TMAX) {
     const int g = __float2int_rn(T * (float)BOYS_INV_H);
-    const float d = T - g * (float)BOYS_H;
-    const float2* r2 = reinterpret_cast<const float2*>(tab + g * BOYS_NCOL + (M & ~1));
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float2 t = __ldg(r2 + q);
-      v[2 * q] = t.x;
-      v[2 * q + 1] = t.y;
-    }
-    const float* row = v + (M & 1);           // row[k] = F_{M+k}(T0), k < 6
-    float s = row[5];
-#pragma unroll
-    for (int k = 4; k >= 0; --k) s = fmaf(s, -d * (1.0f / (float)(k + 1)), row[k]);
-    F[M] = s;
+    const float x = fmaf((float)g, (float)BOYS_H, -T);
+    const float4* r4 = reinterpret_cast<const float4*>(tab + (M * BOYS_NGRID + g) * BOYS_ROWF);
+    const float4 u = __ldg(r4), w = __ldg(r4 + 1);   // c0..c3; c4, c5, e^-T0
+    F[M] = fmaf(fmaf(fmaf(fmaf(fmaf(w.y, x, w.x), x, u.w), x, u.z), x, u.y), x, u.x);
     if (M > 0) {
       const float e = expf(-T);
       const float t2 = T + T;
@@ -192,45 +193,13 @@ __device__ __forceinline__ void boysf(float T, const float* __restrict__ tab, fl
       for (int m = M - 1; m >= 0; --m) F[m] = fmaf(t2, F[m + 1], e) * (1.0f / (float)(2 * m + 1));
     }
   } else {
-    const float it = 1.0f / T;
-    F[0] = 0.886226925f * sqrtf(it);
+    const float rt = rsqrtf(T);
+    F[0] = 0.886226925f * rt;
     if (M > 0) {
       const float e = expf(-T);
-      const float h = 0.5f * it;
+      const float h = 0.5f * rt * rt;
 #pragma unroll
       for (int m = 0; m < M; ++m) F[m + 1] = ((float)(2 * m + 1) * F[m] - e) * h;
-    }
-  }
-}
-
-// F_0..F_M at T, as boys<M> (R = double) or boysf<M> (R = float), reading the Taylor rows from
-// a copy of the table's columns in shared memory: s points at column M of a table of NC columns
-// per grid row (the staged columns start at some order c0 <= M; s = staged + M - c0).
-template <int M, int NC, class R>
-__device__ __forceinline__ void boys_s(R T, const R* __restrict__ s, R* F) {
-  constexpr int NT = sizeof(R) == 8 ? BOYS_NTAY : 6;
-  if (T < (R)BOYS_TMAX) {
-    const int g = (int)rint(T * (R)BOYS_INV_H);
-    const R d = T - g * (R)BOYS_H;
-    const R* row = s + g * NC;
-    R acc = row[NT - 1];
-#pragma unroll
-    for (int k = NT - 2; k >= 0; --k) acc = fma(acc, -d * ((R)1 / (R)(k + 1)), row[k]);
-    F[M] = acc;
-    if (M > 0) {
-      const R e = exp(-T);
-      const R t2 = T + T;
-#pragma unroll
-      for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * ((R)1 / (R)(2 * m + 1));
-    }
-  } else {
-    const R it = (R)1 / T;
-    F[0] = (R)0.88622692545275801365 * sqrt(it);
-    if (M > 0) {
-      const R e = exp(-T);
-      const R h = (R)0.5 * it;
-#pragma unroll
-      for (int m = 0; m < M; ++m) F[m + 1] = ((R)(2 * m + 1) * F[m] - e) * h;
     }
   }
 }

@@ -144,10 +144,33 @@ std::vector<double> boys_table(int ncol) {
 
 namespace {
 
-// the class kernels' table: BOYS_NGRID rows of BOYS_NCOL orders, then e^-T0 per grid point
-std::vector<double> make_boys_table() {
-  std::vector<double> t = sqb::boys_table(BOYS_NCOL);
-  for (int g = 0; g < BOYS_NGRID; ++g) t.push_back((double)expl(-(long double)g * (long double)BOYS_H));
+// The tables every context uploads, computed once per process: F_m(T0) for the gradient kernels
+// and the row tables of boys<M> and boysf<M> (coefficients F_{M+k}(T0) / k!, then e^-T0).
+struct BoysTables {
+  std::vector<double> plain, rows;
+  std::vector<float> rowsf;
+  BoysTables() : plain(sqb::boys_table(BOYS_NCOL)) {
+    rows.assign((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROW, 0.0);
+    rowsf.assign((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF, 0.0f);
+    for (int M = 0; M <= BOYS_MMAX; ++M)
+      for (int g = 0; g < BOYS_NGRID; ++g) {
+        const size_t r = (size_t)M * BOYS_NGRID + g;
+        double f = 1.0;
+        for (int k = 0; k < BOYS_NTAY; ++k) {
+          if (k > 1) f *= k;
+          const double v = plain[(size_t)g * BOYS_NCOL + M + k] / f;
+          rows[r * BOYS_ROW + k] = v;
+          if (k < 6) rowsf[r * BOYS_ROWF + k] = (float)v;
+        }
+        const double e = (double)expl(-(long double)g * (long double)BOYS_H);
+        rows[r * BOYS_ROW + BOYS_NTAY] = e;
+        rowsf[r * BOYS_ROWF + 6] = (float)e;
+      }
+  }
+};
+
+const BoysTables& boys_tables() {
+  static const BoysTables t;
   return t;
 }
 
@@ -296,8 +319,9 @@ struct sqb200_jk {
   void* d_base = nullptr;       // one allocation holding every buffer below
   void* d_pairbase = nullptr;   // one allocation holding the pair classes' device arrays
   size_t pairbase_bytes = 0;
-  double* d_boys = nullptr;
-  float* d_boysf = nullptr;   // the Boys table in FP32 (mixed-precision forms)
+  double* d_boys = nullptr;   // plain Boys table (gradient)
+  double* d_boysr = nullptr;  // row table of boys<M>
+  float* d_boysf = nullptr;   // FP32 row table (mixed-precision forms)
   int* d_shfirst = nullptr;   // per shell first function
   int* d_shn = nullptr;       // per shell function count
   double *d_PA = nullptr, *d_PB = nullptr, *d_PT = nullptr, *d_PM = nullptr;
@@ -317,21 +341,20 @@ struct sqb200_jk {
     sqb::WorkItem* d_items = nullptr;
     int* d_er = nullptr;          // multipole mode: per item, the error-bank slot of its first ket
     int total = 0;
+    int cta = 64;                 // threads per CTA of the class kernels
     sqb::GenItem* d_gitems = nullptr;   // the generic path's items (shells outside the classes)
     int gtotal = 0;
   };
   // key: outer cutoff, fixed cutoff, FP32 threshold, multipole mode
   std::map<std::tuple<double, double, double, int>, Work> work;
   double fp32_below = 0.0;      // quartets with Schwarz product below this use the FP32 form
-  bool use_ws = true;           // warp-specialised form where a class has one (SQB200_WS=0 disables)
-  std::vector<char> ran_ws;     // per class kernel: which form the last build launched
   std::vector<char> form;       // per class kernel: FP64 form to run, 0 narrow / 1 wide / 2 swapped (autotuner)
   std::vector<char> ran_form;   // per class kernel: the FP64 form the last build launched
   std::vector<long long> last_counts;
   long long last_flops = 0;
   int last_launches = 0;        // kernels enqueued by the last build
   // side streams for concurrent class launches: the build forks them off its stream after the
-  // prologue and joins them before k_finalize (SQB200_STREAMS, default 4; 0 = one stream)
+  // prologue and joins them before k_finalize (SQB200_STREAMS, default 8; 0 = one stream)
   int nside = -1;
   std::vector<cudaStream_t> side;
   cudaEvent_t ev_fork = nullptr;
@@ -779,7 +802,7 @@ int compute_schwarz_device(sqb200_jk* c, double* S_host) {
       }
     const long nthr = (long)pc.pairs.size() * fd.nfn;
     k_schwarz<<<(int)((nthr + 127) / 128), 128, 0, c->stream>>>(pc.d_pairs, pc.d_prims, (int)pc.pairs.size(), pc.stride,
-                                                               kNComp[pc.tb], fd, c->d_boys, c->nbf, dS);
+                                                               kNComp[pc.tb], fd, c->d_boysr, c->nbf, dS);
     CUDA_OK(cudaGetLastError());
   }
   if (c->gen.on) {
@@ -837,24 +860,30 @@ int upload_pairs(sqb200_jk* c) {
   return SQB200_OK;
 }
 
-// Threads per CTA of the class kernels (SQB200_CTA: 32, 64 or 128; default 64).  A work item
-// holds one bra pair and up to (threads / isplit) ket pairs, so narrower CTAs give a small
-// molecule's short ket lists CTAs that are not mostly empty: the registers of a CTA are
-// allocated for all its threads, and an idle warp holds them as long as its CTA lives.
-// Measured on B200: benzene/6-31G* 1080 / 1368 / 1340 builds/s at 128 / 64 / 32 threads;
-// C60/6-31G 73.7 / 73.5 / 74.7 ms per build.
-int cta_threads() {
+// Threads per CTA of the class kernels of a build of `ops` emitted operations (SQB200_CTA: 32, 64 or
+// 128 for every build).  A work item holds one bra pair and as many ket pairs as its CTA's threads
+// take, so narrower CTAs give a small molecule's short ket lists CTAs that are not mostly empty:
+// the registers of a CTA are allocated for all its threads, and an idle warp holds them as long as
+// its CTA lives.  Measured on B200 (ms per build at 64 / 32 threads): benzene/6-31G* 0.82 / 0.73,
+// an organic of 4 heavy atoms in DZP 0.91 / 0.76, of 9 in 6-31G* 1.66 / 1.51; C60/6-31G 73.5 / 74.7.
+int cta_threads(double ops) {
   static const int n = [] {
-    int v = 64;
-    if (const char* e = getenv("SQB200_CTA")) v = atoi(e);
-    return (v == 32 || v == 128) ? v : 64;
+    const char* e = getenv("SQB200_CTA");
+    const int v = e ? atoi(e) : 0;
+    return (v == 32 || v == 64 || v == 128) ? v : 0;
   }();
-  return n;
+  return n ? n : ops < 2e10 ? 32 : 64;
 }
+
+// Side streams of a build (SQB200_STREAMS overrides): a small molecule's class kernels do not fill the
+// GPU alone.  Measured on B200, ms per build with 4 / 8 / 12: a 3-heavy-atom radical UHF/6-31G* 0.32 /
+// 0.27 / 0.25, benzene/6-31G* 0.70 / 0.67 / 0.68, an organic of 9 heavy atoms 1.47 / 1.45 / 1.52 (more
+// kernels side by side on an SM share its instruction cache).
+constexpr int kSideStreams = 8;
 
 int ensure_side_streams(sqb200_jk* c) {
   if (c->nside >= 0) return SQB200_OK;
-  int n = 4;
+  int n = kSideStreams;
   if (const char* e = getenv("SQB200_STREAMS")) n = std::max(0, std::min(16, atoi(e)));
   CUDA_OK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
   for (int i = 0; i < n; ++i) {
@@ -869,13 +898,80 @@ int ensure_side_streams(sqb200_jk* c) {
   return SQB200_OK;
 }
 
+// Emitted FP operations of one thread per primitive step of class K (narrow tile: one pass), plus
+// the step's set-up in the same unit (record loads, reciprocal root, table row: a step of SS|SS,
+// 60 operations, takes about as long as 200).
+double step_ops(const sqb::ClassKernel& K) { return 150.0 + (double)K.flops_prim / K.passes; }
+
+// Threads per quartet of a (nbp bra x nkp ket primitives) run: si over the bra x sj over the ket
+// primitives, at most 32 in all, the fewest whose threads run at most `steps` primitive steps
+// (or, when 32 do not reach that, the split with the shortest loop).  Every thread digests its
+// own partial block, so a split costs a digestion per thread; among splits of one size the one
+// over the bra primitives comes first (a thread flushes once per bra primitive).
+int pick_split(int nbp, int nkp, double steps) {
+  int best = 1 | 1 << 16;
+  long best_loop = (long)nbp * nkp, best_n = 1;
+  if (best_loop <= steps) return best;
+  for (int n = 2; n <= 32; ++n) {
+    if (32 / n * n < 28) continue;               // quartets of n threads fill at least 28 of 32 lanes
+    for (int sj = 1; sj <= n; ++sj) {
+      if (n % sj || sj > nkp || n / sj > nbp) continue;
+      const int si = n / sj;
+      const long loop = (long)((nbp + si - 1) / si) * ((nkp + sj - 1) / sj);
+      // a step of the loop saved has to be worth the added threads
+      if (loop < best_loop && (best_loop > steps) && (double)loop * n <= 1.25 * (double)best_loop * best_n + 0.5) {
+        best = si | sj << 16;
+        best_loop = loop;
+        best_n = n;
+      }
+    }
+  }
+  return best;
+}
+
+// Emitted FP64 operations of a build's class-kernel quartets (the Schwarz survivors): per class
+// and pair of sub-lists the survivors by a two-pointer walk of the sorted bounds.
+double build_ops(const sqb200_jk* c, double outer, double fixed) {
+  const double cut = std::max(outer, fixed);
+  double ops = 0.0;
+  for (int ki = 0; ki < sqb::kNumClassKernels; ++ki) {
+    const sqb::ClassKernel& K = sqb::kClassKernels[ki];
+    const PairClass& B = c->cls[K.bra_cls];
+    const PairClass& T = c->cls[K.ket_cls];
+    if (B.pairs.empty() || T.pairs.empty()) continue;
+    const bool same = K.bra_cls == K.ket_cls;
+    for (size_t sx = 0; sx + 1 < B.sub.size(); ++sx)
+      for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
+        const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0 = T.sub[sy];
+        int end = T.sub[sy + 1];
+        double n = 0.0;
+        for (int b = b0; b < b1; ++b) {
+          while (end > k0 && T.pairs[end - 1].schwarz * B.pairs[b].schwarz < cut) --end;
+          n += std::max(0, end - (same && sx == sy ? b : k0));
+        }
+        ops += n * ((double)B.pairs[b0].nprim * T.pairs[k0].nprim * K.flops_prim + K.flops_quartet);
+      }
+  }
+  return ops;
+}
+
+// The longest run of operations a thread of a build of `ops` emitted operations is given.  A
+// build that fills the GPU for milliseconds leaves its quartets whole: each split thread digests
+// its own partial block, atomics included.  A small molecule's build is as long as its longest
+// thread, so its quartets are split, down to a few primitive steps; splitting further costs more
+// in digestion than the shorter chain saves.  Measured on B200 (ms per build, narrow forms, least
+// run / factor): a 3-heavy-atom radical UHF/6-31G* 0.25 / 0.23 / 0.25 at a least run of 1500 / 3000 /
+// 6000; benzene/6-31G* 1.31 / 1.14 / 0.79 / 0.70 at factors 0.5, 1, 2 and 4e-6, an organic of 9 heavy
+// atoms 2.08 / 1.87 / 1.48 / 1.47; C60/6-31G the same whether its quartets are split or not.
+double chain_ops(double ops) { return std::max(3000.0, 4e-6 * ops); }
+
 // Work items of class kernel ki for one molecule (context c): every surviving (bra pair, <=kper
 // ket pairs) unit, with pair indices shifted by bra_base/ket_base (the molecule's first pair in
 // a merged class array; 0 for a single-molecule build).  Kets whose Schwarz product is below the
 // context's fp32_below go to items32 (the FP32 form).  cost64/cost32 accumulate the emitted
 // operations, the launch-order and stream-balancing estimate.
 void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra_base, int ket_base, int mol,
-                 std::vector<sqb::WorkItem>& items, std::vector<sqb::WorkItem>& items32, double& cost64,
+                 double chain, int cta, std::vector<sqb::WorkItem>& items, std::vector<sqb::WorkItem>& items32, double& cost64,
                  double& cost32, std::vector<int>* ers = nullptr, long long* er_run = nullptr,
                  bool allow_f32 = true) {
   const sqb::ClassKernel& K = sqb::kClassKernels[ki];
@@ -896,12 +992,9 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
       if (same && sx > sy) continue;
       const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0s = T.sub[sy], k1s = T.sub[sy + 1];
       const int nbp = B.pairs[b0].nprim, nkp = T.pairs[k0s].nprim;
-      // split the bra primitives over up to 32 threads when a quartet has many primitives
-      // (the warp-specialised form takes 32 kets per CTA, one lane each)
-      const bool ws = c->use_ws && K.ws_r != nullptr;
-      int isplit = 1;
-      while (!ws && !mpm && isplit * 2 <= nbp && isplit * 2 <= 32 && (long)nbp * nkp / (isplit * 2) >= 32) isplit *= 2;
-      const int kper = ws ? 32 : cta_threads() / isplit;
+      // multipole mode needs each quartet's whole block in one thread
+      const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K));
+      const int kper = cta / ((split & 0xffff) * (split >> 16));
       const double pq = (double)nbp * nkp;
       for (int b = b0; b < b1; ++b) {
         const double sb = B.pairs[b].schwarz;
@@ -939,11 +1032,11 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
           mid = l2;
         }
         for (int k0 = start; k0 < mid; k0 += kper) {
-          items.push_back({bra_base + b, ket_base + k0, std::min(kper, mid - k0), isplit, mol});
+          items.push_back({bra_base + b, ket_base + k0, std::min(kper, mid - k0), split, mol});
           if (mpm) ers->push_back((int)(er0 + (k0 - start)));
         }
         for (int k0 = std::max(start, mid); k0 < end; k0 += kper)
-          items32.push_back({bra_base + b, ket_base + k0, std::min(kper, end - k0), isplit, mol});
+          items32.push_back({bra_base + b, ket_base + k0, std::min(kper, end - k0), split, mol});
         cost64 += std::max(0, mid - start) * (pq * K.flops_prim + K.flops_quartet);
         cost32 += std::max(0, end - std::max(start, mid)) * (pq * K.f32_flops_prim + K.f32_flops_quartet);
       }
@@ -951,7 +1044,7 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
 }
 
 // Launch order inside one class kernel: the CTAs with the longest primitive loop first (a
-// thread runs ceil(bra primitives / isplit) x ket primitives iterations; more kets per item next),
+// thread runs ceil(bra primitives / si) x ceil(ket primitives / sj) iterations; more kets per item next),
 // so that a launch does not end on a few long CTAs while the rest of the GPU idles.
 // nprims(item) gives the item's (bra, ket) primitive counts.
 template <class F>
@@ -961,7 +1054,8 @@ void sort_heavy_first(std::vector<sqb::WorkItem>& v, size_t first, F nprims) {
   for (size_t i = 0; i < n; ++i) {
     const sqb::WorkItem& it = v[first + i];
     const std::pair<int, int> np = nprims(it);
-    const long long loop = (long long)((np.first + it.isplit - 1) / it.isplit) * np.second;
+    const int si = it.split & 0xffff, sj = it.split >> 16;
+    const long long loop = (long long)((np.first + si - 1) / si) * ((np.second + sj - 1) / sj);
     key[i] = {-(loop * 4096 + it.cnt), i};
   }
   std::stable_sort(key.begin(), key.end());
@@ -999,17 +1093,19 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
   std::vector<sqb::WorkItem> items, items32;
   std::vector<int> ers;
   long long er_run = 0;
+  const double ops = build_ops(c, outer, fixed), chain = chain_ops(ops);
+  w.cta = cta_threads(ops);
   for (int ki = 0; ki < sqb::kNumClassKernels; ++ki) {
     const int first = (int)items.size();
     items32.clear();
     double cost64 = 0.0, cost32 = 0.0;
-    class_items(c, ki, outer, fixed, 0, 0, 0, items, items32, cost64, cost32, mpm ? &ers : nullptr,
+    class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, cost64, cost32, mpm ? &ers : nullptr,
                 mpm ? &er_run : nullptr);
     if (too_few_f32(items32)) {
       items.resize(first);
       items32.clear();
       cost64 = cost32 = 0.0;
-      class_items(c, ki, outer, fixed, 0, 0, 0, items, items32, cost64, cost32, nullptr, nullptr, false);
+      class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, cost64, cost32, nullptr, nullptr, false);
     }
     if (!mpm) {   // (multipole mode keeps the items with their bank slots in generation order)
       const PairClass& B = c->cls[sqb::kClassKernels[ki].bra_cls];
@@ -1104,16 +1200,6 @@ int pick_form(const sqb::ClassKernel& K, bool f32, int uhf, int form, const void
   return 0;
 }
 
-// Shared-memory accumulators of the wide form: the region follows the staged bra primitives.
-// The kernels index it thread-fastest with a stride of 128 threads, whatever the CTA width.
-void add_acc_region(const sqb::ClassKernel& K, int form_used, SegLaunch& L) {
-  const int dbl = form_used == 1 ? K.w_o_dbl : form_used == 2 ? K.s_o_dbl : 0;
-  if (dbl <= 0) return;
-  const size_t off = (L.smem + 15) / 16 * 16;
-  L.a.so_off = (int)(off / sizeof(double));
-  L.smem = off + (size_t)dbl * 128 * sizeof(double);
-}
-
 // Raise a kernel's dynamic shared-memory limit once per (device, kernel, size class), so that a
 // build captured into a CUDA graph after a first uncaptured build issues only stream work.
 int ensure_smem(const void* fn, size_t smem) {
@@ -1194,7 +1280,7 @@ SegLaunch seg_single(sqb200_jk* c, const sqb200_jk::Work* w, size_t s, const dou
   a.ket_pairs = T.d_pairs; a.ket_prims = T.d_prims;
   a.PA = dPA; a.PB = dPB; a.PT = c->d_PT; a.PM = c->d_PM;
   a.Jacc = c->d_J; a.KAacc = c->d_KA; a.KBacc = c->d_KB;
-  a.boys_tab = c->d_boys;
+  a.boys_tab = c->d_boysr;
   a.boys_tab_f = c->d_boysf;
   a.counters = c->d_counters + 4 * v;
   a.bra_prims_f = B.d_primsf; a.ket_prims_f = T.d_primsf;
@@ -1210,21 +1296,13 @@ SegLaunch seg_single(sqb200_jk* c, const sqb200_jk::Work* w, size_t s, const dou
     a.mp_rmax = c->mp_rmax;
     form = 0;                              // the narrow form carries the multipole mode
   }
-  const bool ws = !f32 && !c->mp_on && c->use_ws && K.ws_r != nullptr;
-  if (!f32) c->ran_ws[kidx] = ws;
-  L.smem = (size_t)B.max_nprim * B.stride * (f32 ? sizeof(float) : sizeof(double)) +
-           (ws ? (size_t)K.ws_warps * K.ws_nr * 32 * sizeof(double) : 0);
+  L.smem = (size_t)B.max_nprim * B.stride * (f32 ? sizeof(float) : sizeof(double));
   int passes = 1;
-  if (ws) {
-    L.fn = uhf ? K.ws_u : K.ws_r;
-  } else {
-    const int fu = pick_form(K, f32, uhf, form < 0 ? c->form[kidx] : form, &L.fn, &passes);
-    if (!f32) c->ran_form[kidx] = (char)fu;
-    add_acc_region(K, fu, L);
-  }
+  const int fu = pick_form(K, f32, uhf, form < 0 ? c->form[kidx] : form, &L.fn, &passes);
+  if (!f32) c->ran_form[kidx] = (char)fu;
   L.grid = dim3(w->count[s], passes);
-  L.block = dim3(ws ? 32 * K.ws_warps : cta_threads());
-  if (c->persistent && !ws) make_persistent(L, c->d_queue + v);
+  L.block = dim3(w->cta);
+  if (c->persistent) make_persistent(L, c->d_queue + v);
   return L;
 }
 
@@ -1449,11 +1527,8 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   CUDA_OK(cudaSetDevice(device));
   sqb200_jk* c = new sqb200_jk();
   c->device = device;
-  const char* ws_env = getenv("SQB200_WS");
-  c->use_ws = !(ws_env && ws_env[0] == '0');
   const char* pe = getenv("SQB200_PERSISTENT");
   c->persistent = pe && pe[0] == '1';
-  c->ran_ws.assign(sqb::kNumClassKernels, 0);
   c->form.assign(sqb::kNumClassKernels, 0);
   c->ran_form.assign(sqb::kNumClassKernels, 0);
   c->nbf = nbf;
@@ -1467,12 +1542,13 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   if (!rc) rc = setup_generic(c);
   if (rc) { sqb200_jk_destroy(c); return rc; }
   const size_t nn = (size_t)nbf * nbf;
-  std::vector<double> tab = make_boys_table();
+  const BoysTables& bt = boys_tables();
   std::vector<int> fst(c->ns), nf(c->ns);
   for (int s = 0; s < c->ns; ++s) { fst[s] = c->shells[s].first; nf[s] = c->shells[s].nfunc; }
   Carve cv;
-  cv.add(&c->d_boys, tab.size() * sizeof(double));
-  cv.add(&c->d_boysf, tab.size() * sizeof(float));
+  cv.add(&c->d_boys, bt.plain.size() * sizeof(double));
+  cv.add(&c->d_boysr, bt.rows.size() * sizeof(double));
+  cv.add(&c->d_boysf, bt.rowsf.size() * sizeof(float));
   cv.add(&c->d_shfirst, c->ns * sizeof(int));
   cv.add(&c->d_shn, c->ns * sizeof(int));
   for (double** m : {&c->d_PA, &c->d_PB, &c->d_PT, &c->d_J, &c->d_KA, &c->d_KB, &c->d_JT, &c->d_KAo, &c->d_KBo})
@@ -1487,9 +1563,9 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
     return fail(SQB200_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = h2d(c->d_boys, tab.data(), tab.size() * sizeof(double), c->stream);
-  std::vector<float> tabf(tab.begin(), tab.end());
-  if (e == cudaSuccess) e = h2d(c->d_boysf, tabf.data(), tabf.size() * sizeof(float), c->stream);
+  if (e == cudaSuccess) e = h2d(c->d_boys, bt.plain.data(), bt.plain.size() * sizeof(double), c->stream);
+  if (e == cudaSuccess) e = h2d(c->d_boysr, bt.rows.data(), bt.rows.size() * sizeof(double), c->stream);
+  if (e == cudaSuccess) e = h2d(c->d_boysf, bt.rowsf.data(), bt.rowsf.size() * sizeof(float), c->stream);
   if (e == cudaSuccess) e = h2d(c->d_shfirst, fst.data(), c->ns * sizeof(int), c->stream);
   if (e == cudaSuccess) e = h2d(c->d_shn, nf.data(), c->ns * sizeof(int), c->stream);
   if (e != cudaSuccess) { sqb200_jk_destroy(c); return fail(SQB200_ECUDA, cudaGetErrorString(e)); }
@@ -1722,7 +1798,7 @@ int sqb200_boys_eval(int device, int mmax, int n, const double* T, double* F) {
   for (int i = 0; i < n; ++i)
     if (!(T[i] >= 0.0)) return fail(SQB200_EINVAL, "sqb200_boys_eval: T must be >= 0");
   CUDA_OK(cudaSetDevice(device));
-  const std::vector<double> tab = make_boys_table();
+  const std::vector<double>& tab = boys_tables().rows;
   double *dT = nullptr, *dF = nullptr, *dtab = nullptr;
   const size_t nf = (size_t)n * (mmax + 1);
   cudaError_t e = cudaMalloc(&dT, n * sizeof(double));
@@ -1907,7 +1983,7 @@ void noalloc_items(const sqb200_jk* c, double outer, double fixed, std::vector<s
             if (T.pairs[mid].schwarz >= thr) lo = mid + 1; else hi = mid;
           }
           const int start = (same && sx == sy) ? b : k0s;
-          for (int k0 = start; k0 < lo; k0 += kper) items.push_back({b, k0, std::min(kper, lo - k0), isplit, 0});
+          for (int k0 = start; k0 < lo; k0 += kper) items.push_back({b, k0, std::min(kper, lo - k0), isplit | 1 << 16, 0});
         }
       }
     if ((int)items.size() > f0) {
@@ -1969,7 +2045,7 @@ extern "C" int sqb200_jk_build_noalloc(sqb200_jk* c, const double* dPA, const do
     a.ket_pairs = T.d_pairs; a.ket_prims = T.d_prims;
     a.PA = dPA; a.PB = dPB; a.PT = PT; a.PM = PM;
     a.Jacc = J; a.KAacc = KA; a.KBacc = KB;
-    a.boys_tab = c->d_boys;
+    a.boys_tab = c->d_boysr;
     a.counters = counters + 4 * kernel[s];
     a.mols = d_mol;
     a.same_class = K.bra_cls == K.ket_cls;
@@ -2025,7 +2101,7 @@ extern "C" int sqb200_oneint(sqb200_jk* c, int natom, const double* Z, const dou
   cudaError_t e = up.upload(&base, c->stream);
   if (e == cudaSuccess) {
     k_oneint<<<(int)((nn + 127) / 128), 128, 0, c->stream>>>(n, d_np, d_off, d_lmn, d_xyz, d_ex, d_nc, natom, d_Z, d_A,
-                                                              c->d_boys, d_out, d_out + nn, d_out + 2 * nn);
+                                                              c->d_boysr, d_out, d_out + nn, d_out + 2 * nn);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(S, d_out, nn * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -2072,6 +2148,7 @@ struct sqb200_batch {
   size_t items_cap = 0;
   bool have_step = false;
   std::vector<unsigned long long> last_counts;
+  int cta = 64;                         // threads per CTA of the class kernels
   std::vector<char> form;               // per class kernel: FP64 form (sqb200_batch_autotune)
   int last_launches = 0;
   int nside = -1;
@@ -2260,6 +2337,10 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
   b->kernel.clear(); b->spin.clear(); b->first.clear(); b->count.clear(); b->cost.clear();
   std::vector<sqb::WorkItem> items, items32;
   const int K_ = sqb::kNumClassKernels;
+  double ops = 0.0;
+  for (int m = 0; m < b->nmol; ++m) ops += build_ops(b->mols[m], scf_cutoff[m], fixed_cutoff[m]);
+  const double chain = chain_ops(ops);
+  b->cta = cta_threads(ops);
   for (int sp = 0; sp < 2; ++sp)
     for (int ki = 0; ki < K_; ++ki) {
       const sqb::ClassKernel& K = sqb::kClassKernels[ki];
@@ -2277,7 +2358,7 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
         if (b->rec[m].uhf != sp) continue;
         const size_t a64 = items.size(), a32 = items32.size();
         class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
-                    b->cls[K.ket_cls].pair_base[m], m, items, items32, c64, c32);
+                    b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32);
         sort_heavy_first(items, a64, np);
         sort_heavy_first(items32, a32, np);
       }
@@ -2289,7 +2370,8 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
           if (b->rec[m].uhf != sp) continue;
           const size_t a64 = items.size();
           class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
-                      b->cls[K.ket_cls].pair_base[m], m, items, items32, c64, c32, nullptr, nullptr, false);
+                      b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32, nullptr, nullptr,
+                      false);
           sort_heavy_first(items, a64, np);
         }
       }
@@ -2335,7 +2417,7 @@ SegLaunch seg_batch(sqb200_batch* b, size_t s, const double* dPA, const double* 
   a.bra_prims_f = B.d_primsf; a.ket_prims_f = T.d_primsf;
   a.PA = dPA; a.PB = dPB; a.PT = b->d_PT; a.PM = b->d_PM;
   a.Jacc = b->d_J; a.KAacc = b->d_KA; a.KBacc = b->d_KB;
-  a.boys_tab = b->mols[0]->d_boys;
+  a.boys_tab = b->mols[0]->d_boysr;
   a.boys_tab_f = b->mols[0]->d_boysf;
   a.counters = b->d_counters + 4 * (uhf * 2 * K_ + v);
   a.mols = b->d_mols;
@@ -2345,8 +2427,7 @@ SegLaunch seg_batch(sqb200_batch* b, size_t s, const double* dPA, const double* 
   int passes = 1;
   const int fu = pick_form(K, f32, uhf, form < 0 ? b->form[kidx] : form, &L.fn, &passes);
   L.grid = dim3(b->count[s], passes);
-  L.block = dim3(cta_threads());
-  add_acc_region(K, fu, L);
+  L.block = dim3(b->cta);
   if (b->persistent) make_persistent(L, b->d_queue + uhf * 2 * K_ + v);
   return L;
 }
@@ -2405,7 +2486,7 @@ extern "C" int sqb200_batch_build_device(sqb200_batch* b, const double* dPA, con
   CUDA_OK(cudaMemsetAsync(b->d_counters, 0, 2 * 8 * K_ * sizeof(unsigned long long), st));
   if (b->persistent) CUDA_OK(cudaMemsetAsync(b->d_queue, 0, 2 * 2 * K_ * sizeof(unsigned long long), st));
   if (b->nside < 0) {
-    int n = 4;
+    int n = kSideStreams;
     if (const char* e = getenv("SQB200_STREAMS")) n = std::max(0, std::min(16, atoi(e)));
     CUDA_OK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
     for (int i = 0; i < n; ++i) {

@@ -18,12 +18,6 @@ struct ClassKernel {
   int flops_prim;         // FP64 ops per primitive quartet as emitted (all passes, repeats included)
   int flops_flush;        // FP64 ops per bra primitive and ket pair (all passes)
   int flops_quartet;      // FP64 ops of one digestion (all passes) of a (partial) quartet block
-  // warp-specialised form (null when the class has one pass or its R buffer does not fit):
-  // one CTA of 32*ws_warps threads = all passes of 32 quartets, R staged in shared memory
-  int ws_warps, ws_nr;
-  const void* ws_r;
-  const void* ws_u;
-  int ws_flops_prim, ws_flops_flush, ws_flops_quartet;
   // mixed form (FP32 Hermite integrals and contraction, FP64 Boys/setup/accumulation); null
   // for the classes of highest angular momentum, whose small quartets stay in FP64
   int passes32;
@@ -39,7 +33,6 @@ struct ClassKernel {
   const void* fn_rw;
   const void* fn_uw;
   int w_flops_prim, w_flops_flush, w_flops_quartet;
-  int w_o_dbl;            // doubles per thread of the wide form's shared-memory accumulators (0: registers)
   // swapped-role FP64 form: outer loop over the thread's ket primitives (global, once per
   // pass), inner loop over the shared bra primitives (shared memory); passes split the bra
   // functions; its flush counter counts ket primitives
@@ -47,7 +40,6 @@ struct ClassKernel {
   const void* fn_rs;
   const void* fn_us;
   int s_flops_prim, s_flops_flush, s_flops_quartet;
-  int s_o_dbl;            // doubles per thread of the swapped form's shared-memory accumulators (0: registers)
 };
 
 extern const ClassKernel kClassKernels[];
