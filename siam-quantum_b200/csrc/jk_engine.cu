@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "jk_common.cuh"
+#include "grad_common.cuh"
 #include "jk_generic.cuh"
 #include "jk_registry.h"
 #include "../../include/sqb200.h"
@@ -150,9 +151,9 @@ struct BoysTables {
   std::vector<double> plain, rows;
   std::vector<float> rowsf;
   BoysTables() : plain(sqb::boys_table(BOYS_NCOL)) {
-    rows.assign((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROW, 0.0);
+    rows.assign((size_t)(BOYS_MMAX + 2) * BOYS_NGRID * BOYS_ROW, 0.0);   // one order more: the gradient
     rowsf.assign((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF, 0.0f);
-    for (int M = 0; M <= BOYS_MMAX; ++M)
+    for (int M = 0; M <= BOYS_MMAX + 1; ++M)
       for (int g = 0; g < BOYS_NGRID; ++g) {
         const size_t r = (size_t)M * BOYS_NGRID + g;
         double f = 1.0;
@@ -160,11 +161,11 @@ struct BoysTables {
           if (k > 1) f *= k;
           const double v = plain[(size_t)g * BOYS_NCOL + M + k] / f;
           rows[r * BOYS_ROW + k] = v;
-          if (k < 6) rowsf[r * BOYS_ROWF + k] = (float)v;
+          if (k < 6 && M <= BOYS_MMAX) rowsf[r * BOYS_ROWF + k] = (float)v;
         }
         const double e = (double)expl(-(long double)g * (long double)BOYS_H);
         rows[r * BOYS_ROW + BOYS_NTAY] = e;
-        rowsf[r * BOYS_ROWF + 6] = (float)e;
+        if (M <= BOYS_MMAX) rowsf[r * BOYS_ROWF + 6] = (float)e;
       }
   }
 };
@@ -3041,6 +3042,163 @@ __global__ void k_grad_1e(int nbf, const int* __restrict__ nprim, const int* __r
 
 }  // namespace
 
+namespace {
+
+constexpr int kGradCta = 64;       // threads per CTA of the gradient class kernels
+constexpr int kGradCopies = 64;    // copies of the gradient the CTAs add into (3 natom addresses would collide)
+
+// grad[x] += the sum of its copies, one thread per component.
+__global__ void k_grad_sum(const double* __restrict__ copies, int ncopy, int stride, int n, double* __restrict__ grad) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  double s = 0.0;
+  for (int k = 0; k < ncopy; ++k) s += copies[(size_t)k * stride + x];
+  grad[x] += s;
+}
+
+// The gradient's pair lists and work items of one call (shells of the class kernels only).
+struct GradWork {
+  struct Cls {
+    std::vector<sqb::GradPair> pairs;
+    std::vector<double> prims;
+    std::vector<int> sub;          // starts of the runs of equal primitive count, and the end
+    int max_nprim = 0;
+    void *d_pairs = nullptr, *d_prims = nullptr;
+  } cls[sqb::kNumPairClasses];
+  struct Seg { int k; size_t first, count; double cost; };
+  std::vector<sqb::WorkItem> items;
+  std::vector<Seg> segs;
+  void* d_items = nullptr;
+};
+
+// Pair records (layout as build_pairs: a run's pairs side by side, field by field) in each run by
+// falling Schwarz x density bound, so that the kets that pass the shell screen with one bra
+// pair are a prefix; then the items of every class, heaviest segment first.
+void grad_work(const sqb200_jk* c, const int* fat, const double* PT, double screen, GradWork& w) {
+  const int n = c->nbf;
+  for (int k = 0; k < sqb::kNumPairClasses; ++k) {
+    const PairClass& pc = c->cls[k];
+    GradWork::Cls& g = w.cls[k];
+    g.sub = pc.sub;
+    g.max_nprim = pc.max_nprim;
+    for (size_t r = 0; r + 1 < pc.sub.size(); ++r) {
+      const int l0 = pc.sub[r], S = pc.sub[r + 1] - l0;
+      std::vector<sqb::GradPair> run(S);
+      for (int l = 0; l < S; ++l) {
+        const sqb::PairRec& rec = pc.pairs[l0 + l];
+        const Shell &A = c->shells[rec.P], &B = c->shells[rec.Q];
+        double pm = 0.0;
+        for (int p = 0; p < A.nfunc; ++p)
+          for (int q = 0; q < B.nfunc; ++q) pm = std::max(pm, fabs(PT[(size_t)(A.first + p) * n + B.first + q]));
+        run[l] = {rec.P, rec.Q, A.first, B.first, rec.nprim, 0, S, fat[A.first], fat[B.first], 0, rec.schwarz, pm};
+      }
+      std::stable_sort(run.begin(), run.end(),
+                       [](const sqb::GradPair& x, const sqb::GradPair& y) { return x.sch * x.pm > y.sch * y.pm; });
+      const size_t base = g.prims.size();
+      const int nf = 15 + c->shells[run[0].P].nfunc + c->shells[run[0].Q].nfunc;
+      g.prims.resize(base + (size_t)S * run[0].nprim * nf);
+      for (int l = 0; l < S; ++l) {
+        sqb::GradPair& t = run[l];
+        t.poff = (int)(base + l);
+        const Shell &A = c->shells[t.P], &B = c->shells[t.Q];
+        const double ra[3] = {A.x, A.y, A.z}, rb[3] = {B.x, B.y, B.z};
+        double ab2 = 0.0;
+        for (int d = 0; d < 3; ++d) ab2 += (ra[d] - rb[d]) * (ra[d] - rb[d]);
+        for (int i = 0; i < A.nprim; ++i)
+          for (int j = 0; j < B.nprim; ++j) {
+            double* f = g.prims.data() + base + l + (size_t)(i * B.nprim + j) * nf * S;
+            const double a = A.exps[i], b = B.exps[j], p = a + b;
+            f[0] = p;
+            f[(size_t)4 * S] = exp(-a * b / p * ab2) / p;
+            f[(size_t)5 * S] = a / p;
+            for (int d = 0; d < 3; ++d) {
+              const double P = (a * ra[d] + b * rb[d]) / p;
+              f[(size_t)(1 + d) * S] = P;
+              f[(size_t)(6 + d) * S] = P - ra[d];
+              f[(size_t)(9 + d) * S] = P - rb[d];
+              f[(size_t)(12 + d) * S] = 2.0 * a * b / p * (ra[d] - rb[d]);
+            }
+            for (int x = 0; x < A.nfunc; ++x) f[(size_t)(15 + x) * S] = A.coef[i][x];
+            for (int x = 0; x < B.nfunc; ++x) f[(size_t)(15 + A.nfunc + x) * S] = B.coef[j][x];
+          }
+        g.pairs.push_back(t);
+      }
+    }
+  }
+  // two passes over the same ranges: the work of the call, then its items (quartets are split
+  // over threads as the J/K builds' are)
+  double chain = 0.0, total = 0.0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int gk = 0; gk < sqb::kNumGradKernels; ++gk) {
+      const sqb::GradKernel& K = sqb::kGradKernels[gk];
+      const GradWork::Cls &B = w.cls[K.bra_cls], &T = w.cls[K.ket_cls];
+      if (B.pairs.empty() || T.pairs.empty()) continue;
+      const bool same = K.bra_cls == K.ket_cls;
+      const size_t first = w.items.size();
+      double cost = 0.0;
+      for (size_t sx = 0; sx + 1 < B.sub.size(); ++sx)
+        for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
+          const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
+          const int split = pass ? pick_split(nbp, nkp, chain / K.ops) : 0;
+          const int kper = pass ? kGradCta / ((split & 0xffff) * (split >> 16)) : 0;
+          int end = T.sub[sy + 1];
+          for (int b = B.sub[sx]; b < B.sub[sx + 1]; ++b) {
+            const double sb = B.pairs[b].sch * B.pairs[b].pm;
+            while (end > T.sub[sy] && T.pairs[end - 1].sch * T.pairs[end - 1].pm * sb < screen * (1.0 - 1e-12)) --end;
+            const int start = same && sx == sy ? b : T.sub[sy];
+            cost += (double)std::max(0, end - start) * nbp * nkp * K.passes * K.ops;
+            if (pass)
+              for (int k0 = start; k0 < end; k0 += kper) w.items.push_back({b, k0, std::min(kper, end - k0), split, 0});
+          }
+        }
+      total += cost;
+      if (pass && w.items.size() > first) {
+        sort_heavy_first(w.items, first, [&](const sqb::WorkItem& it) {
+          return std::make_pair(B.pairs[it.bra].nprim, T.pairs[it.k0].nprim);
+        });
+        w.segs.push_back({gk, first, w.items.size() - first, cost});
+      }
+    }
+    if (!pass) chain = chain_ops(total);
+  }
+  std::stable_sort(w.segs.begin(), w.segs.end(), [](const GradWork::Seg& x, const GradWork::Seg& y) { return x.cost > y.cost; });
+}
+
+// The class kernels on the context's streams (forked off c->stream and joined to it, as a
+// build's), each with its CTAs' bra records in at most 32 KB of shared memory at a time.
+int grad_launch(sqb200_jk* c, const GradWork& w, sqb::GradArgs a) {
+  int rc = ensure_side_streams(c);
+  if (rc) return rc;
+  const int nl = 1 + c->nside;
+  std::vector<double> load(nl, 0.0);
+  if (nl > 1) {
+    CUDA_OK(cudaEventRecord(c->ev_fork, c->stream));
+    for (int l = 1; l < nl; ++l) CUDA_OK(cudaStreamWaitEvent(c->side[l - 1], c->ev_fork, 0));
+  }
+  for (const GradWork::Seg& s : w.segs) {
+    const sqb::GradKernel& K = sqb::kGradKernels[s.k];
+    const int lane = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[lane] += s.cost;
+    const GradWork::Cls &B = w.cls[K.bra_cls], &T = w.cls[K.ket_cls];
+    a.bra_pairs = (const sqb::GradPair*)B.d_pairs; a.bra_prims = (const double*)B.d_prims;
+    a.ket_pairs = (const sqb::GradPair*)T.d_pairs; a.ket_prims = (const double*)T.d_prims;
+    a.same_class = K.bra_cls == K.ket_cls;
+    const size_t rec = (size_t)K.nb * sizeof(double);
+    a.chunk = std::min(B.max_nprim, std::max(1, (int)(32 * 1024 / rec)));
+    const sqb::WorkItem* items = (const sqb::WorkItem*)w.d_items + s.first;
+    void* args[] = {&a, &items};
+    CUDA_OK(cudaLaunchKernel(K.fn, dim3((unsigned)s.count, K.passes), dim3(kGradCta), args, a.chunk * rec,
+                             lane == 0 ? c->stream : c->side[lane - 1]));
+  }
+  for (int l = 1; l < nl; ++l) {
+    CUDA_OK(cudaEventRecord(c->ev_join[l - 1], c->side[l - 1]));
+    CUDA_OK(cudaStreamWaitEvent(c->stream, c->ev_join[l - 1], 0));
+  }
+  return SQB200_OK;
+}
+
+}  // namespace
+
 extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, const double* axyz,
                                      const double* PA, const double* PB, const double* W, int terms, double* grad) {
   if (!c || natom <= 0 || !Z || !axyz || !PA || !PB || !W || !grad) return fail(SQB200_EINVAL, "null argument");
@@ -3146,6 +3304,13 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
     return fail(SQB200_EINVAL, "sqb200_gradient: too many atoms (" + std::to_string(natom) + ") for the per-block sums");
   std::vector<double> PT(nn), PS(nn);
   for (size_t i = 0; i < nn; ++i) { PT[i] = PA[i] + PB[i]; PS[i] = PA[i] - PB[i]; }
+  // every shell in a class: the generated kernels; a basis with f shells (or another layout): one
+  // thread per shell quartet with run-time loops
+  const bool classes = !c->gen.on;
+  GradWork gw;
+  if ((terms & SQB200_GRAD_ERI) && classes) grad_work(c, fat.data(), PT.data(), screen, gw);
+  const int gstride = (3 * natom + 15) / 16 * 16;
+  void* dcopies = nullptr;
   void* d[16] = {nullptr};
   void *dp = nullptr, *dsch = nullptr, *dpm = nullptr, *dg = nullptr;
   Staged up;
@@ -3167,13 +3332,36 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
   up.put(&dp, npairs * sizeof(int2), pairs.data());
   up.put(&dsch, npairs * sizeof(double), psch.data());
   up.put(&dpm, npairs * sizeof(double), ppm.data());
+  for (GradWork::Cls& g : gw.cls) {
+    up.put(&g.d_pairs, g.pairs.size() * sizeof(sqb::GradPair), g.pairs.data());
+    up.put(&g.d_prims, g.prims.size() * sizeof(double), g.prims.data());
+  }
+  up.put(&gw.d_items, gw.items.size() * sizeof(sqb::WorkItem), gw.items.data());
   up.put(&dg, 3 * natom * sizeof(double), nullptr);
+  up.put(&dcopies, (size_t)kGradCopies * gstride * sizeof(double), nullptr);
   void* base = nullptr;
   cudaError_t e = up.upload(&base, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, 3 * natom * sizeof(double), c->stream);
   if (e == cudaSuccess) {
     const dim3 geri((npairs + 127) / 128, npairs);
-    if ((terms & SQB200_GRAD_ERI) && fgrad)
+    if ((terms & SQB200_GRAD_ERI) && classes) {
+      e = cudaMemsetAsync(dcopies, 0, (size_t)kGradCopies * gstride * sizeof(double), c->stream);
+      sqb::GradArgs ga;
+      memset(&ga, 0, sizeof(ga));
+      ga.PT = (const double*)d[9]; ga.PS = (const double*)d[10];
+      ga.boys_tab = c->d_boysr;
+      ga.grad = (double*)dcopies;
+      ga.screen = screen;
+      ga.nbf = n; ga.ncopy = kGradCopies; ga.stride = gstride;
+      const int rc = grad_launch(c, gw, ga);
+      if (rc) {
+        cudaDeviceSynchronize();           // kernels in flight read the buffers freed here
+        cudaFree(base);
+        return rc;
+      }
+      k_grad_sum<<<(3 * natom + 127) / 128, 128, 0, c->stream>>>((const double*)dcopies, kGradCopies, gstride, 3 * natom,
+                                                                  (double*)dg);
+    } else if ((terms & SQB200_GRAD_ERI) && fgrad)
       k_grad_eri<3><<<geri, 128, smem_eri, c->stream>>>(
           npairs, (const int2*)dp, (const double*)dsch, (const double*)dpm, (const GShell*)d[12], (const double*)d[13],
           (const double*)d[14], (const double*)d[9], (const double*)d[10], n, btab, bcol, screen, natom, (double*)dg);

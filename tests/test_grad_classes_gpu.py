@@ -1,0 +1,48 @@
+"""The generated class kernels of the two-electron gradient against the run-time kernel (one thread
+per shell quartet): a basis with every shell type takes the class kernels; the same basis with
+the functions of one d shell in another order is a layout outside the classes and takes the
+run-time kernel.  Both apply the same screens to the same quartets, so they differ by rounding:
+tolerance 1e-11 of the largest component.  Restricted and unrestricted densities (the gradient's
+spin term), screened and with every quartet kept; contraction lengths with remainders, shells
+sharing a centre (same-shell and same-pair degeneracies)."""
+import numpy as np
+import pytest
+
+from conftest import load_sqb200
+from test_split_gpu import _basis
+
+SHELLS = [("S", 0, 5), ("L", 0, 3), ("P", 1, 2), ("D", 2, 2), ("D", 0, 1), ("L", 1, 1), ("S", 2, 1), ("P", 2, 1)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells", [SHELLS, SHELLS[:1] + SHELLS[3:5], [("S", 0, 7), ("S", 1, 1), ("S", 2, 2), ("D", 1, 1)]],
+                         ids=["all", "s_d", "s"])
+@pytest.mark.parametrize("screen", ["1e-10", "0"])
+@pytest.mark.parametrize("restricted", [True, False])
+def test_class_gradient_matches_run_time_kernel(shells, screen, restricted, monkeypatch):
+    monkeypatch.setenv("SQB200_GRAD_SCREEN", screen)
+    sqb = load_sqb200()
+    b = _basis(sqb, shells, 7)
+    n = b.nbf
+    rng = np.random.default_rng(8)
+    PA, PB, W = (0.2 * (A + A.T) for A in rng.standard_normal((3, n, n)))
+    PB = PA if restricted else PB
+    # the permuted layout: the first and fourth functions of the first d shell (xx, xy) swapped
+    d0 = next(i for i in range(n) if b.lmn[i].sum() == 2)
+    perm = np.arange(n)
+    perm[[d0, d0 + 3]] = perm[[d0 + 3, d0]]
+    ex = [b.exps[o:o + k] for o, k in zip(b.offset, b.nprim)]
+    co = [b.coefs[o:o + k] for o, k in zip(b.offset, b.nprim)]
+    no = [b.norms[o:o + k] for o, k in zip(b.offset, b.nprim)]
+    cat = lambda v: np.concatenate([v[i] for i in perm])
+    b2 = sqb.basis.Basis(b.nprim[perm], b.lmn[perm], b.center[perm], cat(ex), cat(co), cat(no))
+    Z = np.array([6.0, 8.0, 1.0])
+    xyz = np.array([[0.0, 0.0, 0.1], [0.0, 1.9, -0.4], [1.3, -0.7, 1.1]])
+    G = []
+    for basis, p in ((b, np.arange(n)), (b2, perm)):
+        eng = sqb.JKEngine(basis)
+        ix = np.ix_(p, p)
+        G.append(eng.gradient(Z, xyz, PA[ix], PB[ix], W[ix], terms=8))
+        eng.close()
+    assert np.abs(G[0]).max() > 0
+    assert np.abs(G[0] - G[1]).max() <= 1e-11 * np.abs(G[1]).max()
