@@ -155,8 +155,9 @@ int sqb200_jk_autotune(sqb200_jk *ctx, const double *dPA, const double *dPB, int
                        double scf_cutoff, double fixed_cutoff, double dscreen_rmax, void *stream);
 
 /* Read (sqb200_jk_tiles) or set (sqb200_jk_set_tiles) the per-class FP64 form: 0, 1 or 2 as
- * above; -1 (read only) class k has one form.  Setting a form a class lacks selects 0.
- * sqb200_jk_tiles returns the number of entries written (at most n). */
+ * above; -1: the class runs its default form (neither tuned nor set; also read for a class with
+ * one form).  Setting a form a class lacks selects 0.  sqb200_jk_tiles returns the number of
+ * entries written (at most n). */
 int sqb200_jk_tiles(sqb200_jk *ctx, int *form, int n);
 int sqb200_jk_set_tiles(sqb200_jk *ctx, const int *form, int n);
 

@@ -26,9 +26,10 @@ jk_DS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const sqb::WorkItem it = items[qi_];
       const sqb::PairRec bp = a.bra_pairs[it.bra];
       const sqb::MolRec mr = a.mols[it.mol];        // the molecule of this work item
-      double* __restrict__ Jacc = a.Jacc + mr.moff;
-      double* __restrict__ KAacc = a.KAacc + mr.moff;
-      double* __restrict__ KBacc = a.KBacc + mr.moff;
+      const long long acc0 = mr.moff + (qi_ & a.copy_mask) * a.copy_stride;   // this item's copy
+      double* __restrict__ Jacc = a.Jacc + acc0;
+      double* __restrict__ KAacc = a.KAacc + acc0;
+      double* __restrict__ KBacc = a.KBacc + acc0;
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 26; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
@@ -36,6 +37,7 @@ jk_DS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
       const int gj = grp / si, gi = grp - gj * si;
+      const unsigned gmask = isplit >= 32 ? 0xffffffffu : ((1u << isplit) - 1u) << ((threadIdx.x & 31) & ~(isplit - 1));
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -551,14 +553,11 @@ jk_DS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
         }
       }
       {
-        const int fP = bp.fP, fQ = bp.fQ;
         const double s2 = 2.0 * deg;
-        { const double v = sqb::warp_sum(s2 * jab0); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 0) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab1); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 1) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab2); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 2) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab3); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 3) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab4); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 4) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab5); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 5) * N + fQ + 0, v); }
+        double v[8] = {s2 * jab0, s2 * jab1, s2 * jab2, s2 * jab3, s2 * jab4, s2 * jab5, 0.0, 0.0};
+        const double s = sqb::warp_sum_scatter<8>(v);
+        const int l = threadIdx.x & 31, ab = l + 0;
+        if (l < 6 && s != 0.0) atomicAdd(Jacc + (bp.fP + ab / 1) * N + bp.fQ + ab % 1, s);
       }
       sqb::count_add(a.counters + 0, (ok && grp == 0 && pass == 0) ? 1ull : 0ull);
       sqb::count_add(a.counters + 1, nprimq);

@@ -26,9 +26,10 @@ jk_LS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const sqb::WorkItem it = items[qi_];
       const sqb::PairRec bp = a.bra_pairs[it.bra];
       const sqb::MolRec mr = a.mols[it.mol];        // the molecule of this work item
-      double* __restrict__ Jacc = a.Jacc + mr.moff;
-      double* __restrict__ KAacc = a.KAacc + mr.moff;
-      double* __restrict__ KBacc = a.KBacc + mr.moff;
+      const long long acc0 = mr.moff + (qi_ & a.copy_mask) * a.copy_stride;   // this item's copy
+      double* __restrict__ Jacc = a.Jacc + acc0;
+      double* __restrict__ KAacc = a.KAacc + acc0;
+      double* __restrict__ KBacc = a.KBacc + acc0;
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 12; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
@@ -36,6 +37,7 @@ jk_LS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
       const int gj = grp / si, gi = grp - gj * si;
+      const unsigned gmask = isplit >= 32 ? 0xffffffffu : ((1u << isplit) - 1u) << ((threadIdx.x & 31) & ~(isplit - 1));
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -296,46 +298,45 @@ jk_LS_LS_R(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             jab1 += o1_0 * ptk0 + o1_1 * ptk1 + o1_2 * ptk2 + o1_3 * ptk3;
             jab2 += o2_0 * ptk0 + o2_1 * ptk1 + o2_2 * ptk2 + o2_3 * ptk3;
             jab3 += o3_0 * ptk0 + o3_1 * ptk1 + o3_2 * ptk2 + o3_3 * ptk3;
-            atomicAdd(Jacc + (fI + 0) * N + fJ + 0, 2.0 * deg * (o0_0 * ptb0 + o1_0 * ptb1 + o2_0 * ptb2 + o3_0 * ptb3));
-            atomicAdd(Jacc + (fI + 1) * N + fJ + 0, 2.0 * deg * (o0_1 * ptb0 + o1_1 * ptb1 + o2_1 * ptb2 + o3_1 * ptb3));
-            atomicAdd(Jacc + (fI + 2) * N + fJ + 0, 2.0 * deg * (o0_2 * ptb0 + o1_2 * ptb1 + o2_2 * ptb2 + o3_2 * ptb3));
-            atomicAdd(Jacc + (fI + 3) * N + fJ + 0, 2.0 * deg * (o0_3 * ptb0 + o1_3 * ptb1 + o2_3 * ptb2 + o3_3 * ptb3));
-            atomicAdd(KAacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Abd0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Aad0_0 + o1_0 * Aad1_0 + o2_0 * Aad2_0 + o3_0 * Aad3_0));
-            atomicAdd(KAacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Abc0_0 + o0_1 * Abc0_1 + o0_2 * Abc0_2 + o0_3 * Abc0_3));
-            atomicAdd(KAacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Aac0_0 + o0_1 * Aac0_1 + o0_2 * Aac0_2 + o0_3 * Aac0_3 + o1_0 * Aac1_0 + o1_1 * Aac1_1 + o1_2 * Aac1_2 + o1_3 * Aac1_3 + o2_0 * Aac2_0 + o2_1 * Aac2_1 + o2_2 * Aac2_2 + o2_3 * Aac2_3 + o3_0 * Aac3_0 + o3_1 * Aac3_1 + o3_2 * Aac3_2 + o3_3 * Aac3_3));
-            atomicAdd(KAacc + (fP + 0) * N + fI + 1, deg * (o0_1 * Abd0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fI + 1, deg * (o0_1 * Aad0_0 + o1_1 * Aad1_0 + o2_1 * Aad2_0 + o3_1 * Aad3_0));
-            atomicAdd(KAacc + (fP + 0) * N + fI + 2, deg * (o0_2 * Abd0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fI + 2, deg * (o0_2 * Aad0_0 + o1_2 * Aad1_0 + o2_2 * Aad2_0 + o3_2 * Aad3_0));
-            atomicAdd(KAacc + (fP + 0) * N + fI + 3, deg * (o0_3 * Abd0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fI + 3, deg * (o0_3 * Aad0_0 + o1_3 * Aad1_0 + o2_3 * Aad2_0 + o3_3 * Aad3_0));
-            atomicAdd(KAacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Abc0_0 + o1_1 * Abc0_1 + o1_2 * Abc0_2 + o1_3 * Abc0_3));
-            atomicAdd(KAacc + (fP + 1) * N + fI + 1, deg * (o1_1 * Abd0_0));
-            atomicAdd(KAacc + (fP + 1) * N + fI + 2, deg * (o1_2 * Abd0_0));
-            atomicAdd(KAacc + (fP + 1) * N + fI + 3, deg * (o1_3 * Abd0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Abc0_0 + o2_1 * Abc0_1 + o2_2 * Abc0_2 + o2_3 * Abc0_3));
-            atomicAdd(KAacc + (fP + 2) * N + fI + 1, deg * (o2_1 * Abd0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fI + 2, deg * (o2_2 * Abd0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fI + 3, deg * (o2_3 * Abd0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Abc0_0 + o3_1 * Abc0_1 + o3_2 * Abc0_2 + o3_3 * Abc0_3));
-            atomicAdd(KAacc + (fP + 3) * N + fI + 1, deg * (o3_1 * Abd0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fI + 2, deg * (o3_2 * Abd0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fI + 3, deg * (o3_3 * Abd0_0));
+            sqb::group_add(Jacc + (fI + 0) * N + fJ + 0, 2.0 * deg * (o0_0 * ptb0 + o1_0 * ptb1 + o2_0 * ptb2 + o3_0 * ptb3), isplit, gmask, grp == 0);
+            sqb::group_add(Jacc + (fI + 1) * N + fJ + 0, 2.0 * deg * (o0_1 * ptb0 + o1_1 * ptb1 + o2_1 * ptb2 + o3_1 * ptb3), isplit, gmask, grp == 0);
+            sqb::group_add(Jacc + (fI + 2) * N + fJ + 0, 2.0 * deg * (o0_2 * ptb0 + o1_2 * ptb1 + o2_2 * ptb2 + o3_2 * ptb3), isplit, gmask, grp == 0);
+            sqb::group_add(Jacc + (fI + 3) * N + fJ + 0, 2.0 * deg * (o0_3 * ptb0 + o1_3 * ptb1 + o2_3 * ptb2 + o3_3 * ptb3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Aad0_0 + o1_0 * Aad1_0 + o2_0 * Aad2_0 + o3_0 * Aad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Abc0_0 + o0_1 * Abc0_1 + o0_2 * Abc0_2 + o0_3 * Abc0_3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Aac0_0 + o0_1 * Aac0_1 + o0_2 * Aac0_2 + o0_3 * Aac0_3 + o1_0 * Aac1_0 + o1_1 * Aac1_1 + o1_2 * Aac1_2 + o1_3 * Aac1_3 + o2_0 * Aac2_0 + o2_1 * Aac2_1 + o2_2 * Aac2_2 + o2_3 * Aac2_3 + o3_0 * Aac3_0 + o3_1 * Aac3_1 + o3_2 * Aac3_2 + o3_3 * Aac3_3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fI + 1, deg * (o0_1 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fI + 1, deg * (o0_1 * Aad0_0 + o1_1 * Aad1_0 + o2_1 * Aad2_0 + o3_1 * Aad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fI + 2, deg * (o0_2 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fI + 2, deg * (o0_2 * Aad0_0 + o1_2 * Aad1_0 + o2_2 * Aad2_0 + o3_2 * Aad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fI + 3, deg * (o0_3 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fI + 3, deg * (o0_3 * Aad0_0 + o1_3 * Aad1_0 + o2_3 * Aad2_0 + o3_3 * Aad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Abc0_0 + o1_1 * Abc0_1 + o1_2 * Abc0_2 + o1_3 * Abc0_3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fI + 1, deg * (o1_1 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fI + 2, deg * (o1_2 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fI + 3, deg * (o1_3 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Abc0_0 + o2_1 * Abc0_1 + o2_2 * Abc0_2 + o2_3 * Abc0_3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fI + 1, deg * (o2_1 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fI + 2, deg * (o2_2 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fI + 3, deg * (o2_3 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Abc0_0 + o3_1 * Abc0_1 + o3_2 * Abc0_2 + o3_3 * Abc0_3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fI + 1, deg * (o3_1 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fI + 2, deg * (o3_2 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fI + 3, deg * (o3_3 * Abd0_0), isplit, gmask, grp == 0);
           }
         } break;
         }
       }
       {
-        const int fP = bp.fP, fQ = bp.fQ;
         const double s2 = 2.0 * deg;
-        { const double v = sqb::warp_sum(s2 * jab0); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 0) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab1); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 1) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab2); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 2) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab3); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 3) * N + fQ + 0, v); }
+        double v[4] = {s2 * jab0, s2 * jab1, s2 * jab2, s2 * jab3};
+        const double s = sqb::warp_sum_scatter<4>(v);
+        const int l = threadIdx.x & 31, ab = l + 0;
+        if (l < 4 && s != 0.0) atomicAdd(Jacc + (bp.fP + ab / 1) * N + bp.fQ + ab % 1, s);
       }
       sqb::count_add(a.counters + 0, (ok && grp == 0 && pass == 0) ? 1ull : 0ull);
       sqb::count_add(a.counters + 1, nprimq);

@@ -26,9 +26,10 @@ jk_LS_SS_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const sqb::WorkItem it = items[qi_];
       const sqb::PairRec bp = a.bra_pairs[it.bra];
       const sqb::MolRec mr = a.mols[it.mol];        // the molecule of this work item
-      double* __restrict__ Jacc = a.Jacc + mr.moff;
-      double* __restrict__ KAacc = a.KAacc + mr.moff;
-      double* __restrict__ KBacc = a.KBacc + mr.moff;
+      const long long acc0 = mr.moff + (qi_ & a.copy_mask) * a.copy_stride;   // this item's copy
+      double* __restrict__ Jacc = a.Jacc + acc0;
+      double* __restrict__ KAacc = a.KAacc + acc0;
+      double* __restrict__ KBacc = a.KBacc + acc0;
       const int N = mr.nbf;
       for (int x = threadIdx.x; x < bp.nprim * 12; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];
       __syncthreads();
@@ -36,6 +37,7 @@ jk_LS_SS_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
       const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
       const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
       const int gj = grp / si, gi = grp - gj * si;
+      const unsigned gmask = isplit >= 32 ? 0xffffffffu : ((1u << isplit) - 1u) << ((threadIdx.x & 31) & ~(isplit - 1));
       const int pass = qp_;                   // block of ket functions handled by this CTA
       bool ok = kl < it.cnt;
       sqb::PairRec kp = bp;
@@ -179,38 +181,37 @@ jk_LS_SS_U(const sqb::JKArgs a, const sqb::WorkItem* __restrict__ items) {
             jab1 += o1_0 * ptk0;
             jab2 += o2_0 * ptk0;
             jab3 += o3_0 * ptk0;
-            atomicAdd(Jacc + (fI + 0) * N + fJ + 0, 2.0 * deg * (o0_0 * ptb0 + o1_0 * ptb1 + o2_0 * ptb2 + o3_0 * ptb3));
-            atomicAdd(KAacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Abd0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Aad0_0 + o1_0 * Aad1_0 + o2_0 * Aad2_0 + o3_0 * Aad3_0));
-            atomicAdd(KAacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Abc0_0));
-            atomicAdd(KAacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Aac0_0 + o1_0 * Aac1_0 + o2_0 * Aac2_0 + o3_0 * Aac3_0));
-            atomicAdd(KAacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Abc0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Abc0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Abd0_0));
-            atomicAdd(KAacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Abc0_0));
-            atomicAdd(KBacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Bbd0_0));
-            atomicAdd(KBacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Bad0_0 + o1_0 * Bad1_0 + o2_0 * Bad2_0 + o3_0 * Bad3_0));
-            atomicAdd(KBacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Bbc0_0));
-            atomicAdd(KBacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Bac0_0 + o1_0 * Bac1_0 + o2_0 * Bac2_0 + o3_0 * Bac3_0));
-            atomicAdd(KBacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Bbd0_0));
-            atomicAdd(KBacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Bbc0_0));
-            atomicAdd(KBacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Bbd0_0));
-            atomicAdd(KBacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Bbc0_0));
-            atomicAdd(KBacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Bbd0_0));
-            atomicAdd(KBacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Bbc0_0));
+            sqb::group_add(Jacc + (fI + 0) * N + fJ + 0, 2.0 * deg * (o0_0 * ptb0 + o1_0 * ptb1 + o2_0 * ptb2 + o3_0 * ptb3), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Aad0_0 + o1_0 * Aad1_0 + o2_0 * Aad2_0 + o3_0 * Aad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Abc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Aac0_0 + o1_0 * Aac1_0 + o2_0 * Aac2_0 + o3_0 * Aac3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Abc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Abc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Abd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KAacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Abc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 0) * N + fI + 0, deg * (o0_0 * Bbd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fQ + 0) * N + fI + 0, deg * (o0_0 * Bad0_0 + o1_0 * Bad1_0 + o2_0 * Bad2_0 + o3_0 * Bad3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 0) * N + fJ + 0, deg * (o0_0 * Bbc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fQ + 0) * N + fJ + 0, deg * (o0_0 * Bac0_0 + o1_0 * Bac1_0 + o2_0 * Bac2_0 + o3_0 * Bac3_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 1) * N + fI + 0, deg * (o1_0 * Bbd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 1) * N + fJ + 0, deg * (o1_0 * Bbc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 2) * N + fI + 0, deg * (o2_0 * Bbd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 2) * N + fJ + 0, deg * (o2_0 * Bbc0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 3) * N + fI + 0, deg * (o3_0 * Bbd0_0), isplit, gmask, grp == 0);
+            sqb::group_add(KBacc + (fP + 3) * N + fJ + 0, deg * (o3_0 * Bbc0_0), isplit, gmask, grp == 0);
           }
         } break;
         }
       }
       {
-        const int fP = bp.fP, fQ = bp.fQ;
         const double s2 = 2.0 * deg;
-        { const double v = sqb::warp_sum(s2 * jab0); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 0) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab1); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 1) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab2); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 2) * N + fQ + 0, v); }
-        { const double v = sqb::warp_sum(s2 * jab3); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + 3) * N + fQ + 0, v); }
+        double v[4] = {s2 * jab0, s2 * jab1, s2 * jab2, s2 * jab3};
+        const double s = sqb::warp_sum_scatter<4>(v);
+        const int l = threadIdx.x & 31, ab = l + 0;
+        if (l < 4 && s != 0.0) atomicAdd(Jacc + (bp.fP + ab / 1) * N + bp.fQ + ab % 1, s);
       }
       sqb::count_add(a.counters + 0, (ok && grp == 0 && pass == 0) ? 1ull : 0ull);
       sqb::count_add(a.counters + 1, nprimq);

@@ -69,6 +69,7 @@ MIN_BLOCKS = int(os.environ.get("SQB_MINB", "0"))   # __launch_bounds__ min CTAs
 # the same bound for the FP64 narrow-tile form only (its state is smallest, so a register cap
 # spills least there); 0 = none
 MIN_BLOCKS_NARROW = int(os.environ.get("SQB_MINB_NARROW", "0"))
+GROUP_MAX = 16             # function quartets of the classes whose split lanes sum before the atomics
 CTA = 128
 # Register caps (__maxnreg__) for kernels where a cap measured faster on B200: with fewer
 # registers per thread more 64-thread CTAs share an SM, which pays where the spills it adds stay
@@ -77,6 +78,27 @@ CTA = 128
 # 3.61 -> 3.12 at 128 (144 uncapped, no spills either way; 3.22 at 112).  LL|LL wide stays
 # uncapped (40.4 ms; 42.3 at 168, 47.2 at 200).  The unrestricted forms are not capped.
 REG_CAP = {"jk_LL_LS_R_w": 128, "jk_LS_LS_R_s": 128}
+
+
+# The FP64 form a class runs without autotuning: 0 narrow, 1 wide, 2 swapped.  Measured on B200
+# (us per launch, narrow / wide / swapped):
+#   an organic of 14 heavy atoms, 6-31G*: DL|LL 538 / 345 / 354, LL|LL 268 / 225 / 215, DL|DL 290 / 203 / 290,
+#   DL|LS 254 / 190 / 236, LL|LS 244 / 212 / 179, LS|SS 159 / 160 / 127, LS|LS 170 / 171 / 124, SS|SS 142 / 142 /
+#   102, DS|LS 144 / 144 / 104, DL|DS 165 / 117 / 179, LL|DS 147 / 122 / 147, DD|LS 90 / 91 / 133;
+#   of 10 heavy atoms, DZP: DP|PP 471 / 305 / 359, DP|PS 363 / 238 / 293, DP|DP 220 / 167 / 196, DP|DS 226 / 142 /
+#   216, PP|PS 352 / 352 / 315, PS|SS 374 / 377 / 323, DP|SS 143 / 143 / 215; C60/6-31G LL|LL 60 / 39 / 45 ms.
+# So: bras of at least 18 functions wide (narrow where they have no wide form), the others swapped
+# on s-type kets, wide otherwise.
+def default_form(bra, ket, has_wide, has_swap):
+    if bra in ("DL", "DP", "DD"):
+        if (bra, ket) == ("DL", "SS"):
+            return 2
+        return 1 if has_wide else 0
+    if ket[1] == "S" and ket != "DS" and has_swap:
+        return 2
+    if (bra, ket) in (("DS", "DS"), ("PP", "DS")):
+        return 0
+    return 1 if has_wide else 0
 
 
 def kernel_qualifiers(name, bounds):
@@ -268,9 +290,10 @@ def gen_class(bra, ket, spin, prec="D", state_max=None, suffix=""):
     em("const sqb::WorkItem it = items[blockIdx.x];")
     em("const sqb::PairRec bp = a.bra_pairs[it.bra];")
     em("const sqb::MolRec mr = a.mols[it.mol];        // the molecule of this work item")
-    em("double* __restrict__ Jacc = a.Jacc + mr.moff;")
-    em("double* __restrict__ KAacc = a.KAacc + mr.moff;")
-    em("double* __restrict__ KBacc = a.KBacc + mr.moff;")
+    em("const long long acc0 = mr.moff + (blockIdx.x & a.copy_mask) * a.copy_stride;   // this item's copy")
+    em("double* __restrict__ Jacc = a.Jacc + acc0;")
+    em("double* __restrict__ KAacc = a.KAacc + acc0;")
+    em("double* __restrict__ KBacc = a.KBacc + acc0;")
     em("const int N = mr.nbf;")
     em("for (int x = threadIdx.x; x < bp.nprim * %d; x += blockDim.x) sbra[x] = a.bra_prims%s[bp.poff + (long long)x * bp.kstride];" % (NB, "_f" if F32 else ""))
     em("__syncthreads();")
@@ -278,6 +301,7 @@ def gen_class(bra, ket, spin, prec="D", state_max=None, suffix=""):
     em("const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;")
     em("const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;")
     em("const int gj = grp / si, gi = grp - gj * si;")
+    em("const unsigned gmask = isplit >= 32 ? 0xffffffffu : ((1u << isplit) - 1u) << ((threadIdx.x & 31) & ~(isplit - 1));")
     em("const int pass = blockIdx.y;                   // block of ket functions handled by this CTA")
     em("bool ok = kl < it.cnt;")
     em("sqb::PairRec kp = bp;")
@@ -419,7 +443,7 @@ def gen_class(bra, ket, spin, prec="D", state_max=None, suffix=""):
         if MP:
             emit_multipole(em, blk, nab, nb_, nd)
         # digestion of this block
-        qf = emit_digest(em, spin, blk, nab, na, nb_, nd)
+        qf = emit_digest(em, spin, blk, nab, na, nb_, nd, ncd)
         fl["quartet"] += qf
         em.ind -= 1
         em("} break;")
@@ -427,13 +451,7 @@ def gen_class(bra, ket, spin, prec="D", state_max=None, suffix=""):
     em.ind -= 1
     em("}")
     # bra J: warp reduce (every lane shares the bra pair)
-    em("{")
-    em("  const int fP = bp.fP, fQ = bp.fQ;")
-    em("  const double s2 = 2.0 * deg;")
-    for ab in range(nab):
-        aa, bb = divmod(ab, nb_)
-        em("  { const double v = sqb::warp_sum(s2 * jab%d); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + %d) * N + fQ + %d, v); }" % (ab, aa, bb))
-    em("}")
+    emit_bra_j(em, list(range(nab)), nb_)
     em("sqb::count_add(a.counters + 0, (ok && grp == 0 && pass == 0) ? 1ull : 0ull);")
     em("sqb::count_add(a.counters + 1, nprimq);")
     em("sqb::count_add(a.counters + 2, nflush);")
@@ -519,9 +537,10 @@ def gen_class_swap(bra, ket, spin, state_max):
     em("const sqb::WorkItem it = items[blockIdx.x];")
     em("const sqb::PairRec bp = a.bra_pairs[it.bra];")
     em("const sqb::MolRec mr = a.mols[it.mol];        // the molecule of this work item")
-    em("double* __restrict__ Jacc = a.Jacc + mr.moff;")
-    em("double* __restrict__ KAacc = a.KAacc + mr.moff;")
-    em("double* __restrict__ KBacc = a.KBacc + mr.moff;")
+    em("const long long acc0 = mr.moff + (blockIdx.x & a.copy_mask) * a.copy_stride;   // this item's copy")
+    em("double* __restrict__ Jacc = a.Jacc + acc0;")
+    em("double* __restrict__ KAacc = a.KAacc + acc0;")
+    em("double* __restrict__ KBacc = a.KBacc + acc0;")
     em("const int N = mr.nbf;")
     em("for (int x = threadIdx.x; x < bp.nprim * %d; x += blockDim.x) sbra[x] = a.bra_prims[bp.poff + (long long)x * bp.kstride];" % NB)
     em("__syncthreads();")
@@ -529,6 +548,7 @@ def gen_class_swap(bra, ket, spin, state_max):
     em("const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;")
     em("const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;")
     em("const int gj = grp / si, gi = grp - gj * si;")
+    em("const unsigned gmask = isplit >= 32 ? 0xffffffffu : ((1u << isplit) - 1u) << ((threadIdx.x & 31) & ~(isplit - 1));")
     em("const int pass = blockIdx.y;                   // block of bra functions handled by this CTA")
     em("bool ok = kl < it.cnt;")
     em("sqb::PairRec kp = bp;")
@@ -634,19 +654,18 @@ def gen_class_swap(bra, ket, spin, state_max):
         em("}")
         fl["prim"] += pf
         fl["flush"] += ff
-        qf = emit_digest(em, spin, list(range(ncd)), nab, na, nb_, nd, ablk=blk)
+        qf = emit_digest(em, spin, list(range(ncd)), nab, na, nb_, nd, ncd, ablk=blk)
         fl["quartet"] += qf
         em.ind -= 1
         em("} break;")
     em("}")
     em.ind -= 1
     em("}")
-    em("{")
-    em("  const int fP = bp.fP, fQ = bp.fQ;")
-    em("  const double s2 = 2.0 * deg;")
-    for ab in range(nab):
-        aa, bb = divmod(ab, nb_)
-        em("  { const double v = sqb::warp_sum(s2 * jab%d); if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(Jacc + (fP + %d) * N + fQ + %d, v); }" % (ab, aa, bb))
+    em("switch (pass) {")
+    for bi, blk in enumerate(blocks):
+        em("case %d:" % bi)
+        emit_bra_j(em, blk, nb_)
+        em("break;")
     em("}")
     em("sqb::count_add(a.counters + 0, (ok && grp == 0 && pass == 0) ? 1ull : 0ull);")
     em("sqb::count_add(a.counters + 1, nprimq);")
@@ -657,6 +676,24 @@ def gen_class_swap(bra, ket, spin, state_max):
     meta = {"name": name, "bra": bra, "ket": ket, "spin": spin, "nab": nab, "ncd": ncd,
             "neb": len(layb), "nek": len(layk), "Lt": pair_L(bra) + pair_L(ket), "flops": fl}
     return "\n".join(out) + "\n", meta
+
+
+def emit_bra_j(em, blk, nb_):
+    """Add the bra-side Coulomb sums jab<ab> (ab in blk) of the warp's lanes, which all share the
+    bra pair: warp sums of up to 32 values at once, each added by one lane."""
+    for s0 in range(0, len(blk), 32):
+        part = blk[s0:s0 + 32]
+        M = 1
+        while M < len(part):
+            M *= 2
+        em("{")
+        em("  const double s2 = 2.0 * deg;")
+        em("  double v[%d] = {%s};" % (M, ", ".join(["s2 * jab%d" % ab for ab in part] + ["0.0"] * (M - len(part)))))
+        em("  const double s = sqb::warp_sum_scatter<%d>(v);" % M)
+        em("  const int l = threadIdx.x & 31, ab = %s;" % ("l + %d" % part[0] if part == list(range(part[0], part[0] + len(part)))
+                                                          else "0"))
+        em("  if (l < %d && s != 0.0) atomicAdd(Jacc + (bp.fP + ab / %d) * N + bp.fQ + ab %% %d, s);" % (len(part), nb_, nb_))
+        em("}")
 
 
 def emit_multipole(em, blk, nab, nb_, nd):
@@ -685,12 +722,17 @@ def emit_multipole(em, blk, nab, nb_, nd):
     em("}")
 
 
-def emit_digest(em, spin, blk, nab, na, nb_, nd, ablk=None):
+def emit_digest(em, spin, blk, nab, na, nb_, nd, ncd_all, ablk=None):
     """Digest the contracted block o<ab>_<cd> (cd in blk, ab in ablk -- all bra functions by
     default) into the J/K accumulators.  Expects PA, PB (unrestricted), PT, N, bp, kp, deg and
     jab<ab> in scope; returns flops."""
     abs_ = list(range(nab)) if ablk is None else list(ablk)
     qf = 0
+    # small blocks, whose long contractions are split over many lanes, sum those lanes' values before
+    # the atomic; larger blocks have too many targets: the inlined sums grow the code past what the
+    # instruction cache holds (every class with them: benzene/6-31G* 0.68 -> 0.75 ms per build)
+    group = nab * ncd_all <= GROUP_MAX
+    add = lambda p, v: em("sqb::group_add(%s, %s, isplit, gmask, grp == 0);" % (p, v) if group else "atomicAdd(%s, %s);" % (p, v))
     cset = sorted({cd // nd for cd in blk})
     dset = sorted({cd % nd for cd in blk})
     em("{  // digest")
@@ -723,7 +765,7 @@ def emit_digest(em, spin, blk, nab, na, nb_, nd, ablk=None):
     for cd in blk:
         c, d = divmod(cd, nd)
         terms = " + ".join("o%d_%d * ptb%d" % (ab, cd, ab) for ab in abs_)
-        em("atomicAdd(Jacc + (fI + %d) * N + fJ + %d, 2.0 * deg * (%s));" % (c, d, terms))
+        add("Jacc + (fI + %d) * N + fJ + %d" % (c, d), "2.0 * deg * (%s)" % terms)
         qf += 2 * len(abs_) + 2
     for s, _ in spins:
         acc = "KAacc" if s == "A" else "KBacc"
@@ -738,7 +780,7 @@ def emit_digest(em, spin, blk, nab, na, nb_, nd, ablk=None):
                 tg.setdefault(("P", aa, "J", d), []).append("%s * %sbc%d_%d" % (o, s, bb, c))
                 tg.setdefault(("Q", bb, "J", d), []).append("%s * %sac%d_%d" % (o, s, aa, c))
         for (rs_, ri, cs_, ci), terms in tg.items():
-            em("atomicAdd(%s + (f%s + %d) * N + f%s + %d, deg * (%s));" % (acc, rs_, ri, cs_, ci, " + ".join(terms)))
+            add("%s + (f%s + %d) * N + f%s + %d" % (acc, rs_, ri, cs_, ci), "deg * (%s)" % " + ".join(terms))
             qf += 2 * len(terms) + 1
     em.ind -= 1
     em("}")
@@ -832,11 +874,12 @@ def main():
             reg.append('   0, nullptr, nullptr, 0, 0, 0,')
         sr, su = r["swap"], u["swap"]
         if sr:
-            reg.append('   %d, (const void*)%s, (const void*)%s, %d, %d, %d},' % (
+            reg.append('   %d, (const void*)%s, (const void*)%s, %d, %d, %d,' % (
                 sr["flops"]["passes"], sr["name"], su["name"], sr["flops"]["prim"], sr["flops"]["flush"],
                 sr["flops"]["quartet"]))
         else:
-            reg.append('   0, nullptr, nullptr, 0, 0, 0},')
+            reg.append('   0, nullptr, nullptr, 0, 0, 0,')
+        reg.append('   %d},' % default_form(r["bra"], r["ket"], bool(wr), bool(sr)))
     reg.append("};")
     reg.append("const int kNumClassKernels = %d;" % (len(metas) // 2))
     reg.append("}  // namespace sqb")

@@ -101,6 +101,11 @@ struct JKArgs {
   // of the launch from this device counter, zeroed before the launch; npass passes per item.
   unsigned long long* queue;
   int nqueue, npass;
+  // Copies of the accumulators (a power of two, less one as a mask; `copy_stride` doubles apart):
+  // work item i adds into copy i & copy_mask, so that the atomics of a small molecule's build do
+  // not all meet on its few elements
+  int copy_mask;
+  long long copy_stride;
 };
 
 constexpr int ERR_MIN = -120;      // src/matrix.c:1745-1747
@@ -209,6 +214,36 @@ __device__ __forceinline__ void count_add(unsigned long long* c, unsigned long l
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(c, v);
+}
+
+// *p += v, summed first over the n lanes (a power of two, aligned: mask gmask) that share one
+// quartet, whose targets are the same; one atomic per quartet instead of n on one address.
+__device__ __forceinline__ void group_add(double* p, double v, int n, unsigned gmask, bool lead) {
+  if (n > 1) {
+    for (int o = n >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(gmask, v, o);
+    if (!lead) return;
+  }
+  atomicAdd(p, v);
+}
+
+// Warp sums of M values (a power of two <= 32) at once: returns in lane l the warp's sum of
+// v[l % M].  Every step halves the values a lane holds, M - 1 + log2(32 / M) exchanges in all
+// where M separate sums take 5 M.
+template <int M>
+__device__ __forceinline__ double warp_sum_scatter(double (&v)[M]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = M / 2; s > 0; s >>= 1) {
+    const bool hi = lane & s;
+#pragma unroll
+    for (int k = 0; k < s; ++k) {
+      const double send = hi ? v[k] : v[k + s], keep = hi ? v[k + s] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+    }
+  }
+#pragma unroll
+  for (int o = M; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -349,7 +349,8 @@ struct sqb200_jk {
   // key: outer cutoff, fixed cutoff, FP32 threshold, multipole mode
   std::map<std::tuple<double, double, double, int>, Work> work;
   double fp32_below = 0.0;      // quartets with Schwarz product below this use the FP32 form
-  std::vector<char> form;       // per class kernel: FP64 form to run, 0 narrow / 1 wide / 2 swapped (autotuner)
+  std::vector<signed char> form;   // per class kernel: FP64 form to run, 0 narrow / 1 wide / 2 swapped (set by the
+                                   // autotuner or the caller), -1 the class's default
   std::vector<char> ran_form;   // per class kernel: the FP64 form the last build launched
   std::vector<long long> last_counts;
   long long last_flops = 0;
@@ -395,14 +396,20 @@ cudaError_t noalloc_lookup(unsigned char** out);
 
 // ---------------------------------------------------------------- device helpers
 
+// Copies of the J/K accumulators of a single-molecule build of n functions (see JKArgs): the fewer
+// their elements, the more of a build's atomics meet on each.  Measured on B200 with 1 / 8 copies
+// of K: an organic of 4 heavy atoms in DZP 0.73 / 0.64 ms per build, a 3-heavy-atom radical 0.30 / 0.28,
+// benzene/6-31G* 0.62 / 0.61, an organic of 9 heavy atoms (192 functions) 1.23 / 1.24.
+int acc_copies(int n) { return n <= 160 ? 8 : 1; }
+
 // PT = PA + PB and zeroed accumulators; the first thread also writes the build's molecule
 // record (offsets 0, sizes and this build's cutoffs), which the class kernels read
 __global__ void k_prep(const double* __restrict__ PA, const double* __restrict__ PB, double* __restrict__ PT,
-                       double* __restrict__ J, double* __restrict__ KA, double* __restrict__ KB, int nn, int uhf,
+                       double* __restrict__ J, double* __restrict__ KA, double* __restrict__ KB, int nn, int ncopy, int uhf,
                        sqb::MolRec* __restrict__ mol, sqb::MolRec mv) {
   if (mol && blockIdx.x == 0 && threadIdx.x == 0) *mol = mv;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-    PT[i] = PA[i] + PB[i];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn * ncopy; i += gridDim.x * blockDim.x) {
+    if (i < nn) PT[i] = PA[i] + PB[i];
     J[i] = 0.0;
     KA[i] = 0.0;
     if (uhf) KB[i] = 0.0;
@@ -439,14 +446,20 @@ void launch_pmax(const double* PA, const double* PB, const double* PT, const int
 
 // JT = J + J^T, KA = -(K + K^T), KB likewise or = KA
 __global__ void k_finalize(const double* __restrict__ J, const double* __restrict__ KA, const double* __restrict__ KB,
-                           double* __restrict__ JT, double* __restrict__ KAo, double* __restrict__ KBo, int n, int uhf) {
+                           double* __restrict__ JT, double* __restrict__ KAo, double* __restrict__ KBo, int n, int ncopy, int uhf) {
   const int nn = n * n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
     const int r = i / n, c = i % n, t = c * n + r;
-    JT[i] = J[i] + J[t];
-    const double ka = -(KA[i] + KA[t]);
+    double j = 0.0, ka = 0.0, kb = 0.0;
+    for (int k = 0; k < ncopy; ++k) {
+      const size_t o = (size_t)k * nn;
+      j += J[o + i] + J[o + t];
+      ka -= KA[o + i] + KA[o + t];
+      if (KBo && uhf) kb -= KB[o + i] + KB[o + t];
+    }
+    JT[i] = j;
     KAo[i] = ka;
-    if (KBo) KBo[i] = uhf ? -(KB[i] + KB[t]) : ka;
+    if (KBo) KBo[i] = uhf ? kb : ka;
   }
 }
 
@@ -882,21 +895,31 @@ int cta_threads(double ops) {
 // kernels side by side on an SM share its instruction cache).
 constexpr int kSideStreams = 8;
 
-int ensure_side_streams(sqb200_jk* c) {
-  if (c->nside >= 0) return SQB200_OK;
-  int n = kSideStreams;
-  if (const char* e = getenv("SQB200_STREAMS")) n = std::max(0, std::min(16, atoi(e)));
-  CUDA_OK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-  for (int i = 0; i < n; ++i) {
+// Side streams for a call of `launches` kernels (created when first needed, kept): the lanes it uses.
+int ensure_side_streams(sqb200_jk* c, size_t launches) {
+  if (c->nside < 0) {
+    CUDA_OK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+    c->nside = kSideStreams;
+    if (const char* e = getenv("SQB200_STREAMS")) c->nside = std::max(0, std::min(16, atoi(e)));
+  }
+  while (c->side.size() < (size_t)c->nside && c->side.size() + 1 < launches) {
     cudaStream_t s;
     cudaEvent_t e;
-    CUDA_OK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const cudaError_t rc = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (rc != cudaSuccess) {
+      cudaEventDestroy(e);
+      return fail(SQB200_ECUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(rc));
+    }
     c->side.push_back(s);
     c->ev_join.push_back(e);
   }
-  c->nside = n;
   return SQB200_OK;
+}
+
+// Lanes of a call of `launches` kernels: its own stream and the side streams.
+int lanes_for(const sqb200_jk* c, size_t launches) {
+  return 1 + (int)std::min<size_t>(c->side.size(), launches > 0 ? launches - 1 : 0);
 }
 
 // Emitted FP operations of one thread per primitive step of class K (narrow tile: one pass), plus
@@ -905,16 +928,17 @@ int ensure_side_streams(sqb200_jk* c) {
 double step_ops(const sqb::ClassKernel& K) { return 150.0 + (double)K.flops_prim / K.passes; }
 
 // Threads per quartet of a (nbp bra x nkp ket primitives) run: si over the bra x sj over the ket
-// primitives, at most 32 in all, the fewest whose threads run at most `steps` primitive steps
-// (or, when 32 do not reach that, the split with the shortest loop).  Every thread digests its
-// own partial block, so a split costs a digestion per thread; among splits of one size the one
-// over the bra primitives comes first (a thread flushes once per bra primitive).
-int pick_split(int nbp, int nkp, double steps) {
+// primitives, at most 32 in all, the fewest whose threads run at most `steps` primitive steps (or,
+// when 32 do not reach that, the split with the shortest loop).  Every thread digests its own
+// partial block, so a split costs a digestion per thread; among splits of one size the one over
+// the bra primitives comes first (a thread flushes once per bra primitive).  pow2: aligned lanes
+// (classes of at most 16 function quartets, whose lanes' sums meet in shuffles before the atomics).
+int pick_split(int nbp, int nkp, double steps, bool pow2) {
   int best = 1 | 1 << 16;
   long best_loop = (long)nbp * nkp, best_n = 1;
   if (best_loop <= steps) return best;
   for (int n = 2; n <= 32; ++n) {
-    if (32 / n * n < 28) continue;               // quartets of n threads fill at least 28 of 32 lanes
+    if (pow2 ? (n & (n - 1)) != 0 : 32 / n * n < 28) continue;   // quartets of n threads fill at least 28 of 32 lanes
     for (int sj = 1; sj <= n; ++sj) {
       if (n % sj || sj > nkp || n / sj > nbp) continue;
       const int si = n / sj;
@@ -994,7 +1018,7 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
       const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0s = T.sub[sy], k1s = T.sub[sy + 1];
       const int nbp = B.pairs[b0].nprim, nkp = T.pairs[k0s].nprim;
       // multipole mode needs each quartet's whole block in one thread
-      const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K));
+      const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K), K.nab * K.ncd <= 16);
       const int kper = cta / ((split & 0xffff) * (split >> 16));
       const double pq = (double)nbp * nkp;
       for (int b = b0; b < b1; ++b) {
@@ -1190,6 +1214,12 @@ bool has_form(const sqb::ClassKernel& K, int form) {
   return form == 0 || (form == 1 && K.fn_rw) || (form == 2 && K.fn_rs);
 }
 
+// The form a class runs: the one set for it, or its default (-1), where the class has it.
+int chosen_form(const sqb::ClassKernel& K, int set) {
+  const int f = set < 0 ? K.dflt : set;
+  return has_form(K, f) ? f : 0;
+}
+
 // The kernel of class K (FP32 form when f32) for spin uhf in FP64 form `form` (falls back to the
 // narrow tile where the class lacks it).  Returns the FP64 form picked (0 for the FP32 form).
 int pick_form(const sqb::ClassKernel& K, bool f32, int uhf, int form, const void** fn, int* passes) {
@@ -1281,6 +1311,8 @@ SegLaunch seg_single(sqb200_jk* c, const sqb200_jk::Work* w, size_t s, const dou
   a.ket_pairs = T.d_pairs; a.ket_prims = T.d_prims;
   a.PA = dPA; a.PB = dPB; a.PT = c->d_PT; a.PM = c->d_PM;
   a.Jacc = c->d_J; a.KAacc = c->d_KA; a.KBacc = c->d_KB;
+  a.copy_mask = acc_copies(c->nbf) - 1;
+  a.copy_stride = (long long)c->nbf * c->nbf;
   a.boys_tab = c->d_boysr;
   a.boys_tab_f = c->d_boysf;
   a.counters = c->d_counters + 4 * v;
@@ -1299,7 +1331,7 @@ SegLaunch seg_single(sqb200_jk* c, const sqb200_jk::Work* w, size_t s, const dou
   }
   L.smem = (size_t)B.max_nprim * B.stride * (f32 ? sizeof(float) : sizeof(double));
   int passes = 1;
-  const int fu = pick_form(K, f32, uhf, form < 0 ? c->form[kidx] : form, &L.fn, &passes);
+  const int fu = pick_form(K, f32, uhf, form < 0 ? chosen_form(K, c->form[kidx]) : form, &L.fn, &passes);
   if (!f32) c->ran_form[kidx] = (char)fu;
   L.grid = dim3(w->count[s], passes);
   L.block = dim3(w->cta);
@@ -1317,7 +1349,9 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   int rc = build_work(c, outer, fixed, &w);
   if (rc) return rc;
   const sqb::MolRec mv{0, 0, n, c->ns, outer, fixed, dscreen, 0, uhf};
-  k_prep<<<grid_for(nn, 256), 256, 0, st>>>(dPA, dPB, c->d_PT, c->d_J, c->d_KA, c->d_KB, nn, uhf, c->d_mol, mv);
+  const int ncopy = acc_copies(n);
+  k_prep<<<grid_for((long)nn * ncopy, 256), 256, 0, st>>>(dPA, dPB, c->d_PT, c->d_J, c->d_KA, c->d_KB, nn, ncopy, uhf,
+                                                          c->d_mol, mv);
   launch_pmax(dPA, dPB, c->d_PT, c->d_shfirst, c->d_shn, c->ns, n, c->d_PM, st);
   CUDA_OK(cudaMemsetAsync(c->d_counters, 0, sizeof(unsigned long long) * 8 * sqb::kNumClassKernels, st));
   if (c->persistent) CUDA_OK(cudaMemsetAsync(c->d_queue, 0, sizeof(unsigned long long) * 2 * sqb::kNumClassKernels, st));
@@ -1325,9 +1359,9 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   // segments largest first, each on the least-loaded lane (lane 0 = st, the others are side
   // streams forked off st); per-class profiling keeps every launch on st so that each event
   // pair times one kernel alone
-  rc = ensure_side_streams(c);
+  rc = ensure_side_streams(c, w->kernel.size());
   if (rc) return rc;
-  const int nlanes = c->profile ? 1 : 1 + c->nside;
+  const int nlanes = c->profile ? 1 : lanes_for(c, w->kernel.size());
   std::vector<size_t> order(w->kernel.size());
   for (size_t s = 0; s < order.size(); ++s) order[s] = s;
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return w->cost[x] > w->cost[y]; });
@@ -1388,7 +1422,7 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   }
   if (c->mp_on && c->er_total > 0)
     k_erbank<<<grid_for(c->er_total, 256), 256, 0, st>>>(c->d_erbank, c->d_erscr, c->er_total);
-  k_finalize<<<grid_for(nn, 256), 256, 0, st>>>(c->d_J, c->d_KA, c->d_KB, dJT, dKA, dKB, n, uhf);
+  k_finalize<<<grid_for(nn, 256), 256, 0, st>>>(c->d_J, c->d_KA, c->d_KB, dJT, dKA, dKB, n, ncopy, uhf);
   CUDA_OK(cudaGetLastError());
   return SQB200_OK;
 }
@@ -1530,7 +1564,7 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   c->device = device;
   const char* pe = getenv("SQB200_PERSISTENT");
   c->persistent = pe && pe[0] == '1';
-  c->form.assign(sqb::kNumClassKernels, 0);
+  c->form.assign(sqb::kNumClassKernels, -1);
   c->ran_form.assign(sqb::kNumClassKernels, 0);
   c->nbf = nbf;
   int rc = build_shells(nbf, nprim, lmn, xyz, exps, ncoefs, c->shells);
@@ -1552,8 +1586,8 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   cv.add(&c->d_boysf, bt.rowsf.size() * sizeof(float));
   cv.add(&c->d_shfirst, c->ns * sizeof(int));
   cv.add(&c->d_shn, c->ns * sizeof(int));
-  for (double** m : {&c->d_PA, &c->d_PB, &c->d_PT, &c->d_J, &c->d_KA, &c->d_KB, &c->d_JT, &c->d_KAo, &c->d_KBo})
-    cv.add(m, nn * sizeof(double));
+  for (double** m : {&c->d_PA, &c->d_PB, &c->d_PT, &c->d_JT, &c->d_KAo, &c->d_KBo}) cv.add(m, nn * sizeof(double));
+  for (double** m : {&c->d_J, &c->d_KA, &c->d_KB}) cv.add(m, nn * acc_copies(nbf) * sizeof(double));
   cv.add(&c->d_PM, (size_t)c->ns * c->ns * sizeof(double));
   cv.add(&c->d_counters, 8 * sqb::kNumClassKernels * sizeof(unsigned long long));
   cv.add(&c->d_queue, 2 * sqb::kNumClassKernels * sizeof(unsigned long long));
@@ -1623,7 +1657,9 @@ int sqb200_jk_autotune(sqb200_jk* c, const double* dPA, const double* dPB, int r
   // the class kernels read PT, PM and the molecule record: set them up as a build does
   const int n = c->nbf, nn = n * n;
   const sqb::MolRec mv{0, 0, n, c->ns, outer, fixed, dscreen, 0, uhf};
-  k_prep<<<grid_for(nn, 256), 256, 0, st>>>(dPA, dPB, c->d_PT, c->d_J, c->d_KA, c->d_KB, nn, uhf, c->d_mol, mv);
+  const int ncopy = acc_copies(n);
+  k_prep<<<grid_for((long)nn * ncopy, 256), 256, 0, st>>>(dPA, dPB, c->d_PT, c->d_J, c->d_KA, c->d_KB, nn, ncopy, uhf,
+                                                          c->d_mol, mv);
   launch_pmax(dPA, dPB, c->d_PT, c->d_shfirst, c->d_shn, c->ns, n, c->d_PM, st);
   for (size_t s = 0; s < w->kernel.size(); ++s) {
     const int v = w->kernel[s];
@@ -1639,7 +1675,7 @@ int sqb200_jk_autotune(sqb200_jk* c, const double* dPA, const double* dPB, int r
       }
       if (tf[0] > kTuneLongMs) break;
     }
-    c->form[v] = (char)pick_tuned(sqb::kClassKernels[v], tf);
+    c->form[v] = (signed char)pick_tuned(sqb::kClassKernels[v], tf);
   }
   CUDA_OK(cudaStreamSynchronize(st));
   return SQB200_OK;
@@ -1657,7 +1693,7 @@ int sqb200_jk_tiles(sqb200_jk* c, int* form, int n) {
 int sqb200_jk_set_tiles(sqb200_jk* c, const int* form, int n) {
   if (!c || !form) return fail(SQB200_EINVAL, "null argument");
   for (int k = 0; k < n && k < sqb::kNumClassKernels; ++k)
-    c->form[k] = (char)(has_form(sqb::kClassKernels[k], form[k]) ? form[k] : 0);
+    c->form[k] = (signed char)(form[k] == -1 ? -1 : has_form(sqb::kClassKernels[k], form[k]) ? form[k] : 0);
   return SQB200_OK;
 }
 
@@ -2033,7 +2069,7 @@ extern "C" int sqb200_jk_build_noalloc(sqb200_jk* c, const double* dPA, const do
   // k_prep zeroes J, KA (and KB when unrestricted); the counters are cleared here
   sqb::MolRec* d_mol = (sqb::MolRec*)(base + kNoAllocMolOff);
   const sqb::MolRec mv{0, 0, n, c->ns, outer, fixed, dscreen, 0, uhf};
-  k_prep<<<grid_for(nn, 256), 256, 0, st>>>(dPA, dPB, PT, J, KA, KB, nn, uhf, d_mol, mv);
+  k_prep<<<grid_for(nn, 256), 256, 0, st>>>(dPA, dPB, PT, J, KA, KB, nn, 1, uhf, d_mol, mv);
   launch_pmax(dPA, dPB, PT, c->d_shfirst, c->d_shn, c->ns, n, PM, st);
   CUDA_OK(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 4 * sqb::kNumClassKernels, st));
   for (size_t s = 0; s < kernel.size(); ++s) {
@@ -2058,7 +2094,7 @@ extern "C" int sqb200_jk_build_noalloc(sqb200_jk* c, const double* dPA, const do
     if (rs) return rs;
     CUDA_OK(cudaLaunchKernel(fn, dim3(count[s], K.passes), dim3(128), args, smem, st));
   }
-  k_finalize<<<grid_for(nn, 256), 256, 0, st>>>(J, KA, KB, dJT, dKA, dKB, n, uhf);
+  k_finalize<<<grid_for(nn, 256), 256, 0, st>>>(J, KA, KB, dJT, dKA, dKB, n, 1, uhf);
   CUDA_OK(cudaGetLastError());
   return SQB200_OK;
 }
@@ -2150,7 +2186,7 @@ struct sqb200_batch {
   bool have_step = false;
   std::vector<unsigned long long> last_counts;
   int cta = 64;                         // threads per CTA of the class kernels
-  std::vector<char> form;               // per class kernel: FP64 form (sqb200_batch_autotune)
+  std::vector<signed char> form;        // per class kernel: FP64 form (sqb200_batch_autotune), -1 the default
   int last_launches = 0;
   int nside = -1;
   std::vector<cudaStream_t> side;
@@ -2293,7 +2329,7 @@ extern "C" int sqb200_batch_create(sqb200_batch** out, int nmol, sqb200_jk* cons
   if (e == cudaSuccess) e = h2d(b->d_shn, nf.data(), nf.size() * sizeof(int), b->stream);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return bail(SQB200_ECUDA, cudaGetErrorString(e));
-  b->form.assign(sqb::kNumClassKernels, 0);
+  b->form.assign(sqb::kNumClassKernels, -1);
   b->persistent = mols[0]->persistent;
   b->rec.resize(nmol);
   for (int m = 0; m < nmol; ++m)
@@ -2426,7 +2462,7 @@ SegLaunch seg_batch(sqb200_batch* b, size_t s, const double* dPA, const double* 
   L.items = b->d_items + b->first[s];
   L.smem = (size_t)B.max_nprim * B.stride * (f32 ? sizeof(float) : sizeof(double));
   int passes = 1;
-  const int fu = pick_form(K, f32, uhf, form < 0 ? b->form[kidx] : form, &L.fn, &passes);
+  const int fu = pick_form(K, f32, uhf, form < 0 ? chosen_form(K, b->form[kidx]) : form, &L.fn, &passes);
   L.grid = dim3(b->count[s], passes);
   L.block = dim3(b->cta);
   if (b->persistent) make_persistent(L, b->d_queue + uhf * 2 * K_ + v);
@@ -2435,7 +2471,7 @@ SegLaunch seg_batch(sqb200_batch* b, size_t s, const double* dPA, const double* 
 
 void batch_prologue(sqb200_batch* b, const double* dPA, const double* dPB, cudaStream_t st) {
   const long long ntot = b->moff[b->nmol];
-  k_prep<<<grid_for(ntot, 256), 256, 0, st>>>(dPA, dPB, b->d_PT, b->d_J, b->d_KA, b->d_KB, (int)ntot, 1,
+  k_prep<<<grid_for(ntot, 256), 256, 0, st>>>(dPA, dPB, b->d_PT, b->d_J, b->d_KA, b->d_KB, (int)ntot, 1, 1,
                                               nullptr, sqb::MolRec{});
   k_pmax_batch<<<dim3((b->max_ns * b->max_ns + 127) / 128, b->nmol), 128, 0, st>>>(
       dPA, dPB, b->d_PT, b->d_shfirst, b->d_shn, b->d_mols, b->d_PM);
@@ -2471,7 +2507,7 @@ extern "C" int sqb200_batch_autotune(sqb200_batch* b, const double* dPA, const d
     }
     for (int f = 0; f < 3; ++f) tf[3 * v + f] += ts[f];
   }
-  for (int k = 0; k < sqb::kNumClassKernels; ++k) b->form[k] = (char)pick_tuned(sqb::kClassKernels[k], &tf[3 * k]);
+  for (int k = 0; k < sqb::kNumClassKernels; ++k) b->form[k] = (signed char)pick_tuned(sqb::kClassKernels[k], &tf[3 * k]);
   CUDA_OK(cudaStreamSynchronize(st));
   return SQB200_OK;
 }
@@ -2541,7 +2577,7 @@ extern "C" int sqb200_batch_stats(sqb200_batch* b, long long* out, int n) {
       const unsigned long long* c = &h[4 * (sp * 2 * K_ + v)];
       q += (long long)c[0];
       pq += (long long)c[1];
-      fl += kernel_flops_form(v, v < K_ ? b->form[v] : 0, c);
+      fl += kernel_flops_form(v, v < K_ ? chosen_form(sqb::kClassKernels[v], b->form[v]) : 0, c);
     }
   long long pairs = 0, shells = 0;
   for (const sqb200_jk* c : b->mols) {
@@ -3139,7 +3175,7 @@ void grad_work(const sqb200_jk* c, const int* fat, const double* PT, double scre
       for (size_t sx = 0; sx + 1 < B.sub.size(); ++sx)
         for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
           const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
-          const int split = pass ? pick_split(nbp, nkp, chain / K.ops) : 0;
+          const int split = pass ? pick_split(nbp, nkp, chain / K.ops, false) : 0;
           const int kper = pass ? kGradCta / ((split & 0xffff) * (split >> 16)) : 0;
           int end = T.sub[sy + 1];
           for (int b = B.sub[sx]; b < B.sub[sx + 1]; ++b) {
@@ -3167,9 +3203,9 @@ void grad_work(const sqb200_jk* c, const int* fat, const double* PT, double scre
 // The class kernels on the context's streams (forked off c->stream and joined to it, as a
 // build's), each with its CTAs' bra records in at most 32 KB of shared memory at a time.
 int grad_launch(sqb200_jk* c, const GradWork& w, sqb::GradArgs a) {
-  int rc = ensure_side_streams(c);
+  int rc = ensure_side_streams(c, w.segs.size());
   if (rc) return rc;
-  const int nl = 1 + c->nside;
+  const int nl = lanes_for(c, w.segs.size());
   std::vector<double> load(nl, 0.0);
   if (nl > 1) {
     CUDA_OK(cudaEventRecord(c->ev_fork, c->stream));

@@ -40,6 +40,7 @@ struct ClassKernel {
   const void* fn_rs;
   const void* fn_us;
   int s_flops_prim, s_flops_flush, s_flops_quartet;
+  int dflt;               // FP64 form without autotuning: 0 narrow, 1 wide, 2 swapped
 };
 
 extern const ClassKernel kClassKernels[];

@@ -186,7 +186,7 @@ class JKEngine:
 
     def tiles(self):
         """Per class kernel: the FP64 form, 0 narrow tile, 1 wide tile, 2 swapped loop roles
-        (-1: the class has one form)."""
+        (-1: its default form, neither tuned nor set; also a class with one form)."""
         out = np.zeros(256, np.int32)
         n = _lib.sqb200_jk_tiles(self._ctx, out, len(out))
         if n < 0:
