@@ -1,0 +1,657 @@
+// generated by gen_fshell_kernels.py -- do not edit
+#include "../jk_generic_dev.cuh"
+
+extern "C" __global__ void __launch_bounds__(128)
+jkf_FF_1(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {
+  extern __shared__ double fsm[];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int ii = blockIdx.x * 4 + wp;
+  if (ii >= nitems) return;                     // whole warps leave
+  const sqb::FItem it = items[ii];
+  const int g = it.cg >> 16, s = lane / g, cc = lane - s * g, cd = (it.cg & 0xffff) + cc;
+  const sqb::GenPairRec A = a.pairs[it.bra];
+  const int kb = a.klist[it.k0 + min(s, it.cnt - 1)];   // idle lanes shadow the last ket
+  const sqb::GenPairRec B = a.pairs[kb];
+  const double r = A.schwarz * B.schwarz;
+  bool ok = s < it.cnt && !(r < a.b.cut_outer) && !(r < a.b.cut_fixed);
+  if (ok && r < a.b.dscreen_rmax) {
+    const bool bf = (A.P > B.P) || (A.P == B.P && A.Q >= B.Q);
+    const int P = bf ? A.P : B.P, Q = bf ? A.Q : B.Q, I = bf ? B.P : A.P, J = bf ? B.Q : A.Q;
+    const double* PM = a.b.PM; const int ns = a.b.ns;
+    const double mp = PM[P * ns + Q] + PM[I * ns + J] + PM[P * ns + I] + PM[P * ns + J] + PM[Q * ns + I] + PM[Q * ns + J];
+    ok = !(r * mp < a.b.cut_fixed);
+  }
+  if (!__any_sync(0xffffffffu, ok)) return;
+  const double deg = (A.P == A.Q ? 0.5 : 1.0) * (B.P == B.Q ? 0.5 : 1.0) * (kb == it.bra ? 0.5 : 1.0);
+  const int L = 6 + B.lP + B.lQ, S1 = L + 1, S2 = S1 * S1;   // uniform over the warp
+  double* __restrict__ box = fsm + wp * sqb::kFWarpDoubles + min(s, it.cnt - 1) * sqb::f_slot(L);   // [t][u][v], then the seeds
+  double* __restrict__ base = box + S1 * S2;
+  const bool mine = s < it.cnt;
+  const unsigned d = __ldg(a.desc + B.doff + cd);
+  const int cx = sqb::dsc(d, 0), dx = sqb::dsc(d, 1), cy = sqb::dsc(d, 2), dy = sqb::dsc(d, 3), cz = sqb::dsc(d, 4), dz = sqb::dsc(d, 5);
+  const int n1 = cy + dy + 1, n2 = cz + dz + 1, nk = (cx + dx + 1) * n1 * n2;
+  unsigned long long npq = 0, nfl = 0;
+  double o2_0 = 0.0;
+  double o2_1 = 0.0;
+  double o2_2 = 0.0;
+  double o2_3 = 0.0;
+  double o2_4 = 0.0;
+  double o2_5 = 0.0;
+  double o2_6 = 0.0;
+  double o2_7 = 0.0;
+  double o2_8 = 0.0;
+  double o2_9 = 0.0;
+  double o3_0 = 0.0;
+  double o3_1 = 0.0;
+  double o3_2 = 0.0;
+  double o3_3 = 0.0;
+  double o3_4 = 0.0;
+  double o3_5 = 0.0;
+  double o3_6 = 0.0;
+  double o3_7 = 0.0;
+  double o3_8 = 0.0;
+  double o3_9 = 0.0;
+  for (int i = 0; i < A.nprim; ++i) {
+    const double* pa = a.prims + (size_t)(A.poff + i) * sqb::kGenPrimStride;
+    const double p = pa[0], Px = pa[1], Py = pa[2], Pz = pa[3], kpa = pa[4];
+    double g000 = 0.0;
+    double g100 = 0.0;
+    double g010 = 0.0;
+    double g001 = 0.0;
+    double g200 = 0.0;
+    double g110 = 0.0;
+    double g101 = 0.0;
+    double g020 = 0.0;
+    double g011 = 0.0;
+    double g002 = 0.0;
+    double g300 = 0.0;
+    double g210 = 0.0;
+    double g201 = 0.0;
+    double g120 = 0.0;
+    double g111 = 0.0;
+    double g102 = 0.0;
+    double g030 = 0.0;
+    double g021 = 0.0;
+    double g012 = 0.0;
+    double g003 = 0.0;
+    double g400 = 0.0;
+    double g310 = 0.0;
+    double g301 = 0.0;
+    double g220 = 0.0;
+    double g211 = 0.0;
+    double g202 = 0.0;
+    double g130 = 0.0;
+    double g121 = 0.0;
+    double g112 = 0.0;
+    double g103 = 0.0;
+    double g040 = 0.0;
+    double g031 = 0.0;
+    double g022 = 0.0;
+    double g013 = 0.0;
+    double g004 = 0.0;
+    double g500 = 0.0;
+    double g410 = 0.0;
+    double g401 = 0.0;
+    double g320 = 0.0;
+    double g311 = 0.0;
+    double g302 = 0.0;
+    double g230 = 0.0;
+    double g221 = 0.0;
+    double g212 = 0.0;
+    double g203 = 0.0;
+    double g140 = 0.0;
+    double g131 = 0.0;
+    double g122 = 0.0;
+    double g113 = 0.0;
+    double g104 = 0.0;
+    double g050 = 0.0;
+    double g041 = 0.0;
+    double g032 = 0.0;
+    double g023 = 0.0;
+    double g014 = 0.0;
+    double g005 = 0.0;
+    double g600 = 0.0;
+    double g510 = 0.0;
+    double g501 = 0.0;
+    double g420 = 0.0;
+    double g411 = 0.0;
+    double g402 = 0.0;
+    double g330 = 0.0;
+    double g321 = 0.0;
+    double g312 = 0.0;
+    double g303 = 0.0;
+    double g240 = 0.0;
+    double g231 = 0.0;
+    double g222 = 0.0;
+    double g213 = 0.0;
+    double g204 = 0.0;
+    double g150 = 0.0;
+    double g141 = 0.0;
+    double g132 = 0.0;
+    double g123 = 0.0;
+    double g114 = 0.0;
+    double g105 = 0.0;
+    double g060 = 0.0;
+    double g051 = 0.0;
+    double g042 = 0.0;
+    double g033 = 0.0;
+    double g024 = 0.0;
+    double g015 = 0.0;
+    double g006 = 0.0;
+    bool any = false;
+    for (int j = 0; j < B.nprim; ++j) {          // one contraction length per warp
+      const double* pb = a.prims + (size_t)(B.poff + j) * sqb::kGenPrimStride;
+      const double q = pb[0], pq = p + q, rs = rsqrt(pq);
+      const bool live = ok && !(TWO_PI_2_5 * kpa * pb[4] * rs < PRIM_CUTOFF);
+      if (!__any_sync(0xffffffffu, live)) continue;
+      any = true;
+      if (live && cd == 0 && false) ++npq;
+      const double X = Px - pb[1], Y = Py - pb[2], Z = Pz - pb[3];
+      __syncwarp();                                // the previous step is done with the box
+      if (mine) sqb::f_seeds(L, p * q * (rs * rs), rs, X, Y, Z, a.boys, base, cc, g);
+      __syncwarp();
+      sqb::f_box(L, X, Y, Z, base, box, cc, g, mine);
+      if (live) {
+        const sqb::EView Ej(a.coef, pb, B);
+        const double *ex = Ej.ax(0, cx, dx), *ey = Ej.ax(1, cy, dy), *ez = Ej.ax(2, cz, dz);
+        const double w = Ej.w(cd);
+        int tau = 0, nu = 0, ph = 0;
+        for (int k = 0; k < nk; ++k) {
+          const double e0 = w * (__ldg(ex + tau) * __ldg(ey + nu)) * __ldg(ez + ph);
+          const double e = ((tau + nu + ph) & 1) ? -e0 : e0;
+          const double* __restrict__ R = box + tau * S2 + nu * S1 + ph;
+          { const double* __restrict__ x = R + 0 * S2 + 0 * S1;
+            g000 = fma(e, x[0], g000);
+            g001 = fma(e, x[1], g001);
+            g002 = fma(e, x[2], g002);
+            g003 = fma(e, x[3], g003);
+            g004 = fma(e, x[4], g004);
+            g005 = fma(e, x[5], g005);
+            g006 = fma(e, x[6], g006);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 1 * S1;
+            g010 = fma(e, x[0], g010);
+            g011 = fma(e, x[1], g011);
+            g012 = fma(e, x[2], g012);
+            g013 = fma(e, x[3], g013);
+            g014 = fma(e, x[4], g014);
+            g015 = fma(e, x[5], g015);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 2 * S1;
+            g020 = fma(e, x[0], g020);
+            g021 = fma(e, x[1], g021);
+            g022 = fma(e, x[2], g022);
+            g023 = fma(e, x[3], g023);
+            g024 = fma(e, x[4], g024);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 3 * S1;
+            g030 = fma(e, x[0], g030);
+            g031 = fma(e, x[1], g031);
+            g032 = fma(e, x[2], g032);
+            g033 = fma(e, x[3], g033);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 4 * S1;
+            g040 = fma(e, x[0], g040);
+            g041 = fma(e, x[1], g041);
+            g042 = fma(e, x[2], g042);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 5 * S1;
+            g050 = fma(e, x[0], g050);
+            g051 = fma(e, x[1], g051);
+          }
+          { const double* __restrict__ x = R + 0 * S2 + 6 * S1;
+            g060 = fma(e, x[0], g060);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 0 * S1;
+            g100 = fma(e, x[0], g100);
+            g101 = fma(e, x[1], g101);
+            g102 = fma(e, x[2], g102);
+            g103 = fma(e, x[3], g103);
+            g104 = fma(e, x[4], g104);
+            g105 = fma(e, x[5], g105);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 1 * S1;
+            g110 = fma(e, x[0], g110);
+            g111 = fma(e, x[1], g111);
+            g112 = fma(e, x[2], g112);
+            g113 = fma(e, x[3], g113);
+            g114 = fma(e, x[4], g114);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 2 * S1;
+            g120 = fma(e, x[0], g120);
+            g121 = fma(e, x[1], g121);
+            g122 = fma(e, x[2], g122);
+            g123 = fma(e, x[3], g123);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 3 * S1;
+            g130 = fma(e, x[0], g130);
+            g131 = fma(e, x[1], g131);
+            g132 = fma(e, x[2], g132);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 4 * S1;
+            g140 = fma(e, x[0], g140);
+            g141 = fma(e, x[1], g141);
+          }
+          { const double* __restrict__ x = R + 1 * S2 + 5 * S1;
+            g150 = fma(e, x[0], g150);
+          }
+          { const double* __restrict__ x = R + 2 * S2 + 0 * S1;
+            g200 = fma(e, x[0], g200);
+            g201 = fma(e, x[1], g201);
+            g202 = fma(e, x[2], g202);
+            g203 = fma(e, x[3], g203);
+            g204 = fma(e, x[4], g204);
+          }
+          { const double* __restrict__ x = R + 2 * S2 + 1 * S1;
+            g210 = fma(e, x[0], g210);
+            g211 = fma(e, x[1], g211);
+            g212 = fma(e, x[2], g212);
+            g213 = fma(e, x[3], g213);
+          }
+          { const double* __restrict__ x = R + 2 * S2 + 2 * S1;
+            g220 = fma(e, x[0], g220);
+            g221 = fma(e, x[1], g221);
+            g222 = fma(e, x[2], g222);
+          }
+          { const double* __restrict__ x = R + 2 * S2 + 3 * S1;
+            g230 = fma(e, x[0], g230);
+            g231 = fma(e, x[1], g231);
+          }
+          { const double* __restrict__ x = R + 2 * S2 + 4 * S1;
+            g240 = fma(e, x[0], g240);
+          }
+          { const double* __restrict__ x = R + 3 * S2 + 0 * S1;
+            g300 = fma(e, x[0], g300);
+            g301 = fma(e, x[1], g301);
+            g302 = fma(e, x[2], g302);
+            g303 = fma(e, x[3], g303);
+          }
+          { const double* __restrict__ x = R + 3 * S2 + 1 * S1;
+            g310 = fma(e, x[0], g310);
+            g311 = fma(e, x[1], g311);
+            g312 = fma(e, x[2], g312);
+          }
+          { const double* __restrict__ x = R + 3 * S2 + 2 * S1;
+            g320 = fma(e, x[0], g320);
+            g321 = fma(e, x[1], g321);
+          }
+          { const double* __restrict__ x = R + 3 * S2 + 3 * S1;
+            g330 = fma(e, x[0], g330);
+          }
+          { const double* __restrict__ x = R + 4 * S2 + 0 * S1;
+            g400 = fma(e, x[0], g400);
+            g401 = fma(e, x[1], g401);
+            g402 = fma(e, x[2], g402);
+          }
+          { const double* __restrict__ x = R + 4 * S2 + 1 * S1;
+            g410 = fma(e, x[0], g410);
+            g411 = fma(e, x[1], g411);
+          }
+          { const double* __restrict__ x = R + 4 * S2 + 2 * S1;
+            g420 = fma(e, x[0], g420);
+          }
+          { const double* __restrict__ x = R + 5 * S2 + 0 * S1;
+            g500 = fma(e, x[0], g500);
+            g501 = fma(e, x[1], g501);
+          }
+          { const double* __restrict__ x = R + 5 * S2 + 1 * S1;
+            g510 = fma(e, x[0], g510);
+          }
+          { const double* __restrict__ x = R + 6 * S2 + 0 * S1;
+            g600 = fma(e, x[0], g600);
+          }
+          if (++ph == n2) { ph = 0; if (++nu == n1) { nu = 0; ++tau; } }
+        }
+        nfl += 2ull * 84 * nk;
+      }
+    }
+    if (!any) continue;
+    const sqb::EView Ei(a.coef, pa, A);
+    const double* __restrict__ E = Ei.e;
+    { double z = 0.0;
+      z = fma(__ldg(E + 21), fma(__ldg(E + 311), g003, fma(__ldg(E + 310), g002, fma(__ldg(E + 309), g001, __ldg(E + 308) * g000))), z);
+      z = fma(__ldg(E + 22), fma(__ldg(E + 311), g103, fma(__ldg(E + 310), g102, fma(__ldg(E + 309), g101, __ldg(E + 308) * g100))), z);
+      z = fma(__ldg(E + 23), fma(__ldg(E + 311), g203, fma(__ldg(E + 310), g202, fma(__ldg(E + 309), g201, __ldg(E + 308) * g200))), z);
+      z = fma(__ldg(E + 24), fma(__ldg(E + 311), g303, fma(__ldg(E + 310), g302, fma(__ldg(E + 309), g301, __ldg(E + 308) * g300))), z);
+      o2_0 = fma(Ei.w(20), z, o2_0); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 133), fma(__ldg(E + 311), g003, fma(__ldg(E + 310), g002, fma(__ldg(E + 309), g001, __ldg(E + 308) * g000))), z);
+      z = fma(__ldg(E + 134), fma(__ldg(E + 311), g013, fma(__ldg(E + 310), g012, fma(__ldg(E + 309), g011, __ldg(E + 308) * g010))), z);
+      z = fma(__ldg(E + 135), fma(__ldg(E + 311), g023, fma(__ldg(E + 310), g022, fma(__ldg(E + 309), g021, __ldg(E + 308) * g020))), z);
+      z = fma(__ldg(E + 136), fma(__ldg(E + 311), g033, fma(__ldg(E + 310), g032, fma(__ldg(E + 309), g031, __ldg(E + 308) * g030))), z);
+      o2_1 = fma(Ei.w(21), z, o2_1); }
+    { double z = 0.0;
+      z += fma(__ldg(E + 335), g006, fma(__ldg(E + 334), g005, fma(__ldg(E + 333), g004, fma(__ldg(E + 332), g003, fma(__ldg(E + 331), g002, fma(__ldg(E + 330), g001, __ldg(E + 329) * g000))))));
+      o2_2 = fma(Ei.w(22), z, o2_2); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 14) * __ldg(E + 119), fma(__ldg(E + 311), g003, fma(__ldg(E + 310), g002, fma(__ldg(E + 309), g001, __ldg(E + 308) * g000))), z);
+      z = fma(__ldg(E + 14) * __ldg(E + 120), fma(__ldg(E + 311), g013, fma(__ldg(E + 310), g012, fma(__ldg(E + 309), g011, __ldg(E + 308) * g010))), z);
+      z = fma(__ldg(E + 15) * __ldg(E + 119), fma(__ldg(E + 311), g103, fma(__ldg(E + 310), g102, fma(__ldg(E + 309), g101, __ldg(E + 308) * g100))), z);
+      z = fma(__ldg(E + 15) * __ldg(E + 120), fma(__ldg(E + 311), g113, fma(__ldg(E + 310), g112, fma(__ldg(E + 309), g111, __ldg(E + 308) * g110))), z);
+      z = fma(__ldg(E + 16) * __ldg(E + 119), fma(__ldg(E + 311), g203, fma(__ldg(E + 310), g202, fma(__ldg(E + 309), g201, __ldg(E + 308) * g200))), z);
+      z = fma(__ldg(E + 16) * __ldg(E + 120), fma(__ldg(E + 311), g213, fma(__ldg(E + 310), g212, fma(__ldg(E + 309), g211, __ldg(E + 308) * g210))), z);
+      o2_3 = fma(Ei.w(23), z, o2_3); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 7) * __ldg(E + 126), fma(__ldg(E + 311), g003, fma(__ldg(E + 310), g002, fma(__ldg(E + 309), g001, __ldg(E + 308) * g000))), z);
+      z = fma(__ldg(E + 7) * __ldg(E + 127), fma(__ldg(E + 311), g013, fma(__ldg(E + 310), g012, fma(__ldg(E + 309), g011, __ldg(E + 308) * g010))), z);
+      z = fma(__ldg(E + 7) * __ldg(E + 128), fma(__ldg(E + 311), g023, fma(__ldg(E + 310), g022, fma(__ldg(E + 309), g021, __ldg(E + 308) * g020))), z);
+      z = fma(__ldg(E + 8) * __ldg(E + 126), fma(__ldg(E + 311), g103, fma(__ldg(E + 310), g102, fma(__ldg(E + 309), g101, __ldg(E + 308) * g100))), z);
+      z = fma(__ldg(E + 8) * __ldg(E + 127), fma(__ldg(E + 311), g113, fma(__ldg(E + 310), g112, fma(__ldg(E + 309), g111, __ldg(E + 308) * g110))), z);
+      z = fma(__ldg(E + 8) * __ldg(E + 128), fma(__ldg(E + 311), g123, fma(__ldg(E + 310), g122, fma(__ldg(E + 309), g121, __ldg(E + 308) * g120))), z);
+      o2_4 = fma(Ei.w(24), z, o2_4); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 14), fma(__ldg(E + 319), g004, fma(__ldg(E + 318), g003, fma(__ldg(E + 317), g002, fma(__ldg(E + 316), g001, __ldg(E + 315) * g000)))), z);
+      z = fma(__ldg(E + 15), fma(__ldg(E + 319), g104, fma(__ldg(E + 318), g103, fma(__ldg(E + 317), g102, fma(__ldg(E + 316), g101, __ldg(E + 315) * g100)))), z);
+      z = fma(__ldg(E + 16), fma(__ldg(E + 319), g204, fma(__ldg(E + 318), g203, fma(__ldg(E + 317), g202, fma(__ldg(E + 316), g201, __ldg(E + 315) * g200)))), z);
+      o2_5 = fma(Ei.w(25), z, o2_5); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 7), fma(__ldg(E + 327), g005, fma(__ldg(E + 326), g004, fma(__ldg(E + 325), g003, fma(__ldg(E + 324), g002, fma(__ldg(E + 323), g001, __ldg(E + 322) * g000))))), z);
+      z = fma(__ldg(E + 8), fma(__ldg(E + 327), g105, fma(__ldg(E + 326), g104, fma(__ldg(E + 325), g103, fma(__ldg(E + 324), g102, fma(__ldg(E + 323), g101, __ldg(E + 322) * g100))))), z);
+      o2_6 = fma(Ei.w(26), z, o2_6); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 126), fma(__ldg(E + 319), g004, fma(__ldg(E + 318), g003, fma(__ldg(E + 317), g002, fma(__ldg(E + 316), g001, __ldg(E + 315) * g000)))), z);
+      z = fma(__ldg(E + 127), fma(__ldg(E + 319), g014, fma(__ldg(E + 318), g013, fma(__ldg(E + 317), g012, fma(__ldg(E + 316), g011, __ldg(E + 315) * g010)))), z);
+      z = fma(__ldg(E + 128), fma(__ldg(E + 319), g024, fma(__ldg(E + 318), g023, fma(__ldg(E + 317), g022, fma(__ldg(E + 316), g021, __ldg(E + 315) * g020)))), z);
+      o2_7 = fma(Ei.w(27), z, o2_7); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 119), fma(__ldg(E + 327), g005, fma(__ldg(E + 326), g004, fma(__ldg(E + 325), g003, fma(__ldg(E + 324), g002, fma(__ldg(E + 323), g001, __ldg(E + 322) * g000))))), z);
+      z = fma(__ldg(E + 120), fma(__ldg(E + 327), g015, fma(__ldg(E + 326), g014, fma(__ldg(E + 325), g013, fma(__ldg(E + 324), g012, fma(__ldg(E + 323), g011, __ldg(E + 322) * g010))))), z);
+      o2_8 = fma(Ei.w(28), z, o2_8); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 7) * __ldg(E + 119), fma(__ldg(E + 319), g004, fma(__ldg(E + 318), g003, fma(__ldg(E + 317), g002, fma(__ldg(E + 316), g001, __ldg(E + 315) * g000)))), z);
+      z = fma(__ldg(E + 7) * __ldg(E + 120), fma(__ldg(E + 319), g014, fma(__ldg(E + 318), g013, fma(__ldg(E + 317), g012, fma(__ldg(E + 316), g011, __ldg(E + 315) * g010)))), z);
+      z = fma(__ldg(E + 8) * __ldg(E + 119), fma(__ldg(E + 319), g104, fma(__ldg(E + 318), g103, fma(__ldg(E + 317), g102, fma(__ldg(E + 316), g101, __ldg(E + 315) * g100)))), z);
+      z = fma(__ldg(E + 8) * __ldg(E + 120), fma(__ldg(E + 319), g114, fma(__ldg(E + 318), g113, fma(__ldg(E + 317), g112, fma(__ldg(E + 316), g111, __ldg(E + 315) * g110)))), z);
+      o2_9 = fma(Ei.w(29), z, o2_9); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 77) * __ldg(E + 140), g000, z);
+      z = fma(__ldg(E + 77) * __ldg(E + 141), g010, z);
+      z = fma(__ldg(E + 78) * __ldg(E + 140), g100, z);
+      z = fma(__ldg(E + 78) * __ldg(E + 141), g110, z);
+      z = fma(__ldg(E + 79) * __ldg(E + 140), g200, z);
+      z = fma(__ldg(E + 79) * __ldg(E + 141), g210, z);
+      z = fma(__ldg(E + 80) * __ldg(E + 140), g300, z);
+      z = fma(__ldg(E + 80) * __ldg(E + 141), g310, z);
+      z = fma(__ldg(E + 81) * __ldg(E + 140), g400, z);
+      z = fma(__ldg(E + 81) * __ldg(E + 141), g410, z);
+      z = fma(__ldg(E + 82) * __ldg(E + 140), g500, z);
+      z = fma(__ldg(E + 82) * __ldg(E + 141), g510, z);
+      o3_0 = fma(Ei.w(30), z, o3_0); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 56) * __ldg(E + 161), g000, z);
+      z = fma(__ldg(E + 56) * __ldg(E + 162), g010, z);
+      z = fma(__ldg(E + 56) * __ldg(E + 163), g020, z);
+      z = fma(__ldg(E + 56) * __ldg(E + 164), g030, z);
+      z = fma(__ldg(E + 56) * __ldg(E + 165), g040, z);
+      z = fma(__ldg(E + 57) * __ldg(E + 161), g100, z);
+      z = fma(__ldg(E + 57) * __ldg(E + 162), g110, z);
+      z = fma(__ldg(E + 57) * __ldg(E + 163), g120, z);
+      z = fma(__ldg(E + 57) * __ldg(E + 164), g130, z);
+      z = fma(__ldg(E + 57) * __ldg(E + 165), g140, z);
+      z = fma(__ldg(E + 58) * __ldg(E + 161), g200, z);
+      z = fma(__ldg(E + 58) * __ldg(E + 162), g210, z);
+      z = fma(__ldg(E + 58) * __ldg(E + 163), g220, z);
+      z = fma(__ldg(E + 58) * __ldg(E + 164), g230, z);
+      z = fma(__ldg(E + 58) * __ldg(E + 165), g240, z);
+      o3_1 = fma(Ei.w(31), z, o3_1); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 56) * __ldg(E + 140), fma(__ldg(E + 248), g003, fma(__ldg(E + 247), g002, fma(__ldg(E + 246), g001, __ldg(E + 245) * g000))), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 141), fma(__ldg(E + 248), g013, fma(__ldg(E + 247), g012, fma(__ldg(E + 246), g011, __ldg(E + 245) * g010))), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 140), fma(__ldg(E + 248), g103, fma(__ldg(E + 247), g102, fma(__ldg(E + 246), g101, __ldg(E + 245) * g100))), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 141), fma(__ldg(E + 248), g113, fma(__ldg(E + 247), g112, fma(__ldg(E + 246), g111, __ldg(E + 245) * g110))), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 140), fma(__ldg(E + 248), g203, fma(__ldg(E + 247), g202, fma(__ldg(E + 246), g201, __ldg(E + 245) * g200))), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 141), fma(__ldg(E + 248), g213, fma(__ldg(E + 247), g212, fma(__ldg(E + 246), g211, __ldg(E + 245) * g210))), z);
+      o3_2 = fma(Ei.w(32), z, o3_2); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 70) * __ldg(E + 147), g000, z);
+      z = fma(__ldg(E + 70) * __ldg(E + 148), g010, z);
+      z = fma(__ldg(E + 70) * __ldg(E + 149), g020, z);
+      z = fma(__ldg(E + 71) * __ldg(E + 147), g100, z);
+      z = fma(__ldg(E + 71) * __ldg(E + 148), g110, z);
+      z = fma(__ldg(E + 71) * __ldg(E + 149), g120, z);
+      z = fma(__ldg(E + 72) * __ldg(E + 147), g200, z);
+      z = fma(__ldg(E + 72) * __ldg(E + 148), g210, z);
+      z = fma(__ldg(E + 72) * __ldg(E + 149), g220, z);
+      z = fma(__ldg(E + 73) * __ldg(E + 147), g300, z);
+      z = fma(__ldg(E + 73) * __ldg(E + 148), g310, z);
+      z = fma(__ldg(E + 73) * __ldg(E + 149), g320, z);
+      z = fma(__ldg(E + 74) * __ldg(E + 147), g400, z);
+      z = fma(__ldg(E + 74) * __ldg(E + 148), g410, z);
+      z = fma(__ldg(E + 74) * __ldg(E + 149), g420, z);
+      o3_3 = fma(Ei.w(33), z, o3_3); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 63) * __ldg(E + 154), g000, z);
+      z = fma(__ldg(E + 63) * __ldg(E + 155), g010, z);
+      z = fma(__ldg(E + 63) * __ldg(E + 156), g020, z);
+      z = fma(__ldg(E + 63) * __ldg(E + 157), g030, z);
+      z = fma(__ldg(E + 64) * __ldg(E + 154), g100, z);
+      z = fma(__ldg(E + 64) * __ldg(E + 155), g110, z);
+      z = fma(__ldg(E + 64) * __ldg(E + 156), g120, z);
+      z = fma(__ldg(E + 64) * __ldg(E + 157), g130, z);
+      z = fma(__ldg(E + 65) * __ldg(E + 154), g200, z);
+      z = fma(__ldg(E + 65) * __ldg(E + 155), g210, z);
+      z = fma(__ldg(E + 65) * __ldg(E + 156), g220, z);
+      z = fma(__ldg(E + 65) * __ldg(E + 157), g230, z);
+      z = fma(__ldg(E + 66) * __ldg(E + 154), g300, z);
+      z = fma(__ldg(E + 66) * __ldg(E + 155), g310, z);
+      z = fma(__ldg(E + 66) * __ldg(E + 156), g320, z);
+      z = fma(__ldg(E + 66) * __ldg(E + 157), g330, z);
+      o3_4 = fma(Ei.w(34), z, o3_4); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 70) * __ldg(E + 140), fma(__ldg(E + 232), g001, __ldg(E + 231) * g000), z);
+      z = fma(__ldg(E + 70) * __ldg(E + 141), fma(__ldg(E + 232), g011, __ldg(E + 231) * g010), z);
+      z = fma(__ldg(E + 71) * __ldg(E + 140), fma(__ldg(E + 232), g101, __ldg(E + 231) * g100), z);
+      z = fma(__ldg(E + 71) * __ldg(E + 141), fma(__ldg(E + 232), g111, __ldg(E + 231) * g110), z);
+      z = fma(__ldg(E + 72) * __ldg(E + 140), fma(__ldg(E + 232), g201, __ldg(E + 231) * g200), z);
+      z = fma(__ldg(E + 72) * __ldg(E + 141), fma(__ldg(E + 232), g211, __ldg(E + 231) * g210), z);
+      z = fma(__ldg(E + 73) * __ldg(E + 140), fma(__ldg(E + 232), g301, __ldg(E + 231) * g300), z);
+      z = fma(__ldg(E + 73) * __ldg(E + 141), fma(__ldg(E + 232), g311, __ldg(E + 231) * g310), z);
+      z = fma(__ldg(E + 74) * __ldg(E + 140), fma(__ldg(E + 232), g401, __ldg(E + 231) * g400), z);
+      z = fma(__ldg(E + 74) * __ldg(E + 141), fma(__ldg(E + 232), g411, __ldg(E + 231) * g410), z);
+      o3_5 = fma(Ei.w(35), z, o3_5); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 63) * __ldg(E + 140), fma(__ldg(E + 240), g002, fma(__ldg(E + 239), g001, __ldg(E + 238) * g000)), z);
+      z = fma(__ldg(E + 63) * __ldg(E + 141), fma(__ldg(E + 240), g012, fma(__ldg(E + 239), g011, __ldg(E + 238) * g010)), z);
+      z = fma(__ldg(E + 64) * __ldg(E + 140), fma(__ldg(E + 240), g102, fma(__ldg(E + 239), g101, __ldg(E + 238) * g100)), z);
+      z = fma(__ldg(E + 64) * __ldg(E + 141), fma(__ldg(E + 240), g112, fma(__ldg(E + 239), g111, __ldg(E + 238) * g110)), z);
+      z = fma(__ldg(E + 65) * __ldg(E + 140), fma(__ldg(E + 240), g202, fma(__ldg(E + 239), g201, __ldg(E + 238) * g200)), z);
+      z = fma(__ldg(E + 65) * __ldg(E + 141), fma(__ldg(E + 240), g212, fma(__ldg(E + 239), g211, __ldg(E + 238) * g210)), z);
+      z = fma(__ldg(E + 66) * __ldg(E + 140), fma(__ldg(E + 240), g302, fma(__ldg(E + 239), g301, __ldg(E + 238) * g300)), z);
+      z = fma(__ldg(E + 66) * __ldg(E + 141), fma(__ldg(E + 240), g312, fma(__ldg(E + 239), g311, __ldg(E + 238) * g310)), z);
+      o3_6 = fma(Ei.w(36), z, o3_6); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 56) * __ldg(E + 154), fma(__ldg(E + 232), g001, __ldg(E + 231) * g000), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 155), fma(__ldg(E + 232), g011, __ldg(E + 231) * g010), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 156), fma(__ldg(E + 232), g021, __ldg(E + 231) * g020), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 157), fma(__ldg(E + 232), g031, __ldg(E + 231) * g030), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 154), fma(__ldg(E + 232), g101, __ldg(E + 231) * g100), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 155), fma(__ldg(E + 232), g111, __ldg(E + 231) * g110), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 156), fma(__ldg(E + 232), g121, __ldg(E + 231) * g120), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 157), fma(__ldg(E + 232), g131, __ldg(E + 231) * g130), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 154), fma(__ldg(E + 232), g201, __ldg(E + 231) * g200), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 155), fma(__ldg(E + 232), g211, __ldg(E + 231) * g210), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 156), fma(__ldg(E + 232), g221, __ldg(E + 231) * g220), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 157), fma(__ldg(E + 232), g231, __ldg(E + 231) * g230), z);
+      o3_7 = fma(Ei.w(37), z, o3_7); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 56) * __ldg(E + 147), fma(__ldg(E + 240), g002, fma(__ldg(E + 239), g001, __ldg(E + 238) * g000)), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 148), fma(__ldg(E + 240), g012, fma(__ldg(E + 239), g011, __ldg(E + 238) * g010)), z);
+      z = fma(__ldg(E + 56) * __ldg(E + 149), fma(__ldg(E + 240), g022, fma(__ldg(E + 239), g021, __ldg(E + 238) * g020)), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 147), fma(__ldg(E + 240), g102, fma(__ldg(E + 239), g101, __ldg(E + 238) * g100)), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 148), fma(__ldg(E + 240), g112, fma(__ldg(E + 239), g111, __ldg(E + 238) * g110)), z);
+      z = fma(__ldg(E + 57) * __ldg(E + 149), fma(__ldg(E + 240), g122, fma(__ldg(E + 239), g121, __ldg(E + 238) * g120)), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 147), fma(__ldg(E + 240), g202, fma(__ldg(E + 239), g201, __ldg(E + 238) * g200)), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 148), fma(__ldg(E + 240), g212, fma(__ldg(E + 239), g211, __ldg(E + 238) * g210)), z);
+      z = fma(__ldg(E + 58) * __ldg(E + 149), fma(__ldg(E + 240), g222, fma(__ldg(E + 239), g221, __ldg(E + 238) * g220)), z);
+      o3_8 = fma(Ei.w(38), z, o3_8); }
+    { double z = 0.0;
+      z = fma(__ldg(E + 63) * __ldg(E + 147), fma(__ldg(E + 232), g001, __ldg(E + 231) * g000), z);
+      z = fma(__ldg(E + 63) * __ldg(E + 148), fma(__ldg(E + 232), g011, __ldg(E + 231) * g010), z);
+      z = fma(__ldg(E + 63) * __ldg(E + 149), fma(__ldg(E + 232), g021, __ldg(E + 231) * g020), z);
+      z = fma(__ldg(E + 64) * __ldg(E + 147), fma(__ldg(E + 232), g101, __ldg(E + 231) * g100), z);
+      z = fma(__ldg(E + 64) * __ldg(E + 148), fma(__ldg(E + 232), g111, __ldg(E + 231) * g110), z);
+      z = fma(__ldg(E + 64) * __ldg(E + 149), fma(__ldg(E + 232), g121, __ldg(E + 231) * g120), z);
+      z = fma(__ldg(E + 65) * __ldg(E + 147), fma(__ldg(E + 232), g201, __ldg(E + 231) * g200), z);
+      z = fma(__ldg(E + 65) * __ldg(E + 148), fma(__ldg(E + 232), g211, __ldg(E + 231) * g210), z);
+      z = fma(__ldg(E + 65) * __ldg(E + 149), fma(__ldg(E + 232), g221, __ldg(E + 231) * g220), z);
+      z = fma(__ldg(E + 66) * __ldg(E + 147), fma(__ldg(E + 232), g301, __ldg(E + 231) * g300), z);
+      z = fma(__ldg(E + 66) * __ldg(E + 148), fma(__ldg(E + 232), g311, __ldg(E + 231) * g310), z);
+      z = fma(__ldg(E + 66) * __ldg(E + 149), fma(__ldg(E + 232), g321, __ldg(E + 231) * g320), z);
+      o3_9 = fma(Ei.w(39), z, o3_9); }
+    if (ok) nfl += 1064;
+  }
+  const int N = a.b.nbf, fP = A.fP, fQ = A.fQ;
+  const int fc = B.fP + cd / B.nfQ, fd = B.fQ + cd % B.nfQ;
+  const double* __restrict__ PT = a.b.PT;
+  const double s2 = 2.0 * deg;
+  if (ok) {
+    double z = 0.0;
+    z = fma(o2_0, __ldg(PT + (fP + 2) * N + fQ + 0), z);
+    z = fma(o2_1, __ldg(PT + (fP + 2) * N + fQ + 1), z);
+    z = fma(o2_2, __ldg(PT + (fP + 2) * N + fQ + 2), z);
+    z = fma(o2_3, __ldg(PT + (fP + 2) * N + fQ + 3), z);
+    z = fma(o2_4, __ldg(PT + (fP + 2) * N + fQ + 4), z);
+    z = fma(o2_5, __ldg(PT + (fP + 2) * N + fQ + 5), z);
+    z = fma(o2_6, __ldg(PT + (fP + 2) * N + fQ + 6), z);
+    z = fma(o2_7, __ldg(PT + (fP + 2) * N + fQ + 7), z);
+    z = fma(o2_8, __ldg(PT + (fP + 2) * N + fQ + 8), z);
+    z = fma(o2_9, __ldg(PT + (fP + 2) * N + fQ + 9), z);
+    z = fma(o3_0, __ldg(PT + (fP + 3) * N + fQ + 0), z);
+    z = fma(o3_1, __ldg(PT + (fP + 3) * N + fQ + 1), z);
+    z = fma(o3_2, __ldg(PT + (fP + 3) * N + fQ + 2), z);
+    z = fma(o3_3, __ldg(PT + (fP + 3) * N + fQ + 3), z);
+    z = fma(o3_4, __ldg(PT + (fP + 3) * N + fQ + 4), z);
+    z = fma(o3_5, __ldg(PT + (fP + 3) * N + fQ + 5), z);
+    z = fma(o3_6, __ldg(PT + (fP + 3) * N + fQ + 6), z);
+    z = fma(o3_7, __ldg(PT + (fP + 3) * N + fQ + 7), z);
+    z = fma(o3_8, __ldg(PT + (fP + 3) * N + fQ + 8), z);
+    z = fma(o3_9, __ldg(PT + (fP + 3) * N + fQ + 9), z);
+    atomicAdd(a.b.J + fc * N + fd, s2 * z);
+    for (int sp = 0; sp < (a.b.uhf ? 2 : 1); ++sp) {
+      const double* __restrict__ D = sp ? a.b.PB : a.b.PA;
+      double* __restrict__ K = sp ? a.b.KB : a.b.KA;
+      {  // K[p][c], K[q][c] from D[.][d]
+        const double q0 = D[(fQ + 0) * N + fd];
+        double kq0 = 0.0;
+        const double q1 = D[(fQ + 1) * N + fd];
+        double kq1 = 0.0;
+        const double q2 = D[(fQ + 2) * N + fd];
+        double kq2 = 0.0;
+        const double q3 = D[(fQ + 3) * N + fd];
+        double kq3 = 0.0;
+        const double q4 = D[(fQ + 4) * N + fd];
+        double kq4 = 0.0;
+        const double q5 = D[(fQ + 5) * N + fd];
+        double kq5 = 0.0;
+        const double q6 = D[(fQ + 6) * N + fd];
+        double kq6 = 0.0;
+        const double q7 = D[(fQ + 7) * N + fd];
+        double kq7 = 0.0;
+        const double q8 = D[(fQ + 8) * N + fd];
+        double kq8 = 0.0;
+        const double q9 = D[(fQ + 9) * N + fd];
+        double kq9 = 0.0;
+        { const double px = D[(fP + 2) * N + fd]; double kp = 0.0;
+          kp = fma(o2_0, q0, kp); kq0 = fma(o2_0, px, kq0);
+          kp = fma(o2_1, q1, kp); kq1 = fma(o2_1, px, kq1);
+          kp = fma(o2_2, q2, kp); kq2 = fma(o2_2, px, kq2);
+          kp = fma(o2_3, q3, kp); kq3 = fma(o2_3, px, kq3);
+          kp = fma(o2_4, q4, kp); kq4 = fma(o2_4, px, kq4);
+          kp = fma(o2_5, q5, kp); kq5 = fma(o2_5, px, kq5);
+          kp = fma(o2_6, q6, kp); kq6 = fma(o2_6, px, kq6);
+          kp = fma(o2_7, q7, kp); kq7 = fma(o2_7, px, kq7);
+          kp = fma(o2_8, q8, kp); kq8 = fma(o2_8, px, kq8);
+          kp = fma(o2_9, q9, kp); kq9 = fma(o2_9, px, kq9);
+          atomicAdd(K + (fP + 2) * N + fc, deg * kp); }
+        { const double px = D[(fP + 3) * N + fd]; double kp = 0.0;
+          kp = fma(o3_0, q0, kp); kq0 = fma(o3_0, px, kq0);
+          kp = fma(o3_1, q1, kp); kq1 = fma(o3_1, px, kq1);
+          kp = fma(o3_2, q2, kp); kq2 = fma(o3_2, px, kq2);
+          kp = fma(o3_3, q3, kp); kq3 = fma(o3_3, px, kq3);
+          kp = fma(o3_4, q4, kp); kq4 = fma(o3_4, px, kq4);
+          kp = fma(o3_5, q5, kp); kq5 = fma(o3_5, px, kq5);
+          kp = fma(o3_6, q6, kp); kq6 = fma(o3_6, px, kq6);
+          kp = fma(o3_7, q7, kp); kq7 = fma(o3_7, px, kq7);
+          kp = fma(o3_8, q8, kp); kq8 = fma(o3_8, px, kq8);
+          kp = fma(o3_9, q9, kp); kq9 = fma(o3_9, px, kq9);
+          atomicAdd(K + (fP + 3) * N + fc, deg * kp); }
+        atomicAdd(K + (fQ + 0) * N + fc, deg * kq0);
+        atomicAdd(K + (fQ + 1) * N + fc, deg * kq1);
+        atomicAdd(K + (fQ + 2) * N + fc, deg * kq2);
+        atomicAdd(K + (fQ + 3) * N + fc, deg * kq3);
+        atomicAdd(K + (fQ + 4) * N + fc, deg * kq4);
+        atomicAdd(K + (fQ + 5) * N + fc, deg * kq5);
+        atomicAdd(K + (fQ + 6) * N + fc, deg * kq6);
+        atomicAdd(K + (fQ + 7) * N + fc, deg * kq7);
+        atomicAdd(K + (fQ + 8) * N + fc, deg * kq8);
+        atomicAdd(K + (fQ + 9) * N + fc, deg * kq9);
+      }
+      {  // K[p][d], K[q][d] from D[.][c]
+        const double q0 = D[(fQ + 0) * N + fc];
+        double kq0 = 0.0;
+        const double q1 = D[(fQ + 1) * N + fc];
+        double kq1 = 0.0;
+        const double q2 = D[(fQ + 2) * N + fc];
+        double kq2 = 0.0;
+        const double q3 = D[(fQ + 3) * N + fc];
+        double kq3 = 0.0;
+        const double q4 = D[(fQ + 4) * N + fc];
+        double kq4 = 0.0;
+        const double q5 = D[(fQ + 5) * N + fc];
+        double kq5 = 0.0;
+        const double q6 = D[(fQ + 6) * N + fc];
+        double kq6 = 0.0;
+        const double q7 = D[(fQ + 7) * N + fc];
+        double kq7 = 0.0;
+        const double q8 = D[(fQ + 8) * N + fc];
+        double kq8 = 0.0;
+        const double q9 = D[(fQ + 9) * N + fc];
+        double kq9 = 0.0;
+        { const double px = D[(fP + 2) * N + fc]; double kp = 0.0;
+          kp = fma(o2_0, q0, kp); kq0 = fma(o2_0, px, kq0);
+          kp = fma(o2_1, q1, kp); kq1 = fma(o2_1, px, kq1);
+          kp = fma(o2_2, q2, kp); kq2 = fma(o2_2, px, kq2);
+          kp = fma(o2_3, q3, kp); kq3 = fma(o2_3, px, kq3);
+          kp = fma(o2_4, q4, kp); kq4 = fma(o2_4, px, kq4);
+          kp = fma(o2_5, q5, kp); kq5 = fma(o2_5, px, kq5);
+          kp = fma(o2_6, q6, kp); kq6 = fma(o2_6, px, kq6);
+          kp = fma(o2_7, q7, kp); kq7 = fma(o2_7, px, kq7);
+          kp = fma(o2_8, q8, kp); kq8 = fma(o2_8, px, kq8);
+          kp = fma(o2_9, q9, kp); kq9 = fma(o2_9, px, kq9);
+          atomicAdd(K + (fP + 2) * N + fd, deg * kp); }
+        { const double px = D[(fP + 3) * N + fc]; double kp = 0.0;
+          kp = fma(o3_0, q0, kp); kq0 = fma(o3_0, px, kq0);
+          kp = fma(o3_1, q1, kp); kq1 = fma(o3_1, px, kq1);
+          kp = fma(o3_2, q2, kp); kq2 = fma(o3_2, px, kq2);
+          kp = fma(o3_3, q3, kp); kq3 = fma(o3_3, px, kq3);
+          kp = fma(o3_4, q4, kp); kq4 = fma(o3_4, px, kq4);
+          kp = fma(o3_5, q5, kp); kq5 = fma(o3_5, px, kq5);
+          kp = fma(o3_6, q6, kp); kq6 = fma(o3_6, px, kq6);
+          kp = fma(o3_7, q7, kp); kq7 = fma(o3_7, px, kq7);
+          kp = fma(o3_8, q8, kp); kq8 = fma(o3_8, px, kq8);
+          kp = fma(o3_9, q9, kp); kq9 = fma(o3_9, px, kq9);
+          atomicAdd(K + (fP + 3) * N + fd, deg * kp); }
+        atomicAdd(K + (fQ + 0) * N + fd, deg * kq0);
+        atomicAdd(K + (fQ + 1) * N + fd, deg * kq1);
+        atomicAdd(K + (fQ + 2) * N + fd, deg * kq2);
+        atomicAdd(K + (fQ + 3) * N + fd, deg * kq3);
+        atomicAdd(K + (fQ + 4) * N + fd, deg * kq4);
+        atomicAdd(K + (fQ + 5) * N + fd, deg * kq5);
+        atomicAdd(K + (fQ + 6) * N + fd, deg * kq6);
+        atomicAdd(K + (fQ + 7) * N + fd, deg * kq7);
+        atomicAdd(K + (fQ + 8) * N + fd, deg * kq8);
+        atomicAdd(K + (fQ + 9) * N + fd, deg * kq9);
+      }
+    }
+    nfl += 2ull * 20 * (2 + 4 * (a.b.uhf ? 2 : 1));
+  }
+  {  // J[p][q]: every lane shares the bra pair
+    const double w = ok ? s2 * __ldg(PT + fc * N + fd) : 0.0;
+    { double v[32] = {w * o2_0, w * o2_1, w * o2_2, w * o2_3, w * o2_4, w * o2_5, w * o2_6, w * o2_7, w * o2_8, w * o2_9, w * o3_0, w * o3_1, w * o3_2, w * o3_3, w * o3_4, w * o3_5, w * o3_6, w * o3_7, w * o3_8, w * o3_9, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      const double z = sqb::warp_sum_scatter<32>(v); const int x = lane + 0;
+      if (lane < 20 && z != 0.0) atomicAdd(a.b.J + (fP + 2 + x / 10) * N + fQ + x % 10, z); }
+  }
+  sqb::count_add(a.counters + 0, ok && cd == 0 && false ? 1ull : 0ull);
+  sqb::count_add(a.counters + 1, npq);
+  sqb::count_add(a.counters + 2, nfl);
+}

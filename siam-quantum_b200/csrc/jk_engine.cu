@@ -345,6 +345,8 @@ struct sqb200_jk {
     int cta = 64;                 // threads per CTA of the class kernels
     sqb::GenItem* d_gitems = nullptr;   // the generic path's items (shells outside the classes)
     int gtotal = 0;
+    sqb::FItem* d_fitems = nullptr;     // the f-shell kernels' items, by class fseg[q] .. fseg[q + 1]
+    int fseg[6] = {0, 0, 0, 0, 0, 0};
   };
   // key: outer cutoff, fixed cutoff, FP32 threshold, multipole mode
   std::map<std::tuple<double, double, double, int>, Work> work;
@@ -1161,13 +1163,18 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
   }
   if (c->gen.on) {
     std::vector<sqb::GenItem> gi;
-    double gcost = 0.0;
-    sqb::gen_items(c->gen, outer, fixed, gi, gcost, mpm ? &er_run : nullptr);
-    if (gi.size() > (size_t)INT_MAX) return fail(SQB200_EINVAL, "generic path: more than 2^31 work items");
+    std::vector<sqb::FItem> fi;
+    sqb::gen_items(c->gen, outer, fixed, gi, fi, w.fseg, mpm ? &er_run : nullptr);
+    if (gi.size() > (size_t)INT_MAX || fi.size() > (size_t)INT_MAX)
+      return fail(SQB200_EINVAL, "generic path: more than 2^31 work items");
     w.gtotal = (int)gi.size();
     if (!gi.empty()) {
       CUDA_OK(cudaMalloc(&w.d_gitems, gi.size() * sizeof(sqb::GenItem)));
       CUDA_OK(h2d(w.d_gitems, gi.data(), gi.size() * sizeof(sqb::GenItem), c->stream));
+    }
+    if (!fi.empty()) {
+      CUDA_OK(cudaMalloc(&w.d_fitems, fi.size() * sizeof(sqb::FItem)));
+      CUDA_OK(h2d(w.d_fitems, fi.data(), fi.size() * sizeof(sqb::FItem), c->stream));
     }
   }
   if (mpm) {
@@ -1355,24 +1362,30 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   launch_pmax(dPA, dPB, c->d_PT, c->d_shfirst, c->d_shn, c->ns, n, c->d_PM, st);
   CUDA_OK(cudaMemsetAsync(c->d_counters, 0, sizeof(unsigned long long) * 8 * sqb::kNumClassKernels, st));
   if (c->persistent) CUDA_OK(cudaMemsetAsync(c->d_queue, 0, sizeof(unsigned long long) * 2 * sqb::kNumClassKernels, st));
-  c->last_launches = 3 + (int)w->kernel.size() + (w->gtotal > 0 ? 1 : 0);
+  int gsegs = w->gtotal > 0 ? 1 : 0;             // launches of the generic path
+  for (int k = 0; k < sqb::kNumFKernels; ++k) gsegs += w->fseg[sqb::kFKernels[k].q + 1] > w->fseg[sqb::kFKernels[k].q];
+  c->last_launches = 3 + (int)w->kernel.size() + gsegs;
   // segments largest first, each on the least-loaded lane (lane 0 = st, the others are side
   // streams forked off st); per-class profiling keeps every launch on st so that each event
   // pair times one kernel alone
-  rc = ensure_side_streams(c, w->kernel.size());
+  rc = ensure_side_streams(c, w->kernel.size() + gsegs);
   if (rc) return rc;
-  const int nlanes = c->profile ? 1 : lanes_for(c, w->kernel.size());
+  const int nlanes = c->profile ? 1 : lanes_for(c, w->kernel.size() + gsegs);
   std::vector<size_t> order(w->kernel.size());
   for (size_t s = 0; s < order.size(); ++s) order[s] = s;
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return w->cost[x] > w->cost[y]; });
   std::vector<double> load(nlanes, 0.0);
   std::vector<char> used(nlanes, 0);
+  if (c->gen.on) {
+    rc = sqb::gen_zero(c->gen, st);
+    if (rc) return rc;
+  }
   if (nlanes > 1) {
     CUDA_OK(cudaEventRecord(c->ev_fork, st));
     for (int l = 1; l < nlanes; ++l) CUDA_OK(cudaStreamWaitEvent(c->side[l - 1], c->ev_fork, 0));
   }
   if (c->gen.on) {
-    // the generic path's quartets (f shells), on lane 0 ahead of the class kernels
+    // the generic path's quartets (f shells), ahead of the class kernels
     sqb::GenBuild gb{dPA, dPB, c->d_PT, c->d_PM, c->d_J, c->d_KA, c->d_KB, n, c->ns, uhf, outer, fixed, dscreen,
                      nullptr, nullptr, nullptr, nullptr, 0.0};
     if (c->mp_on && c->d_erbank) {
@@ -1383,12 +1396,14 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
       gb.mp_rmax = c->mp_rmax;
     }
     sqb200_jk::Ev ev{kGenericKernel, nullptr, nullptr};
-    if (c->profile && w->gtotal > 0) {
+    if (c->profile && gsegs > 0) {
       CUDA_OK(cudaEventCreate(&ev.a));
       CUDA_OK(cudaEventCreate(&ev.b));
       CUDA_OK(cudaEventRecord(ev.a, st));
     }
-    rc = sqb::gen_launch(c->gen, w->d_gitems, w->gtotal, gb, st);
+    std::vector<cudaStream_t> lanes(1, st);
+    lanes.insert(lanes.end(), c->side.begin(), c->side.begin() + (nlanes - 1));
+    rc = sqb::gen_launch(c->gen, w->d_gitems, w->gtotal, w->d_fitems, w->fseg, gb, lanes.data(), nlanes);
     if (rc) return rc;
     if (ev.a) {
       CUDA_OK(cudaEventRecord(ev.b, st));
@@ -1632,7 +1647,7 @@ int sqb200_jk_destroy(sqb200_jk* c) {
     cudaEventDestroy(c->ev_join[i]);
   }
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-  for (auto& kv : c->work) { cudaFree(kv.second.d_items); cudaFree(kv.second.d_er); cudaFree(kv.second.d_gitems); }
+  for (auto& kv : c->work) { cudaFree(kv.second.d_items); cudaFree(kv.second.d_er); cudaFree(kv.second.d_gitems); cudaFree(kv.second.d_fitems); }
   sqb::gen_free(c->gen);
   if (c->d_mpbase) cudaFree(c->d_mpbase);
   if (c->d_erbase) cudaFree(c->d_erbase);

@@ -19,11 +19,15 @@
 // Boys-scaled seeds, two buffers of the R recursion (tetrahedral order t+u+v <= 12), and G and
 // the contracted block O for a chunk of ket function pairs (chunks when a (ff|ff)-sized block
 // does not fit).
-#include "jk_generic.cuh"
+#include "jk_generic_dev.cuh"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <set>
 #include <string>
 
 #include "jk_common.cuh"
@@ -41,34 +45,21 @@ using sqb::GenPairRec;
 using sqb::kGenPrimStride;
 
 using sqb::kGenBoysCols;
-constexpr int kGenR = 455;                             // tetrahedral entries with t+u+v <= 12
 constexpr int kGenWarps = 2;                           // warps per CTA
 constexpr int kGenKets = 16;                           // kets per work item
 constexpr int kGenGO = 1024;                           // doubles for G and O of one chunk
-constexpr int kGenWarpDoubles = 16 + 2 * kGenR + kGenGO;
+constexpr int kGenWarpDoubles = 16 + 2 * sqb::kGenR + kGenGO;
 constexpr size_t kGenSmem = (size_t)kGenWarps * kGenWarpDoubles * sizeof(double);   // 31,200 B
 
-static_assert(sqb::kGenMmax == 12 && (sqb::kGenMmax + 1) * (sqb::kGenMmax + 2) * (sqb::kGenMmax + 3) / 6 == kGenR,
-              "R table size");
+using sqb::dsc;
+using sqb::EView;
+using sqb::gen_boys;
+using sqb::gtet;
+using sqb::g_tuv;
+using sqb::kGenR;
+
 static_assert(sizeof(GenPairRec) == 56, "pair record layout");
 static_assert(kGenSmem <= 48 * 1024, "the generic kernels launch without a shared-memory opt-in");
-
-// (t, u, v) of tetrahedral index k: order n = t+u+v, then m = u+v, then v ascending
-struct TuvTable {
-  unsigned int v[kGenR];
-  constexpr TuvTable() : v() {
-    int k = 0;
-    for (int n = 0; n <= sqb::kGenMmax; ++n)
-      for (int m = 0; m <= n; ++m)
-        for (int w = 0; w <= m; ++w) v[k++] = (unsigned)(n - m) | ((unsigned)(m - w) << 8) | ((unsigned)w << 16);
-  }
-};
-__device__ const TuvTable g_tuv = TuvTable();
-
-__device__ __forceinline__ int gtet(int t, int u, int v) {
-  const int n = t + u + v, m = u + v;
-  return n * (n + 1) * (n + 2) / 6 + m * (m + 1) / 2 + v;
-}
 
 struct GenArgs {
   const GenPairRec* __restrict__ pairs;
@@ -79,42 +70,6 @@ struct GenArgs {
   sqb::GenBuild b;
   unsigned long long* counters;
 };
-
-// A primitive pair's tables in `coef`: axis d, E^{ij}_t at e + d*sz + (i*lq1 + j)*lt + t
-// (i <= lP, j <= lQ, t <= i+j; lq1 = lQ+1, lt = lP+lQ+1, sz = (lP+1) lq1 lt); then the weights
-// c_a c_b exp(-ab|AB|^2/p)/p of its function pairs at e + 3*sz.
-struct EView {
-  const double* e;
-  int lq1, lt, sz;
-  __device__ EView(const double* coef, const double* rec, const GenPairRec& P)
-      : e(coef + (long long)rec[11]), lq1(P.lQ + 1), lt(P.lP + P.lQ + 1), sz((P.lP + 1) * (P.lQ + 1) * (P.lP + P.lQ + 1)) {}
-  __device__ __forceinline__ const double* ax(int d, int i, int j) const { return e + d * sz + (i * lq1 + j) * lt; }
-  __device__ __forceinline__ double w(int ab) const { return __ldg(e + 3 * sz + ab); }
-};
-
-// component exponents of a function pair: a_x, b_x, a_y, b_y, a_z, b_z in 2 bits each
-__device__ __forceinline__ int dsc(unsigned d, int k) { return (d >> (2 * k)) & 3; }
-
-// F_n(T) for one order n <= 12: below BOYS_TMAX the 9-term Taylor expansion about the nearest
-// grid point, F_n(T0+d) = sum_k F_{n+k}(T0) (-d)^k / k!, from the table's own column n; above,
-// F_0 = sqrt(pi/T)/2 and the upward recursion F_{m+1} = ((2m+1) F_m - e^-T)/(2T).
-__device__ double gen_boys(int n, double T, const double* __restrict__ tab) {
-  if (T < BOYS_TMAX) {
-    const int g = __double2int_rn(T * BOYS_INV_H);
-    const double d = T - g * BOYS_H;
-    const double* row = tab + g * kGenBoysCols + n;
-    double s = __ldg(row + BOYS_NTAY - 1);
-    for (int k = BOYS_NTAY - 2; k >= 0; --k) s = fma(s, -d * (1.0 / (double)(k + 1)), __ldg(row + k));
-    return s;
-  }
-  const double it = 1.0 / T;
-  double F = 0.88622692545275801365 * sqrt(it);   // sqrt(pi)/2 / sqrt(T)
-  if (n > 0) {
-    const double e = exp(-T), h = 0.5 * it;
-    for (int m = 0; m < n; ++m) F = ((2 * m + 1) * F - e) * h;
-  }
-  return F;
-}
 
 // Seeds base[n] = 2 pi^(5/2)/sqrt(p+q) (-2 alpha)^n F_n(T), n <= L, one lane per order.
 __device__ __forceinline__ void gen_seeds(int L, double alpha, double rs, double T, const double* tab, double* base,
@@ -546,7 +501,28 @@ void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* 
   g.coef.clear();
   g.desc.clear();
   g.gen_idx.clear();
+  g.fclass.clear();
+  g.klist.clear();
+  g.kgroup.clear();
   const int ns = (int)sh.size();
+  // canonical layouts the f-shell kernels are generated for
+  auto layout = [&](const GenShell& x) {
+    static const int comp[5][10][3] = {
+        {{0, 0, 0}},
+        {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
+        {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}},
+        {{2, 0, 0}, {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1}},
+        {{3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0}, {1, 2, 0}, {2, 0, 1}, {1, 0, 2}, {0, 2, 1}, {0, 1, 2}, {1, 1, 1}}};
+    static const int n[5] = {1, 4, 3, 6, 10};
+    for (int k = 0; k < 5; ++k) {
+      if (x.nfunc != n[k]) continue;
+      bool same = true;
+      for (int f = 0; f < n[k]; ++f)
+        for (int d = 0; d < 3; ++d) same = same && x.lmn[3 * f + d] == comp[k][f][d];
+      if (same) return k;
+    }
+    return -1;
+  };
   struct Tmp { double s; int P, Q; };
   std::vector<Tmp> all;
   all.reserve((size_t)ns * (ns + 1) / 2);
@@ -599,12 +575,40 @@ void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* 
         for (int fa = 0; fa < A.nfunc; ++fa)
           for (int fb = 0; fb < B.nfunc; ++fb) g.coef.push_back(A.coef[i * 16 + fa] * B.coef[j * 16 + fb] * kp);
       }
-    if (rec.gen) g.gen_idx.push_back((int)g.pairs.size());
+    if (rec.gen) {
+      g.gen_idx.push_back((int)g.pairs.size());
+      g.fclass.push_back(layout(A) == 4 ? layout(B) : -1);
+    }
     g.pairs.push_back(rec);
   }
+  std::map<std::array<int, 6>, std::vector<int>> groups;
+  for (int k = 0; k < (int)g.pairs.size(); ++k) {
+    const GenPairRec& r = g.pairs[k];
+    groups[{r.nfP, r.nfQ, r.lP, r.lQ, r.nprim, r.gen}].push_back(k);
+  }
+  for (const auto& kv : groups) {
+    g.kgroup.push_back((int)g.klist.size());
+    g.klist.insert(g.klist.end(), kv.second.begin(), kv.second.end());
+  }
+  g.kgroup.push_back((int)g.klist.size());
 }
 
 int gen_upload(GenPath& g, cudaStream_t st) {
+  // the f-shell kernels' shared memory is above the default limit: raised once per device
+  {
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (e == cudaSuccess && !done.count(dev)) {
+      for (int k = 0; k < kNumFKernels && e == cudaSuccess; ++k)
+        e = cudaFuncSetAttribute(kFKernels[k].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kFWarps * kFWarpDoubles * (int)sizeof(double));
+      if (e == cudaSuccess) done.insert(dev);
+    }
+    if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("f-shell kernels: ") + cudaGetErrorString(e));
+  }
   const std::vector<double> tab = boys_table(kGenBoysCols);
   struct Slot { void** dst; size_t bytes; const void* src; };
   const Slot slots[] = {
@@ -613,6 +617,7 @@ int gen_upload(GenPath& g, cudaStream_t st) {
       {(void**)&g.d_coef, g.coef.size() * sizeof(double), g.coef.data()},
       {(void**)&g.d_desc, g.desc.size() * sizeof(int), g.desc.data()},
       {(void**)&g.d_gen_idx, g.gen_idx.size() * sizeof(int), g.gen_idx.data()},
+      {(void**)&g.d_klist, g.klist.size() * sizeof(int), g.klist.data()},
       {(void**)&g.d_boys, tab.size() * sizeof(double), tab.data()},
       {(void**)&g.d_counters, 3 * sizeof(unsigned long long), nullptr},
   };
@@ -651,8 +656,26 @@ int gen_schwarz(const GenPath& g, int nbf, double* S, cudaStream_t st) {
   return SQB200_OK;
 }
 
-void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, double& cost,
-               long long* er_run) {
+// The lanes' function pairs of a ket of n: chunks (c0, g), one lane each, 32 / g kets side by side.
+// Up to 16 at once; a larger rest as 16 and a rest of at most 8 when that fills the warps better
+// (18 = 16 + 2, 24 = 16 + 8), else whole.
+static void f_chunks(int n, std::vector<std::pair<int, int>>& out) {
+  out.clear();
+  int c0 = 0;
+  while (n - c0 > 32) {
+    out.push_back({c0, 32});
+    c0 += 32;
+  }
+  const int rest = n - c0;
+  if (rest > 16 && rest <= 24) {
+    out.push_back({c0, 16});
+    c0 += 16;
+  }
+  if (n > c0) out.push_back({c0, n - c0});
+}
+
+void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, std::vector<FItem>& fitems,
+               int fseg[6], long long* er_run) {
   const double cut = std::max(outer, fixed);
   const int np = (int)g.pairs.size();
   // kets with schwarz >= c / S(A) (less a relative 1e-12 that the kernel's exact test takes
@@ -666,7 +689,10 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
     }
     return lo;
   };
-  for (int a : g.gen_idx) {
+  std::vector<FItem> seg[5];
+  std::vector<std::pair<int, int>> chunks;
+  for (size_t x = 0; x < g.gen_idx.size(); ++x) {
+    const int a = g.gen_idx[x];
     const GenPairRec& A = g.pairs[a];
     if (!(A.schwarz > 0.0)) continue;
     const int lo = prefix(cut, A.schwarz);
@@ -675,20 +701,65 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
       er = (int)*er_run;
       *er_run += prefix(outer, A.schwarz);
     }
-    for (int k0 = 0; k0 < lo; k0 += kGenKets) items.push_back({a, k0, std::min(kGenKets, lo - k0), er});
-    cost += (double)lo * A.nprim * A.nfP * A.nfQ * 200.0;
+    if (er_run || g.fclass[x] < 0) {
+      for (int k0 = 0; k0 < lo; k0 += kGenKets) items.push_back({a, k0, std::min(kGenKets, lo - k0), er});
+      continue;
+    }
+    for (size_t k = 0; k + 1 < g.kgroup.size(); ++k) {
+      const int *b = g.klist.data() + g.kgroup[k], *e = g.klist.data() + g.kgroup[k + 1];
+      const GenPairRec& B = g.pairs[*b];
+      if (B.gen) b = std::lower_bound(b, e, a);   // two generic pairs: taken once, from the earlier position
+      e = std::lower_bound(b, e, lo);
+      if (b >= e) continue;
+      const int L = A.lP + A.lQ + B.lP + B.lQ;
+      f_chunks(B.nfP * B.nfQ, chunks);
+      for (const auto& c : chunks) {
+        const int ng = std::max(1, std::min(32 / c.second, kFWarpDoubles / f_slot(L)));
+        for (const int* q = b; q < e; q += ng)
+          seg[g.fclass[x]].push_back({a, (int)(q - g.klist.data()), (int)std::min<long>(ng, e - q), c.first | c.second << 16});
+      }
+    }
+  }
+  // heaviest primitive loops and largest kets first
+  fseg[0] = 0;
+  for (int q = 0; q < 5; ++q) {
+    auto key = [&](const FItem& it) {
+      const GenPairRec &A = g.pairs[it.bra], &B = g.pairs[g.klist[it.k0]];
+      return (long long)A.nprim * B.nprim * (20 + B.nfP * B.nfQ);
+    };
+    std::stable_sort(seg[q].begin(), seg[q].end(), [&](const FItem& x, const FItem& y) { return key(x) > key(y); });
+    fitems.insert(fitems.end(), seg[q].begin(), seg[q].end());
+    fseg[q + 1] = (int)fitems.size();
   }
 }
 
-int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const GenBuild& b, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(g.d_counters, 0, 3 * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("generic counters: ") + cudaGetErrorString(e));
-  if (nitems <= 0) return SQB200_OK;
-  GenArgs a = make_args(g);
-  a.b = b;
-  k_jk_gen<<<nitems, 32 * kGenWarps, kGenSmem, st>>>(a, d_items);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("k_jk_gen: ") + cudaGetErrorString(e));
+int gen_zero(const GenPath& g, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(g.d_counters, 0, 3 * sizeof(unsigned long long), st);
+  return e == cudaSuccess ? SQB200_OK : set_error(SQB200_ECUDA, std::string("generic counters: ") + cudaGetErrorString(e));
+}
+
+int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FItem* d_fitems, const int fseg[6],
+               const GenBuild& b, const cudaStream_t* lanes, int nlanes) {
+  cudaError_t e = cudaSuccess;
+  if (nitems > 0) {
+    GenArgs a = make_args(g);
+    a.b = b;
+    k_jk_gen<<<nitems, 32 * kGenWarps, kGenSmem, lanes[0]>>>(a, d_items);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("k_jk_gen: ") + cudaGetErrorString(e));
+  }
+  FArgs f{g.d_pairs, g.d_prims, g.d_coef, g.d_desc, g.d_klist, g.d_boys, b, g.d_counters};
+  int lane = 0;
+  for (int k = kNumFKernels - 1; k >= 0; --k) {      // the largest bras first
+    const int q = kFKernels[k].q;
+    int n = fseg[q + 1] - fseg[q];
+    if (n <= 0) continue;
+    const FItem* items = d_fitems + fseg[q];
+    void* args[] = {&f, &items, &n};
+    e = cudaLaunchKernel(kFKernels[k].fn, dim3((n + kFWarps - 1) / kFWarps), dim3(32 * kFWarps), args,
+                         kFWarps * kFWarpDoubles * sizeof(double), lanes[lane++ % nlanes]);
+    if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("f-shell kernel: ") + cudaGetErrorString(e));
+  }
   return SQB200_OK;
 }
 
@@ -701,6 +772,7 @@ void gen_free(GenPath& g) {
   g.d_coef = nullptr;
   g.d_desc = nullptr;
   g.d_gen_idx = nullptr;
+  g.d_klist = nullptr;
   g.d_boys = nullptr;
   g.d_counters = nullptr;
 }

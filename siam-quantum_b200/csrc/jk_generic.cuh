@@ -46,6 +46,18 @@ struct GenItem {
   int bra, k0, cnt, er;
 };
 
+// A warp's unit of the f-shell kernels (gen_fshell_kernels.py): one bra pair and the cnt ket pairs
+// klist[k0 ..], g function pairs from c0 of each (cg = c0 | g << 16), one lane per function pair.
+struct FItem {
+  int bra, k0, cnt, cg;
+};
+
+// Shared memory of one warp of the f-shell kernels (doubles), and of one quartet of total order L:
+// the box of R and its seeds.  16 KB a warp holds a box of order 11; (ff|ff), order 12, needs 17.3 KB.
+constexpr int kFWarps = 4;
+constexpr int kFWarpDoubles = 2212;
+constexpr __host__ __device__ int f_slot(int L) { return ((L + 1) * (L + 1) * (L + 1) + L + 1) | 1; }
+
 struct GenPath {
   bool on = false;                  // the basis has generic shells
   std::vector<GenPairRec> pairs;    // every shell pair, by decreasing Schwarz bound
@@ -53,6 +65,12 @@ struct GenPath {
   std::vector<double> coef;         // per primitive pair: its 1-D Hermite tables, then its weights
   std::vector<int> desc;            // per pair: one component descriptor per function pair
   std::vector<int> gen_idx;         // positions of the generic pairs in `pairs`
+  // f-shell kernels: per generic pair (as gen_idx) the class of its second shell (0 s, 1 sp, 2 p, 3 d,
+  // 4 f) when both shells have the canonical layouts and the first is an f shell, else -1; every
+  // pair by ket group (function counts, angular momenta, contraction length), positions ascending
+  std::vector<int> fclass;
+  std::vector<int> klist;
+  std::vector<int> kgroup;          // starts of the groups in klist, and the end
   // device (one allocation)
   void* d_base = nullptr;
   size_t bytes = 0;
@@ -61,6 +79,7 @@ struct GenPath {
   double* d_coef = nullptr;
   int* d_desc = nullptr;
   int* d_gen_idx = nullptr;
+  int* d_klist = nullptr;
   double* d_boys = nullptr;         // Boys table, BOYS_NGRID x kGenBoysCols
   unsigned long long* d_counters = nullptr;   // quartets, primitive quartets, operations of the last build
 };
@@ -80,19 +99,41 @@ struct GenBuild {
   double mp_rmax;
 };
 
+// Arguments and table of the f-shell kernels.
+struct FArgs {
+  const GenPairRec* pairs;
+  const double* prims;
+  const double* coef;
+  const int* desc;
+  const int* klist;
+  const double* boys;
+  GenBuild b;
+  unsigned long long* counters;
+};
+struct FKernel {
+  int q;                            // class of the bra's second shell
+  const void* fn;
+};
+extern const FKernel kFKernels[];
+extern const int kNumFKernels;
+
 // Pair records and primitive data for every shell pair; `schwarz` is the basis-level matrix.
 void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* schwarz, int nbf);
 // Device copies of the pair data and the generic Boys table.
 int gen_upload(GenPath& g, cudaStream_t st);
 // Schwarz entries sqrt|(pq|pq)| of the generic pairs' functions into S (nbf x nbf, device).
 int gen_schwarz(const GenPath& g, int nbf, double* S, cudaStream_t st);
-// Work items of one build at these cutoffs; cost: a relative estimate for launch ordering.
-// er_run != nullptr (multipole mode): every generic bra takes error-bank slots for its kets
+// Work items of one build at these cutoffs: bras of the f-shell kernels to fitems (grouped by class,
+// fseg[q] .. fseg[q + 1]), the others to items.
+// er_run != nullptr (multipole mode): every bra to items; it takes error-bank slots for its kets
 // that pass the outer cutoff, numbered on from *er_run.
-void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, double& cost,
-               long long* er_run = nullptr);
-// One launch over the items (counters zeroed first).
-int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const GenBuild& b, cudaStream_t st);
+void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, std::vector<FItem>& fitems,
+               int fseg[6], long long* er_run = nullptr);
+// The launches over the items (counters zeroed first on lanes[0], which the other lanes must wait
+// for): the run-time kernel on lanes[0], the f-shell kernels over all lanes.
+int gen_zero(const GenPath& g, cudaStream_t st);
+int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FItem* d_fitems, const int fseg[6],
+               const GenBuild& b, const cudaStream_t* lanes, int nlanes);
 void gen_free(GenPath& g);
 
 }  // namespace sqb

@@ -9,7 +9,8 @@ import pytest
 from conftest import load_oracle, load_sqb200
 
 FUNCS = {"S": [(0, 0, 0)], "L": [(0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1)], "P": [(1, 0, 0), (0, 1, 0), (0, 0, 1)],
-         "D": [(2, 0, 0), (0, 2, 0), (0, 0, 2), (1, 1, 0), (1, 0, 1), (0, 1, 1)]}
+         "D": [(2, 0, 0), (0, 2, 0), (0, 0, 2), (1, 1, 0), (1, 0, 1), (0, 1, 1)],
+         "F": [(3, 0, 0), (0, 3, 0), (0, 0, 3), (2, 1, 0), (1, 2, 0), (2, 0, 1), (1, 0, 2), (0, 2, 1), (0, 1, 2), (1, 1, 1)]}
 
 
 def _basis(sqb, shells, seed):
