@@ -254,6 +254,27 @@ int build_shells(int nbf, const int* nprim, const int* lmn, const double* xyz,
   return SQB200_OK;
 }
 
+// 1-D Hermite expansion coefficients E^{ij}_t (i <= la, j <= lb <= 2, t <= i+j) of a Gaussian pair
+// product relative to the product centre: E^{00}_0 = 1,
+// E^{i+1,j}_t = E^{ij}_{t-1}/(2p) + XPA E^{ij}_t + (t+1) E^{ij}_{t+1}, likewise for j.
+inline void hermite_1d(double p, double xpa, double xpb, int la, int lb, double E[3][3][5]) {
+  const double h = 0.5 / p;
+  E[0][0][0] = 1.0;
+  for (int i = 0; i <= la; ++i)
+    for (int j = 0; j <= lb; ++j) {
+      if (i == 0 && j == 0) continue;
+      const double* src = i > 0 ? E[i - 1][j] : E[i][j - 1];
+      const double X = i > 0 ? xpa : xpb;
+      const int n = i + j - 1;                    // the source's highest t
+      for (int t = 0; t <= i + j; ++t) {
+        double v = t <= n ? X * src[t] : 0.0;
+        if (t > 0) v += h * src[t - 1];
+        if (t + 1 <= n) v += (t + 1) * src[t + 1];
+        E[i][j][t] = v;
+      }
+    }
+}
+
 // 1-D Hermite expansion coefficients E^{ij}_t (i <= 3, j <= 3, t <= i+j: up to f) of a
 // Gaussian pair product relative to the product centre: E^{00}_0 = 1,
 // E^{i+1,j}_t = E^{ij}_{t-1}/(2p) + XPA E^{ij}_t + (t+1) E^{ij}_{t+1}, likewise for j.
@@ -741,60 +762,80 @@ void build_pairs(sqb200_jk* c) {
     pc.tb = s1.type;
     pc.ne = etable_size(pc.ta, pc.tb);
     pc.stride = 5 + pc.ne;
-    for (const Tmp& t : lists[k]) {
-      const Shell& A = sh[t.P];
-      const Shell& B = sh[t.Q];
-      sqb::PairRec rec;
-      rec.P = t.P; rec.Q = t.Q; rec.fP = A.first; rec.fQ = B.first;
-      rec.nprim = A.nprim * B.nprim;
-      rec.poff = (int)pc.prims.size();
-      rec.kstride = 1;
-      rec.pad_ = 0;
-      rec.schwarz = t.s;
-      pc.max_nprim = std::max(pc.max_nprim, rec.nprim);
-      const double ab2 = (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y) + (A.z - B.z) * (A.z - B.z);
-      for (int i = 0; i < A.nprim; ++i)
-        for (int j = 0; j < B.nprim; ++j) {
-          const double a = A.exps[i], b = B.exps[j], p = a + b;
-          const double Px = (a * A.x + b * B.x) / p, Py = (a * A.y + b * B.y) / p, Pz = (a * A.z + b * B.z) / p;
-          const double kp = std::exp(-a * b * ab2 / p) / p;
-          double Ex[4][4][7], Ey[4][4][7], Ez[4][4][7];
-          hermite_e(p, Px - A.x, Px - B.x, Ex);
-          hermite_e(p, Py - A.y, Py - B.y, Ey);
-          hermite_e(p, Pz - A.z, Pz - B.z, Ez);
-          pc.prims.push_back(p);
-          pc.prims.push_back(Px);
-          pc.prims.push_back(Py);
-          pc.prims.push_back(Pz);
-          pc.prims.push_back(kp);
-          for (int fa = 0; fa < A.nfunc; ++fa)
-            for (int fb = 0; fb < B.nfunc; ++fb) {
-              const int* la = kComp[A.type][fa];
-              const int* lb = kComp[B.type][fb];
-              const double w = A.coef[i][fa] * B.coef[j][fb] * kp;
-              for (int tt = 0; tt <= la[0] + lb[0]; ++tt)
-                for (int uu = 0; uu <= la[1] + lb[1]; ++uu)
-                  for (int vv = 0; vv <= la[2] + lb[2]; ++vv)
-                    pc.prims.push_back(w * Ex[la[0]][lb[0]][tt] * Ey[la[1]][lb[1]][uu] * Ez[la[2]][lb[2]][vv]);
+    // (a, b) -> its 1-D orders per axis, once per class
+    struct Comp { int i[3], j[3]; };
+    std::vector<Comp> comp;
+    for (int fa = 0; fa < kNComp[pc.ta]; ++fa)
+      for (int fb = 0; fb < kNComp[pc.tb]; ++fb) {
+        Comp q;
+        for (int d = 0; d < 3; ++d) { q.i[d] = kComp[pc.ta][fa][d]; q.j[d] = kComp[pc.tb][fb][d]; }
+        comp.push_back(q);
+      }
+    const int la = pc.ta == 3 ? 2 : pc.ta == 0 ? 0 : 1, lb = pc.tb == 3 ? 2 : pc.tb == 0 ? 0 : 1;
+    const int nfb = kNComp[pc.tb];
+    size_t total = 0;
+    for (const Tmp& t : lists[k]) total += (size_t)t.np * pc.stride;
+    pc.prims.resize(total);
+    pc.pairs.resize(lists[k].size());
+    // records of 8 pairs of a run side by side in `blk`, then whole cache lines into the run's layout
+    std::vector<double> blk;
+    size_t base = 0;
+    for (size_t r = 0; r + 1 < pc.sub.size(); ++r) {
+      const int l0 = pc.sub[r], S = pc.sub[r + 1] - l0;
+      const size_t per = (size_t)lists[k][l0].np * pc.stride;   // elements per pair
+      blk.resize(8 * per);
+      for (int lb8 = 0; lb8 < S; lb8 += 8) {
+        const int nl = std::min(8, S - lb8);
+        for (int l = 0; l < nl; ++l) {
+          const Tmp& t = lists[k][l0 + lb8 + l];
+          const Shell& A = sh[t.P];
+          const Shell& B = sh[t.Q];
+          sqb::PairRec& rec = pc.pairs[l0 + lb8 + l];
+          rec.P = t.P; rec.Q = t.Q; rec.fP = A.first; rec.fQ = B.first;
+          rec.nprim = t.np;
+          rec.poff = aos ? (int)(base + (size_t)(lb8 + l) * per) : (int)(base + lb8 + l);
+          rec.kstride = aos ? 1 : S;
+          rec.pad_ = 0;
+          rec.schwarz = t.s;
+          pc.max_nprim = std::max(pc.max_nprim, rec.nprim);
+          const double ab2 = (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y) + (A.z - B.z) * (A.z - B.z);
+          double* out = blk.data() + l;
+          for (int i = 0; i < A.nprim; ++i)
+            for (int j = 0; j < B.nprim; ++j) {
+              const double a = A.exps[i], b = B.exps[j], p = a + b;
+              const double Px = (a * A.x + b * B.x) / p, Py = (a * A.y + b * B.y) / p, Pz = (a * A.z + b * B.z) / p;
+              const double kp = std::exp(-a * b * ab2 / p) / p;
+              double E[3][3][3][5];
+              hermite_1d(p, Px - A.x, Px - B.x, la, lb, E[0]);
+              hermite_1d(p, Py - A.y, Py - B.y, la, lb, E[1]);
+              hermite_1d(p, Pz - A.z, Pz - B.z, la, lb, E[2]);
+              out[0] = p; out[8] = Px; out[16] = Py; out[24] = Pz; out[32] = kp;
+              out += 40;
+              for (size_t f = 0; f < comp.size(); ++f) {
+                const Comp& q = comp[f];
+                const double w = A.coef[i][f / nfb] * B.coef[j][f % nfb] * kp;
+                const double *ex = E[0][q.i[0]][q.j[0]], *ey = E[1][q.i[1]][q.j[1]], *ez = E[2][q.i[2]][q.j[2]];
+                const int nx = q.i[0] + q.j[0], ny = q.i[1] + q.j[1], nz = q.i[2] + q.j[2];
+                for (int tt = 0; tt <= nx; ++tt)
+                  for (int uu = 0; uu <= ny; ++uu)
+                    for (int vv = 0; vv <= nz; ++vv) {
+                      *out = w * ex[tt] * ey[uu] * ez[vv];
+                      out += 8;
+                    }
+              }
             }
         }
-      pc.pairs.push_back(rec);
-    }
-    if (!aos) {
-      // records were appended contiguously (pair-major); transpose every sub-list run
-      std::vector<double> soa(pc.prims.size());
-      for (size_t r = 0; r + 1 < pc.sub.size(); ++r) {
-        const int l0 = pc.sub[r], l1 = pc.sub[r + 1], S = l1 - l0;
-        const size_t base = (size_t)pc.pairs[l0].poff;
-        const size_t per = (size_t)pc.pairs[l0].nprim * pc.stride;   // elements per pair
-        for (int l = 0; l < S; ++l) {
-          const double* src = pc.prims.data() + base + (size_t)l * per;
-          for (size_t e = 0; e < per; ++e) soa[base + e * S + l] = src[e];
-          pc.pairs[l0 + l].poff = (int)(base + l);
-          pc.pairs[l0 + l].kstride = S;
+        if (aos) {
+          for (int l = 0; l < nl; ++l)
+            for (size_t e = 0; e < per; ++e) pc.prims[base + (size_t)(lb8 + l) * per + e] = blk[8 * e + l];
+        } else {
+          for (size_t e = 0; e < per; ++e) {
+            double* dst = pc.prims.data() + base + e * S + lb8;
+            for (int l = 0; l < nl; ++l) dst[l] = blk[8 * e + l];
+          }
         }
       }
-      pc.prims.swap(soa);
+      base += per * S;
     }
   }
 }
