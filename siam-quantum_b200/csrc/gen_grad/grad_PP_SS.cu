@@ -1,6 +1,7 @@
 // generated by gen_grad_kernels.py -- do not edit
 #include "../grad_common.cuh"
 
+static __constant__ unsigned char kCd_grad_PP_SS[1] = {0};
 static __constant__ unsigned char kOrb_grad_PP_SS[1] = {0};
 static __constant__ unsigned char kPerm_grad_PP_SS[1] = {36};
 extern "C" __global__ void __launch_bounds__(64)
@@ -11,8 +12,8 @@ grad_PP_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;
   const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;
   const int gj = grp / si, gi = grp - gj * si;
-  const int cd = blockIdx.y, c = cd / 1, d = cd - c * 1;
-  const int orbit = kOrb_grad_PP_SS[cd], pi = kPerm_grad_PP_SS[cd];
+  const int cd = kCd_grad_PP_SS[blockIdx.y], c = cd / 1, d = cd - c * 1;
+  const int orbit = kOrb_grad_PP_SS[blockIdx.y], pi = kPerm_grad_PP_SS[blockIdx.y];
   const int p0 = pi & 3, p1 = (pi >> 2) & 3, p2 = pi >> 4;   // axis r of this pass = molecule axis p<r>
   const bool have = kl < it.cnt;
   const sqb::GradPair kp = a.ket_pairs[it.k0 + min(kl, it.cnt - 1)];

@@ -55,10 +55,17 @@ extern "C" __global__ void grad_PL_DD(const sqb::GradArgs, const sqb::WorkItem*)
 extern "C" __global__ void grad_LL_DD(const sqb::GradArgs, const sqb::WorkItem*);
 extern "C" __global__ void grad_DP_DD(const sqb::GradArgs, const sqb::WorkItem*);
 extern "C" __global__ void grad_DL_DD(const sqb::GradArgs, const sqb::WorkItem*);
-extern "C" __global__ void grad_DD_DD(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_0(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_1(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_2(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_3(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_4(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_5(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_6(const sqb::GradArgs, const sqb::WorkItem*);
+extern "C" __global__ void grad_DD_DD_7(const sqb::GradArgs, const sqb::WorkItem*);
 
 namespace sqb {
-const GradKernel kGradKernels[55] = {
+const GradKernel kGradKernels[62] = {
   {0, 0, (const void*)grad_SS_SS, 1, 15, 90},
   {3, 0, (const void*)grad_PS_SS, 1, 26, 156},
   {3, 3, (const void*)grad_PS_PS, 3, 26, 192},
@@ -113,7 +120,14 @@ const GradKernel kGradKernels[55] = {
   {2, 9, (const void*)grad_LL_DD, 36, 54, 942},
   {8, 9, (const void*)grad_DP_DD, 36, 91, 1503},
   {7, 9, (const void*)grad_DL_DD, 36, 92, 1803},
-  {9, 9, (const void*)grad_DD_DD, 36, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_0, 3, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_1, 6, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_2, 6, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_3, 3, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_4, 6, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_5, 3, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_6, 3, 157, 3654},
+  {9, 9, (const void*)grad_DD_DD_7, 6, 157, 3654},
 };
-const int kNumGradKernels = 55;
+const int kNumGradKernels = 62;
 }  // namespace sqb

@@ -134,7 +134,8 @@ def func_perm(t, k):
     return "p%d" % k if k < 3 else "2 + %s" % {3: "p0 + p1", 4: "p0 + p2", 5: "p1 + p2"}[k]
 
 
-def gen_grad(bra, ket):
+def gen_grad(bra, ket, only=None):
+    """The kernel of a class, or of one orbit of its ket function pairs (`only`)."""
     ta, tb = bra
     tc, td = ket
     fA, fB, fC, fD = COMP[ta], COMP[tb], COMP[tc], COMP[td]
@@ -148,12 +149,14 @@ def gen_grad(bra, ket):
     T0 = NHEAD + na + nb                              # E tables, then derivative tables
     reps, orb = ket_orbits(ket)
     Hb, Hb1, Hbd = simplex(Lb), simplex(Lb + 1), simplex(max(0, Lb - 1))
-    name = "grad_%s_%s" % (bra, ket)
+    name = "grad_%s_%s" % (bra, ket) + ("" if only is None else "_%d" % only)
+    cds = [k for k, (o, _) in enumerate(orb) if only is None or o == only]
     hn = lambda h: "%d%d%d" % h
     em = Emitter()
-    out = ['static __constant__ unsigned char kOrb_%s[%d] = {%s};' % (name, nc * nd, ", ".join(str(o) for o, _ in orb)),
+    out = ['static __constant__ unsigned char kCd_%s[%d] = {%s};' % (name, len(cds), ", ".join(str(k) for k in cds)),
+           'static __constant__ unsigned char kOrb_%s[%d] = {%s};' % (name, len(cds), ", ".join(str(orb[k][0]) for k in cds)),
            'static __constant__ unsigned char kPerm_%s[%d] = {%s};' % (
-               name, nc * nd, ", ".join(str(pi[0] | pi[1] << 2 | pi[2] << 4) for _, pi in orb)),
+               name, len(cds), ", ".join(str(orb[k][1][0] | orb[k][1][1] << 2 | orb[k][1][2] << 4) for k in cds)),
            'extern "C" __global__ void __launch_bounds__(%d)' % CTA,
            "%s(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {" % name]
     em("extern __shared__ double sb[];                // [chunk][%d] bra primitive records" % NB)
@@ -162,8 +165,8 @@ def gen_grad(bra, ket):
     em("const int si = it.split & 0xffff, sj = it.split >> 16, isplit = si * sj;")
     em("const int kl = threadIdx.x / isplit, grp = threadIdx.x - kl * isplit;")
     em("const int gj = grp / si, gi = grp - gj * si;")
-    em("const int cd = blockIdx.y, c = cd / %d, d = cd - c * %d;" % (nd, nd))
-    em("const int orbit = kOrb_%s[cd], pi = kPerm_%s[cd];" % (name, name))
+    em("const int cd = kCd_%s[blockIdx.y], c = cd / %d, d = cd - c * %d;" % (name, nd, nd))
+    em("const int orbit = kOrb_%s[blockIdx.y], pi = kPerm_%s[blockIdx.y];" % (name, name))
     em("const int p0 = pi & 3, p1 = (pi >> 2) & 3, p2 = pi >> 4;   // axis r of this pass = molecule axis p<r>")
     em("const bool have = kl < it.cnt;")
     em("const sqb::GradPair kp = a.ket_pairs[it.k0 + min(kl, it.cnt - 1)];")
@@ -242,6 +245,8 @@ def gen_grad(bra, ket):
     em.ind += 1
     em("switch (orbit) {")
     for oi, (lc, ld) in enumerate(reps):
+        if only is not None and oi != only:
+            continue
         em("case %d: {  // ket functions like %s %s" % (oi, lc, ld))
         em.ind += 1
         em("for (int i = (gi + si - i0 % si) % si; i < ni; i += si) {   // bra primitives gi, gi + si, ...")
@@ -403,7 +408,7 @@ def gen_grad(bra, ket):
     out += em.lines
     out.append("}")
     ops = 60 + 6 * L + 3 * len(simplex(L)) + 10 * na * nb + 4 * len(Hb) * na * nb // 2
-    return "\n".join(out) + "\n", {"name": name, "bra": bra, "ket": ket, "nb": NB, "passes": nc * nd, "ops": ops}
+    return "\n".join(out) + "\n", {"name": name, "bra": bra, "ket": ket, "nb": NB, "passes": len(cds), "ops": ops}
 
 
 def main():
@@ -412,10 +417,15 @@ def main():
     head = "// generated by gen_grad_kernels.py -- do not edit\n#include \"../grad_common.cuh\"\n\n"
     files, reg = [], []
     for x, y in quartet_classes():
-        src, m = gen_grad(*roles(x, y))
-        write_if_changed(os.path.join(outdir, m["name"] + ".cu"), head + src)
-        files.append(m["name"] + ".cu")
-        reg.append(m)
+        bra, ket = roles(x, y)
+        # one kernel per orbit where the whole class is more code than ptxas allocates registers for
+        # ((dd|dd) in one kernel: 18 KB of stack a thread, 1.07 ms for an organic of 8 heavy atoms)
+        parts = range(len(ket_orbits(ket)[0])) if pair_L(bra) + pair_L(ket) >= 8 else [None]
+        for only in parts:
+            src, m = gen_grad(bra, ket, only)
+            write_if_changed(os.path.join(outdir, m["name"] + ".cu"), head + src)
+            files.append(m["name"] + ".cu")
+            reg.append(m)
     text = head + "".join('extern "C" __global__ void %s(const sqb::GradArgs, const sqb::WorkItem*);\n' % m["name"] for m in reg)
     text += "\nnamespace sqb {\nconst GradKernel kGradKernels[%d] = {\n" % len(reg)
     for m in reg:
