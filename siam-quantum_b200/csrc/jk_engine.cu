@@ -25,6 +25,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -173,6 +174,36 @@ struct BoysTables {
 const BoysTables& boys_tables() {
   static const BoysTables t;
   return t;
+}
+
+// The tables on the device: static arrays of about 0.6 MB, filled when the first context of a device
+// is created and read by all of them (a copy in every context's own allocation took a small
+// molecule's context past the size the driver carves from a pool: 1.6 -> 3.8 ms to create).
+constexpr int kBoysPlain = BOYS_NGRID * BOYS_NCOL;
+constexpr int kBoysRows = (BOYS_MMAX + 2) * BOYS_NGRID * BOYS_ROW;
+constexpr int kBoysRowsF = (BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF;
+__device__ __align__(128) double g_boys_plain[kBoysPlain];
+__device__ __align__(128) double g_boys_rows[kBoysRows];
+__device__ __align__(128) float g_boys_rowsf[kBoysRowsF];
+
+// Addresses of the tables on the current device, filled on first use.
+cudaError_t boys_device(double** plain, double** rows, float** rowsf, cudaStream_t st) {
+  static std::mutex mu;
+  static std::set<int> filled;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)plain, g_boys_plain);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)rows, g_boys_rows);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)rowsf, g_boys_rowsf);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (filled.count(dev)) return cudaSuccess;
+  const BoysTables& bt = boys_tables();
+  e = h2d(*plain, bt.plain.data(), bt.plain.size() * sizeof(double), st);
+  if (e == cudaSuccess) e = h2d(*rows, bt.rows.data(), bt.rows.size() * sizeof(double), st);
+  if (e == cudaSuccess) e = h2d(*rowsf, bt.rowsf.data(), bt.rowsf.size() * sizeof(float), st);
+  if (e == cudaSuccess) filled.insert(dev);
+  return e;
 }
 
 // ---------------------------------------------------------------- shells
@@ -1040,14 +1071,15 @@ double build_ops(const sqb200_jk* c, double outer, double fixed) {
 }
 
 // The longest run of operations a thread of a build of `ops` emitted operations is given.  A
-// build that fills the GPU for milliseconds leaves its quartets whole: each split thread digests
-// its own partial block, atomics included.  A small molecule's build is as long as its longest
-// thread, so its quartets are split, down to a few primitive steps; splitting further costs more
-// in digestion than the shorter chain saves.  Measured on B200 (ms per build, narrow forms, least
-// run / factor): a 3-heavy-atom radical UHF/6-31G* 0.25 / 0.23 / 0.25 at a least run of 1500 / 3000 /
-// 6000; benzene/6-31G* 1.31 / 1.14 / 0.79 / 0.70 at factors 0.5, 1, 2 and 4e-6, an organic of 9 heavy
-// atoms 2.08 / 1.87 / 1.48 / 1.47; C60/6-31G the same whether its quartets are split or not.
-double chain_ops(double ops) { return std::max(3000.0, 4e-6 * ops); }
+// build that fills the GPU for tens of milliseconds leaves its quartets whole: each split thread
+// digests its own partial block, atomics included.  A small molecule's build is as long as its
+// longest thread, so its quartets are split, down to a few primitive steps; splitting further costs
+// more in digestion than the shorter chain saves.  Measured on B200 (ms per build): a 3-heavy-atom
+// radical UHF/6-31G* (4e8 operations) 0.25 / 0.23 / 0.25 at runs of 1500 / 3000 / 6000; benzene/6-31G*
+// (3e9) 1.31 / 1.14 / 0.79 / 0.70 at 2, 3, 7 and 13 thousand; an organic of 9 heavy atoms (1e10) 2.08 / 1.87 /
+// 1.48 / 1.47 at 5, 10, 20 and 40; a batch of 24 organics (6e10) 14.0 / 14.3 / 14.9 / 15.1 at 10, 30, 100 and
+// 240; C60/6-31G (8e11) 68.2 / 57.4 / 56.0 / 56.2 at 10, 30 and 100 thousand and unsplit.
+double chain_ops(double ops) { return std::max({3000.0, std::min(4e-6 * ops, 2e4), 1.5e-7 * ops}); }
 
 // Work items of class kernel ki for one molecule (context c): every surviving (bra pair, <=kper
 // ket pairs) unit, with pair indices shifted by bra_base/ket_base (the molecule's first pair in
@@ -1070,82 +1102,71 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
   const bool mpm = er_run != nullptr;
   const bool mixed = allow_f32 && !mpm && c->fp32_below > 0.0 && K.fn_r32 != nullptr;
   // every (bra sub-list, ket sub-list) combination; inside one class each unordered pair of
-  // sub-lists once, and inside one sub-list each unordered pair of pairs once (k >= b)
+  // sub-lists once, and inside one sub-list each unordered pair of pairs once (k >= b).  The
+  // combinations with the longest primitive loops first, so that a launch does not end on a few
+  // long CTAs while the rest of the GPU idles.
+  struct Run { long loop; size_t sx, sy; int split; };
+  std::vector<Run> runs;
   for (size_t sx = 0; sx + 1 < B.sub.size(); ++sx)
-    for (size_t sy = 0; sy + 1 < T.sub.size(); ++sy) {
-      if (same && sx > sy) continue;
-      const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0s = T.sub[sy], k1s = T.sub[sy + 1];
-      const int nbp = B.pairs[b0].nprim, nkp = T.pairs[k0s].nprim;
+    for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
+      const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
       // multipole mode needs each quartet's whole block in one thread
       const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K), K.nab * K.ncd <= 16);
-      const int kper = cta / ((split & 0xffff) * (split >> 16));
-      const double pq = (double)nbp * nkp;
-      for (int b = b0; b < b1; ++b) {
-        const double sb = B.pairs[b].schwarz;
-        if (!(sb > 0.0)) break;   // sorted: the rest are zero
-        const double thr = cut / sb * (1.0 - 1e-12);
-        // ket pairs of the sub-list with schwarz >= thr form a prefix of it
-        int lo = k0s, hi = k1s;
-        while (lo < hi) {
-          const int mid = (lo + hi) / 2;
-          if (T.pairs[mid].schwarz >= thr) lo = mid + 1; else hi = mid;
-        }
-        const int end = lo;
-        const int start = (same && sx == sy) ? b : k0s;
-        long long er0 = 0;
-        if (mpm) {
-          // outer-cutoff survivors of this run: the bank slots er0 .. er0 + count - 1
-          const double tho = outer / sb * (1.0 - 1e-12);
-          int lo2 = k0s, hi2 = k1s;
-          while (lo2 < hi2) {
-            const int m2 = (lo2 + hi2) / 2;
-            if (T.pairs[m2].schwarz >= tho) lo2 = m2 + 1; else hi2 = m2;
-          }
-          er0 = *er_run;
-          *er_run += std::max(0, lo2 - start);
-        }
-        // kets with Sch(bra)*Sch(ket) >= fp32_below (a prefix) stay FP64, the rest go FP32
-        int mid = end;
-        if (mixed) {
-          const double t32 = c->fp32_below / sb;
-          int l2 = start, h2 = end;
-          while (l2 < h2) {
-            const int m2 = (l2 + h2) / 2;
-            if (T.pairs[m2].schwarz >= t32) l2 = m2 + 1; else h2 = m2;
-          }
-          mid = l2;
-        }
-        for (int k0 = start; k0 < mid; k0 += kper) {
-          items.push_back({bra_base + b, ket_base + k0, std::min(kper, mid - k0), split, mol});
-          if (mpm) ers->push_back((int)(er0 + (k0 - start)));
-        }
-        for (int k0 = std::max(start, mid); k0 < end; k0 += kper)
-          items32.push_back({bra_base + b, ket_base + k0, std::min(kper, end - k0), split, mol});
-        cost64 += std::max(0, mid - start) * (pq * K.flops_prim + K.flops_quartet);
-        cost32 += std::max(0, end - std::max(start, mid)) * (pq * K.f32_flops_prim + K.f32_flops_quartet);
-      }
+      const int si = split & 0xffff, sj = split >> 16;
+      runs.push_back({(long)((nbp + si - 1) / si) * ((nkp + sj - 1) / sj), sx, sy, split});
     }
-}
-
-// Launch order inside one class kernel: the CTAs with the longest primitive loop first (a
-// thread runs ceil(bra primitives / si) x ceil(ket primitives / sj) iterations; more kets per item next),
-// so that a launch does not end on a few long CTAs while the rest of the GPU idles.
-// nprims(item) gives the item's (bra, ket) primitive counts.
-template <class F>
-void sort_heavy_first(std::vector<sqb::WorkItem>& v, size_t first, F nprims) {
-  const size_t n = v.size() - first;
-  std::vector<std::pair<long long, size_t>> key(n);
-  for (size_t i = 0; i < n; ++i) {
-    const sqb::WorkItem& it = v[first + i];
-    const std::pair<int, int> np = nprims(it);
-    const int si = it.split & 0xffff, sj = it.split >> 16;
-    const long long loop = (long long)((np.first + si - 1) / si) * ((np.second + sj - 1) / sj);
-    key[i] = {-(loop * 4096 + it.cnt), i};
+  std::stable_sort(runs.begin(), runs.end(), [](const Run& x, const Run& y) { return x.loop > y.loop; });
+  for (const Run& run : runs) {
+    const size_t sx = run.sx, sy = run.sy;
+    const int split = run.split, kper = cta / ((split & 0xffff) * (split >> 16));
+    const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0s = T.sub[sy], k1s = T.sub[sy + 1];
+    const int nbp = B.pairs[b0].nprim, nkp = T.pairs[k0s].nprim;
+    const double pq = (double)nbp * nkp;
+    for (int b = b0; b < b1; ++b) {
+      const double sb = B.pairs[b].schwarz;
+      if (!(sb > 0.0)) break;   // sorted: the rest are zero
+      const double thr = cut / sb * (1.0 - 1e-12);
+      // ket pairs of the sub-list with schwarz >= thr form a prefix of it
+      int lo = k0s, hi = k1s;
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (T.pairs[mid].schwarz >= thr) lo = mid + 1; else hi = mid;
+      }
+      const int end = lo;
+      const int start = (same && sx == sy) ? b : k0s;
+      long long er0 = 0;
+      if (mpm) {
+        // outer-cutoff survivors of this run: the bank slots er0 .. er0 + count - 1
+        const double tho = outer / sb * (1.0 - 1e-12);
+        int lo2 = k0s, hi2 = k1s;
+        while (lo2 < hi2) {
+          const int m2 = (lo2 + hi2) / 2;
+          if (T.pairs[m2].schwarz >= tho) lo2 = m2 + 1; else hi2 = m2;
+        }
+        er0 = *er_run;
+        *er_run += std::max(0, lo2 - start);
+      }
+      // kets with Sch(bra)*Sch(ket) >= fp32_below (a prefix) stay FP64, the rest go FP32
+      int mid = end;
+      if (mixed) {
+        const double t32 = c->fp32_below / sb;
+        int l2 = start, h2 = end;
+        while (l2 < h2) {
+          const int m2 = (l2 + h2) / 2;
+          if (T.pairs[m2].schwarz >= t32) l2 = m2 + 1; else h2 = m2;
+        }
+        mid = l2;
+      }
+      for (int k0 = start; k0 < mid; k0 += kper) {
+        items.push_back({bra_base + b, ket_base + k0, std::min(kper, mid - k0), split, mol});
+        if (mpm) ers->push_back((int)(er0 + (k0 - start)));
+      }
+      for (int k0 = std::max(start, mid); k0 < end; k0 += kper)
+        items32.push_back({bra_base + b, ket_base + k0, std::min(kper, end - k0), split, mol});
+      cost64 += std::max(0, mid - start) * (pq * K.flops_prim + K.flops_quartet);
+      cost32 += std::max(0, end - std::max(start, mid)) * (pq * K.f32_flops_prim + K.f32_flops_quartet);
+    }
   }
-  std::stable_sort(key.begin(), key.end());
-  std::vector<sqb::WorkItem> tmp(n);
-  for (size_t i = 0; i < n; ++i) tmp[i] = v[first + key[i].second];
-  std::copy(tmp.begin(), tmp.end(), v.begin() + first);
 }
 
 // A class whose FP32 work items would number fewer than this runs all its quartets in FP64: a
@@ -1191,13 +1212,6 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
       items32.clear();
       cost64 = cost32 = 0.0;
       class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, cost64, cost32, nullptr, nullptr, false);
-    }
-    if (!mpm) {   // (multipole mode keeps the items with their bank slots in generation order)
-      const PairClass& B = c->cls[sqb::kClassKernels[ki].bra_cls];
-      const PairClass& T = c->cls[sqb::kClassKernels[ki].ket_cls];
-      auto np = [&](const sqb::WorkItem& it) { return std::make_pair(B.pairs[it.bra].nprim, T.pairs[it.k0].nprim); };
-      sort_heavy_first(items, first, np);
-      sort_heavy_first(items32, 0, np);
     }
     const int cnt = (int)items.size() - first;
     if (cnt > 0) {
@@ -1712,13 +1726,9 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   if (!rc) rc = setup_generic(c);
   if (rc) { sqb200_jk_destroy(c); return rc; }
   const size_t nn = (size_t)nbf * nbf;
-  const BoysTables& bt = boys_tables();
   std::vector<int> fst(c->ns), nf(c->ns);
   for (int s = 0; s < c->ns; ++s) { fst[s] = c->shells[s].first; nf[s] = c->shells[s].nfunc; }
   Carve cv;
-  cv.add(&c->d_boys, bt.plain.size() * sizeof(double));
-  cv.add(&c->d_boysr, bt.rows.size() * sizeof(double));
-  cv.add(&c->d_boysf, bt.rowsf.size() * sizeof(float));
   cv.add(&c->d_shfirst, c->ns * sizeof(int));
   cv.add(&c->d_shn, c->ns * sizeof(int));
   for (double** m : {&c->d_PA, &c->d_PB, &c->d_PT, &c->d_JT, &c->d_KAo, &c->d_KBo}) cv.add(m, nn * sizeof(double));
@@ -1733,9 +1743,7 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
     return fail(SQB200_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = h2d(c->d_boys, bt.plain.data(), bt.plain.size() * sizeof(double), c->stream);
-  if (e == cudaSuccess) e = h2d(c->d_boysr, bt.rows.data(), bt.rows.size() * sizeof(double), c->stream);
-  if (e == cudaSuccess) e = h2d(c->d_boysf, bt.rowsf.data(), bt.rowsf.size() * sizeof(float), c->stream);
+  if (e == cudaSuccess) e = boys_device(&c->d_boys, &c->d_boysr, &c->d_boysf, c->stream);
   if (e == cudaSuccess) e = h2d(c->d_shfirst, fst.data(), c->ns * sizeof(int), c->stream);
   if (e == cudaSuccess) e = h2d(c->d_shn, nf.data(), c->ns * sizeof(int), c->stream);
   if (e != cudaSuccess) { sqb200_jk_destroy(c); return fail(SQB200_ECUDA, cudaGetErrorString(e)); }
@@ -2525,20 +2533,12 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
       const int f64 = (int)items.size();
       items32.clear();
       double c64 = 0.0, c32 = 0.0;
-      // heaviest first inside each molecule's run of items: sorting across molecules would
-      // interleave their pair data and J/K blocks in L2 (measured 4% slower on 256 molecules)
-      auto np = [&](const sqb::WorkItem& it) {
-        const sqb200_jk* mc = b->mols[it.mol];
-        return std::make_pair(mc->cls[K.bra_cls].pairs[it.bra - b->cls[K.bra_cls].pair_base[it.mol]].nprim,
-                              mc->cls[K.ket_cls].pairs[it.k0 - b->cls[K.ket_cls].pair_base[it.mol]].nprim);
-      };
+      // (the items come longest loops first inside each molecule: across molecules that would
+      // interleave their pair data and J/K blocks in L2, measured 4% slower on 256 molecules)
       for (int m = 0; m < b->nmol; ++m) {
         if (b->rec[m].uhf != sp) continue;
-        const size_t a64 = items.size(), a32 = items32.size();
         class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
                     b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32);
-        sort_heavy_first(items, a64, np);
-        sort_heavy_first(items32, a32, np);
       }
       if (too_few_f32(items32)) {
         items.resize(f64);
@@ -2546,11 +2546,9 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
         c64 = c32 = 0.0;
         for (int m = 0; m < b->nmol; ++m) {
           if (b->rec[m].uhf != sp) continue;
-          const size_t a64 = items.size();
           class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
                       b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32, nullptr, nullptr,
                       false);
-          sort_heavy_first(items, a64, np);
         }
       }
       if ((int)items.size() > f64) {
@@ -3331,28 +3329,32 @@ void grad_work(const sqb200_jk* c, const int* fat, const double* PT, double scre
       const bool same = K.bra_cls == K.ket_cls;
       const size_t first = w.items.size();
       double cost = 0.0;
+      struct Run { long loop; size_t sx, sy; int split; };
+      std::vector<Run> runs;                  // longest primitive loops first
       for (size_t sx = 0; sx + 1 < B.sub.size(); ++sx)
         for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
           const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
-          const int split = pass ? pick_split(nbp, nkp, chain / K.ops, false) : 0;
-          const int kper = pass ? kGradCta / ((split & 0xffff) * (split >> 16)) : 0;
-          int end = T.sub[sy + 1];
-          for (int b = B.sub[sx]; b < B.sub[sx + 1]; ++b) {
-            const double sb = B.pairs[b].sch * B.pairs[b].pm;
-            while (end > T.sub[sy] && T.pairs[end - 1].sch * T.pairs[end - 1].pm * sb < screen * (1.0 - 1e-12)) --end;
-            const int start = same && sx == sy ? b : T.sub[sy];
-            cost += (double)std::max(0, end - start) * nbp * nkp * K.passes * K.ops;
-            if (pass)
-              for (int k0 = start; k0 < end; k0 += kper) w.items.push_back({b, k0, std::min(kper, end - k0), split, 0});
-          }
+          const int split = pass ? pick_split(nbp, nkp, chain / K.ops, false) : 1 | 1 << 16;
+          const int si = split & 0xffff, sj = split >> 16;
+          runs.push_back({(long)((nbp + si - 1) / si) * ((nkp + sj - 1) / sj), sx, sy, split});
         }
-      total += cost;
-      if (pass && w.items.size() > first) {
-        sort_heavy_first(w.items, first, [&](const sqb::WorkItem& it) {
-          return std::make_pair(B.pairs[it.bra].nprim, T.pairs[it.k0].nprim);
-        });
-        w.segs.push_back({gk, first, w.items.size() - first, cost});
+      std::stable_sort(runs.begin(), runs.end(), [](const Run& x, const Run& y) { return x.loop > y.loop; });
+      for (const Run& run : runs) {
+        const size_t sx = run.sx, sy = run.sy;
+        const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
+        const int kper = kGradCta / ((run.split & 0xffff) * (run.split >> 16));
+        int end = T.sub[sy + 1];
+        for (int b = B.sub[sx]; b < B.sub[sx + 1]; ++b) {
+          const double sb = B.pairs[b].sch * B.pairs[b].pm;
+          while (end > T.sub[sy] && T.pairs[end - 1].sch * T.pairs[end - 1].pm * sb < screen * (1.0 - 1e-12)) --end;
+          const int start = same && sx == sy ? b : T.sub[sy];
+          cost += (double)std::max(0, end - start) * nbp * nkp * K.passes * K.ops;
+          if (pass)
+            for (int k0 = start; k0 < end; k0 += kper) w.items.push_back({b, k0, std::min(kper, end - k0), run.split, 0});
+        }
       }
+      total += cost;
+      if (pass && w.items.size() > first) w.segs.push_back({gk, first, w.items.size() - first, cost});
     }
     if (!pass) chain = chain_ops(total);
   }
