@@ -4,7 +4,7 @@
 static __constant__ unsigned char kCd_grad_DS_SS[1] = {0};
 static __constant__ unsigned char kOrb_grad_DS_SS[1] = {0};
 static __constant__ unsigned char kPerm_grad_DS_SS[1] = {36};
-extern "C" __global__ void __launch_bounds__(64)
+extern "C" __global__ void __launch_bounds__(64, 1)
 grad_DS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   extern __shared__ double sb[];                // [chunk][44] bra primitive records
   const sqb::WorkItem it = items[blockIdx.x];

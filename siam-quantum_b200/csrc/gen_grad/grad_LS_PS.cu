@@ -4,7 +4,7 @@
 static __constant__ unsigned char kCd_grad_LS_PS[3] = {0, 1, 2};
 static __constant__ unsigned char kOrb_grad_LS_PS[3] = {0, 0, 0};
 static __constant__ unsigned char kPerm_grad_LS_PS[3] = {36, 33, 18};
-extern "C" __global__ void __launch_bounds__(64)
+extern "C" __global__ void __launch_bounds__(64, 1)
 grad_LS_PS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   extern __shared__ double sb[];                // [chunk][27] bra primitive records
   const sqb::WorkItem it = items[blockIdx.x];

@@ -4,7 +4,7 @@
 static __constant__ unsigned char kCd_grad_PL_LS[4] = {0, 1, 2, 3};
 static __constant__ unsigned char kOrb_grad_PL_LS[4] = {0, 1, 1, 1};
 static __constant__ unsigned char kPerm_grad_PL_LS[4] = {36, 36, 33, 18};
-extern "C" __global__ void __launch_bounds__(64)
+extern "C" __global__ void __launch_bounds__(64, 1)
 grad_PL_LS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   extern __shared__ double sb[];                // [chunk][53] bra primitive records
   const sqb::WorkItem it = items[blockIdx.x];

@@ -157,7 +157,9 @@ def gen_grad(bra, ket, only=None):
            'static __constant__ unsigned char kOrb_%s[%d] = {%s};' % (name, len(cds), ", ".join(str(orb[k][0]) for k in cds)),
            'static __constant__ unsigned char kPerm_%s[%d] = {%s};' % (
                name, len(cds), ", ".join(str(orb[k][1][0] | orb[k][1][1] << 2 | orb[k][1][2] << 4) for k in cds)),
-           'extern "C" __global__ void __launch_bounds__(%d)' % CTA,
+           # at least one CTA per SM: without it ptxas falls back to 32 registers and 18 KB of stack a thread in
+           # the largest classes (a launch then takes 5 GB of local memory)
+           'extern "C" __global__ void __launch_bounds__(%d, 1)' % CTA,
            "%s(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {" % name]
     em("extern __shared__ double sb[];                // [chunk][%d] bra primitive records" % NB)
     em("const sqb::WorkItem it = items[blockIdx.x];")
