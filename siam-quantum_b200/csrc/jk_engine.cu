@@ -96,9 +96,26 @@ struct Staged : Carve {
   template <class T>
   void put(T** dst, size_t bytes, const void* host) { add(dst, bytes); src.push_back(host); }
   cudaError_t upload(void** base, cudaStream_t st) {
+    const cudaError_t e = alloc(base);
+    return e == cudaSuccess ? fill(*base, st) : e;
+  }
+  // The same into a workspace of *cap bytes that the caller keeps: grown (by a new allocation) when
+  // this call needs more.
+  cudaError_t upload_kept(void** base, size_t* cap, cudaStream_t st) {
+    if (*cap < bytes()) {
+      cudaFree(*base);
+      *base = nullptr;
+      *cap = 0;
+      const cudaError_t e = alloc(base);
+      if (e != cudaSuccess) return e;
+      *cap = bytes();
+    } else {
+      place(*base);
+    }
+    return fill(*base, st);
+  }
+  cudaError_t fill(void* base, cudaStream_t st) {
     src.resize(slots.size(), nullptr);
-    cudaError_t e = alloc(base);
-    if (e != cudaSuccess) return e;
     size_t o = 0, end = 0;
     std::vector<size_t> at;
     for (size_t i = 0; i < slots.size(); ++i) {
@@ -110,7 +127,7 @@ struct Staged : Carve {
     std::vector<char> img(end, 0);
     for (size_t i = 0; i < slots.size(); ++i)
       if (src[i] && slots[i].second) memcpy(img.data() + at[i], src[i], slots[i].second);
-    return h2d(*base, img.data(), end, st);
+    return h2d(base, img.data(), end, st);
   }
 };
 
@@ -371,6 +388,8 @@ struct sqb200_jk {
   cudaStream_t stream = nullptr;
   void* d_base = nullptr;       // one allocation holding every buffer below
   void* d_pairbase = nullptr;   // one allocation holding the pair classes' device arrays
+  void* d_grad = nullptr;       // workspace of the gradient, as large as its largest call so far
+  size_t grad_bytes = 0;
   size_t pairbase_bytes = 0;
   double* d_boys = nullptr;   // plain Boys table (gradient)
   double* d_boysr = nullptr;  // row table of boys<M>
@@ -1784,6 +1803,7 @@ int sqb200_jk_destroy(sqb200_jk* c) {
   if (c->d_erbase) cudaFree(c->d_erbase);
   for (auto& e : c->events) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
   free_pairs(c);
+  cudaFree(c->d_grad);
   cudaFree(c->d_base);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -3536,8 +3556,9 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
   up.put(&gw.d_items, gw.items.size() * sizeof(sqb::WorkItem), gw.items.data());
   up.put(&dg, 3 * natom * sizeof(double), nullptr);
   up.put(&dcopies, (size_t)kGradCopies * gstride * sizeof(double), nullptr);
-  void* base = nullptr;
-  cudaError_t e = up.upload(&base, c->stream);
+  // the workspace stays with the context: a cudaMalloc and a cudaFree of some megabytes in every call
+  // took 0.4 ms, and the free synchronised the device
+  cudaError_t e = up.upload_kept(&c->d_grad, &c->grad_bytes, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, 3 * natom * sizeof(double), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(dcopies, 0, (size_t)kGradCopies * gstride * sizeof(double), c->stream);
   if (e == cudaSuccess) {
@@ -3552,8 +3573,7 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
       ga.nbf = n; ga.ncopy = kGradCopies; ga.stride = gstride;
       const int rc = grad_launch(c, gw, ga);
       if (rc) {
-        cudaDeviceSynchronize();           // kernels in flight read the buffers freed here
-        cudaFree(base);
+        cudaDeviceSynchronize();           // kernels in flight read the buffers of the next call
         return rc;
       }
     } else if ((terms & SQB200_GRAD_ERI) && fgrad)
@@ -3581,7 +3601,6 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(grad, dg, 3 * natom * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(base);
   if (e != cudaSuccess) return fail(SQB200_ECUDA, std::string("sqb200_gradient: ") + cudaGetErrorString(e));
   // nuclear repulsion (GradVnn, src/grad.c:43)
   if (terms & SQB200_GRAD_NUCLEAR)
