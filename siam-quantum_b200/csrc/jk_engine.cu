@@ -1004,7 +1004,54 @@ int cta_threads(double ops) {
 // kernels side by side on an SM share its instruction cache).
 constexpr int kSideStreams = 8;
 
-// Side streams for a call of `launches` kernels (created when first needed, kept): the lanes it uses.
+// Side streams and their join events, per device.  A context or batch takes the ones it needs and gives
+// them back, idle, when it is destroyed; at most kSidePool stay for the next (creating and destroying
+// eight takes over a millisecond of a short SCF job's set-up and end).
+struct SidePool {
+  std::mutex mu;
+  std::map<int, std::vector<std::pair<cudaStream_t, cudaEvent_t>>> idle;
+};
+constexpr size_t kSidePool = 64;
+SidePool& side_pool() {
+  static SidePool* p = new SidePool;      // never destroyed: contexts may outlive static objects
+  return *p;
+}
+
+cudaError_t side_take(int device, cudaStream_t* s, cudaEvent_t* ev) {
+  SidePool& p = side_pool();
+  {
+    std::lock_guard<std::mutex> lock(p.mu);
+    auto& v = p.idle[device];
+    if (!v.empty()) {
+      *s = v.back().first;
+      *ev = v.back().second;
+      v.pop_back();
+      return cudaSuccess;
+    }
+  }
+  cudaError_t e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) return e;
+  e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) cudaEventDestroy(*ev);
+  return e;
+}
+
+// The stream's work is waited for; a stream in error is destroyed.
+void side_give(int device, cudaStream_t s, cudaEvent_t ev) {
+  SidePool& p = side_pool();
+  if (cudaStreamSynchronize(s) == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(p.mu);
+    auto& v = p.idle[device];
+    if (v.size() < kSidePool) {
+      v.push_back({s, ev});
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+  cudaEventDestroy(ev);
+}
+
+// Side streams for a call of `launches` kernels (taken when first needed, kept): the lanes it uses.
 int ensure_side_streams(sqb200_jk* c, size_t launches) {
   if (c->nside < 0) {
     CUDA_OK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
@@ -1014,12 +1061,7 @@ int ensure_side_streams(sqb200_jk* c, size_t launches) {
   while (c->side.size() < (size_t)c->nside && c->side.size() + 1 < launches) {
     cudaStream_t s;
     cudaEvent_t e;
-    CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    const cudaError_t rc = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (rc != cudaSuccess) {
-      cudaEventDestroy(e);
-      return fail(SQB200_ECUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(rc));
-    }
+    CUDA_OK(side_take(c->device, &s, &e));
     c->side.push_back(s);
     c->ev_join.push_back(e);
   }
@@ -1788,11 +1830,7 @@ int sqb200_jk_destroy(sqb200_jk* c) {
   if (!c) return SQB200_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (size_t i = 0; i < c->side.size(); ++i) {
-    cudaStreamSynchronize(c->side[i]);
-    cudaStreamDestroy(c->side[i]);
-    cudaEventDestroy(c->ev_join[i]);
-  }
+  for (size_t i = 0; i < c->side.size(); ++i) side_give(c->device, c->side[i], c->ev_join[i]);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   for (auto& kv : c->work)
     for (auto& g : kv.second.graph)
@@ -2407,11 +2445,7 @@ __global__ void k_finalize_batch(const double* __restrict__ J, const double* __r
 }
 
 void free_batch(sqb200_batch* b) {
-  for (size_t i = 0; i < b->side.size(); ++i) {
-    cudaStreamSynchronize(b->side[i]);
-    cudaStreamDestroy(b->side[i]);
-    cudaEventDestroy(b->ev_join[i]);
-  }
+  for (size_t i = 0; i < b->side.size(); ++i) side_give(b->device, b->side[i], b->ev_join[i]);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
   if (b->stream) { cudaStreamSynchronize(b->stream); cudaStreamDestroy(b->stream); }
   for (auto& k : b->cls) { cudaFree(k.d_pairs); cudaFree(k.d_prims); cudaFree(k.d_primsf); }
@@ -2688,8 +2722,7 @@ extern "C" int sqb200_batch_build_device(sqb200_batch* b, const double* dPA, con
     for (int i = 0; i < n; ++i) {
       cudaStream_t s;
       cudaEvent_t e;
-      CUDA_OK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-      CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      CUDA_OK(side_take(b->device, &s, &e));
       b->side.push_back(s);
       b->ev_join.push_back(e);
     }
