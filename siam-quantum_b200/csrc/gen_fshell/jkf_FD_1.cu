@@ -61,7 +61,8 @@ jkf_FD_1(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {
   double o9_3 = 0.0;
   double o9_4 = 0.0;
   double o9_5 = 0.0;
-  for (int i = 0; i < A.nprim; ++i) {
+  const int gi = it.split & 255, gj = (it.split >> 8) & 255, si = (it.split >> 16) & 255, sj = it.split >> 24;
+  for (int i = gi; i < A.nprim; i += si) {      // this item's part of the primitives
     const double* pa = a.prims + (size_t)(A.poff + i) * sqb::kGenPrimStride;
     const double p = pa[0], Px = pa[1], Py = pa[2], Pz = pa[3], kpa = pa[4];
     double g000 = 0.0;
@@ -121,7 +122,7 @@ jkf_FD_1(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {
     double g014 = 0.0;
     double g005 = 0.0;
     bool any = false;
-    for (int j = 0; j < B.nprim; ++j) {          // one contraction length per warp
+    for (int j = gj; j < B.nprim; j += sj) {     // one contraction length per warp
       const double* pb = a.prims + (size_t)(B.poff + j) * sqb::kGenPrimStride;
       const double q = pb[0], pq = p + q, rs = rsqrt(pq);
       const bool live = ok && !(TWO_PI_2_5 * kpa * pb[4] * rs < PRIM_CUTOFF);

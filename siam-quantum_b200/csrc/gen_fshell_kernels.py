@@ -79,14 +79,15 @@ def gen_kernel(qt, blk):
     for a_ in fa:
         for b_ in range(nb):
             em("double o%d_%d = 0.0;" % (a_, b_))
-    em("for (int i = 0; i < A.nprim; ++i) {")
+    em("const int gi = it.split & 255, gj = (it.split >> 8) & 255, si = (it.split >> 16) & 255, sj = it.split >> 24;")
+    em("for (int i = gi; i < A.nprim; i += si) {      // this item's part of the primitives")
     em.ind += 1
     em("const double* pa = a.prims + (size_t)(A.poff + i) * sqb::kGenPrimStride;")
     em("const double p = pa[0], Px = pa[1], Py = pa[2], Pz = pa[3], kpa = pa[4];")
     for h in H:
         em("double g%s = 0.0;" % hn(h))
     em("bool any = false;")
-    em("for (int j = 0; j < B.nprim; ++j) {          // one contraction length per warp")
+    em("for (int j = gj; j < B.nprim; j += sj) {     // one contraction length per warp")
     em.ind += 1
     em("const double* pb = a.prims + (size_t)(B.poff + j) * sqb::kGenPrimStride;")
     em("const double q = pb[0], pq = p + q, rs = rsqrt(pq);")
@@ -197,7 +198,7 @@ def gen_kernel(qt, blk):
         em("    const double z = sqb::warp_sum_scatter<%d>(v); const int x = lane + %d;" % (M, s0))
         em("    if (lane < %d && z != 0.0) atomicAdd(a.b.J + (fP + %d + x / %d) * N + fQ + x %% %d, z); }" % (len(part), fa[0], nb, nb))
     em("}")
-    em("sqb::count_add(a.counters + 0, ok && cd == 0%s ? 1ull : 0ull);" % ("" if blk == 0 else " && false"))
+    em("sqb::count_add(a.counters + 0, ok && cd == 0%s ? 1ull : 0ull);" % (" && gi == 0 && gj == 0" if blk == 0 else " && false"))
     em("sqb::count_add(a.counters + 1, npq);")
     em("sqb::count_add(a.counters + 2, nfl);")
     out = ['extern "C" __global__ void __launch_bounds__(%d)' % (32 * WARPS),

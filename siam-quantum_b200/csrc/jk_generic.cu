@@ -656,6 +656,13 @@ int gen_schwarz(const GenPath& g, int nbf, double* S, cudaStream_t st) {
   return SQB200_OK;
 }
 
+// Primitive quartets one warp of the f-shell kernels runs in a row.  Whole contractions (up to 216 in
+// water/QZP: an f shell with a core s shell against two core s shells) kept a few warps busy for a
+// millisecond while the SMs idled (20% of the time active).  Measured on B200, ms per build at 4 / 8 / 16 /
+// 36 and whole: water/QZP 2.50 / 2.48 / 2.51 / 2.99 / 3.12, ammonia/QZP 5.64 / 5.59 / 5.56 / 5.75, OH/QZP (UHF)
+// 1.12 / 1.11 / 1.20 / 1.77.
+constexpr int kFSteps = 8;
+
 // The lanes' function pairs of a ket of n: chunks (c0, g), one lane each, 32 / g kets side by side.
 // Up to 16 at once; a larger rest as 16 and a rest of at most 8 when that fills the warps better
 // (18 = 16 + 2, 24 = 16 + 8), else whole.
@@ -713,10 +720,20 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
       if (b >= e) continue;
       const int L = A.lP + A.lQ + B.lP + B.lQ;
       f_chunks(B.nfP * B.nfQ, chunks);
+      // contracted quartets in parts of at most kFSteps primitive quartets, which digest their own
+      // partial blocks: one bra primitive each, then runs of ket primitives
+      unsigned si = 1, sj = 1;
+      if (A.nprim * B.nprim > kFSteps) {
+        si = std::min(A.nprim, 255);
+        sj = std::min((B.nprim + kFSteps - 1) / kFSteps, 255);
+      }
       for (const auto& c : chunks) {
         const int ng = std::max(1, std::min(32 / c.second, kFWarpDoubles / f_slot(L)));
         for (const int* q = b; q < e; q += ng)
-          seg[g.fclass[x]].push_back({a, (int)(q - g.klist.data()), (int)std::min<long>(ng, e - q), c.first | c.second << 16});
+          for (unsigned gi = 0; gi < si; ++gi)
+            for (unsigned gj = 0; gj < sj; ++gj)
+              seg[g.fclass[x]].push_back({a, (int)(q - g.klist.data()), (int)std::min<long>(ng, e - q),
+                                          c.first | c.second << 16, gi | gj << 8 | si << 16 | sj << 24});
       }
     }
   }
@@ -725,7 +742,8 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
   for (int q = 0; q < 5; ++q) {
     auto key = [&](const FItem& it) {
       const GenPairRec &A = g.pairs[it.bra], &B = g.pairs[g.klist[it.k0]];
-      return (long long)A.nprim * B.nprim * (20 + B.nfP * B.nfQ);
+      const int si = (it.split >> 16) & 255, sj = it.split >> 24;
+      return (long long)((A.nprim + si - 1) / si) * ((B.nprim + sj - 1) / sj) * (20 + B.nfP * B.nfQ);
     };
     std::stable_sort(seg[q].begin(), seg[q].end(), [&](const FItem& x, const FItem& y) { return key(x) > key(y); });
     fitems.insert(fitems.end(), seg[q].begin(), seg[q].end());

@@ -47,9 +47,12 @@ struct GenItem {
 };
 
 // A warp's unit of the f-shell kernels (gen_fshell_kernels.py): one bra pair and the cnt ket pairs
-// klist[k0 ..], g function pairs from c0 of each (cg = c0 | g << 16), one lane per function pair.
+// klist[k0 ..], g function pairs from c0 of each (cg = c0 | g << 16), one lane per function pair; of
+// the primitives the bra's gi, gi + si, ... and the ket's gj, gj + sj, ... (split = gi | gj << 8 |
+// si << 16 | sj << 24).
 struct FItem {
   int bra, k0, cnt, cg;
+  unsigned split;
 };
 
 // Shared memory of one warp of the f-shell kernels (doubles), and of one quartet of total order L:
