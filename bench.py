@@ -591,8 +591,7 @@ def run_reference_split(args, atoms, bname, PA, desc, procs, sqb):
 # kernel, from one `ncu --set full` capture of the same workload; the summary with its command
 # is profiles/<kernel>_<workload>.md.  Kernels without a capture report null.
 TRAFFIC = {("benzene", "jk_DL_LL_R"): 970752, ("benzene", "jk_DL_LL_R_w"): 890112,
-           ("benzene", "jk_DL_LL_R_s"): 1268992, ("c60-synthetic", "jk_LL_LL_R_w"): 18592768, ("c60", "jk_LL_LL_R_w"): 20667648,
-           ("water-qzp", "k_jk_gen"): 1336320}
+           ("benzene", "jk_DL_LL_R_s"): 1268992, ("c60-synthetic", "jk_LL_LL_R_w"): 18592768, ("c60", "jk_LL_LL_R_w"): 20667648}
 
 
 def max_over_ranks(dist, t_local, device):
@@ -718,8 +717,8 @@ def run_ours(args, sqb):
     dom32 = dom["class"].endswith(" f32")
     total_flops = sum(r["flops"] for r in prof)
     peak = fp32_peak if dom32 else fp64_peak
-    # (the generic kernel of quartets with f shells counts the operations it executes)
-    dom_name = "k_jk_gen" if dom["class"].startswith("generic") else "jk_" + dom["class"].replace(" f32", "").replace("|", "_") + (
+    # (the f-shell kernels, one row for all of them, count the operations they execute)
+    dom_name = "jkf_F*" if dom["class"].startswith("generic") else "jk_" + dom["class"].replace(" f32", "").replace("|", "_") + (
         "_R_f32" if dom32 else {1: "_R_w", 2: "_R_s"}.get(int(tiles[dom["index"]]) if dom["index"] < len(tiles) else 0, "_R"))
     roof = {"bound": "fp32" if dom32 else "fp64",
             "kernel": dom_name,
@@ -735,7 +734,7 @@ def run_ours(args, sqb):
         roof["traffic"] = tb
         roof["traffic_source"] = "ncu dram__bytes_read.sum + dram__bytes_write.sum, profiles/%s" % (
             {"benzene": "jk_DL_LL_R_forms_benzene_631gs.md", "c60-synthetic": "jk_LL_LL_R_w_c60_631g_synthetic.md",
-             "c60": "jk_LL_LL_R_w_c60_631g_refdensity.md", "water-qzp": "k_jk_gen_water_qzp.md"}.get(
+             "c60": "jk_LL_LL_R_w_c60_631g_refdensity.md"}.get(
                 args.workload, args.workload))
     line = {"metric": METRIC, "value": value, "unit": "builds/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_max / args.steps, "higher_is_better": True,
@@ -747,7 +746,7 @@ def run_ours(args, sqb):
                        "quartets_per_build": st["quartets"], "prim_quartets_per_build": st["prim_quartets"],
                        "tiles": ("autotuned forms per class: %d narrow, %d wide, %d swapped" % (
                            int((tiles == 0).sum()), int((tiles == 1).sum()), int((tiles == 2).sum()))
-                                 if not args.no_autotune else "narrow")
+                                 if not args.no_autotune else "default forms")
                                 if not args.tiles_from else "forms per class from %s" % args.tiles_from},
             "quartets_per_s": value * st["quartets"], "prim_quartets_per_s": value * st["prim_quartets"],
             "e2e": e2e, "roofline": roof, "clocks": clk,
@@ -805,7 +804,7 @@ def main():
     ap.add_argument("--slots", type=int, default=32, help="concurrent jobs of the serve workload")
     ap.add_argument("--cpu-seconds", type=float, default=12.0)
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-autotune", action="store_true", help="keep every class on its narrow tile")
+    ap.add_argument("--no-autotune", action="store_true", help="keep every class on its default form")
     ap.add_argument("--save-tiles", default="", help="write the per-class forms the run used to this file")
     ap.add_argument("--tiles-from", default="",
                     help="J/K workloads: take the per-class forms from this file (written by --save-tiles) "
