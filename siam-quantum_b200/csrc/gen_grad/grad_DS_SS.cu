@@ -39,7 +39,7 @@ grad_DS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   double g3 = 0.0;
   double g4 = 0.0;
   double g5 = 0.0;
-  double gmax = 0.0;
+  double gmax = 0.0, gsum = 0.0;
   if (ok) {
     const double ptk = 4.0 * PT[fc * N + fd];
     const double ta0c = PT[fa0 * N + fc], sa0c = PS[fa0 * N + fc];
@@ -57,17 +57,18 @@ grad_DS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     const double tb0c = PT[fb0 * N + fc], sb0c = PS[fb0 * N + fc];
     const double tb0d = PT[fb0 * N + fd], sb0d = PS[fb0 * N + fd];
     g0 = deg * (ptk * PT[fa0 * N + fb0] - (ta0c * tb0d + ta0d * tb0c + sa0c * sb0d + sa0d * sb0c));
-    gmax = fmax(gmax, fabs(g0));
+    gmax = fmax(gmax, fabs(g0)); gsum += g0;
     g1 = deg * (ptk * PT[fa1 * N + fb0] - (ta1c * tb0d + ta1d * tb0c + sa1c * sb0d + sa1d * sb0c));
-    gmax = fmax(gmax, fabs(g1));
+    gmax = fmax(gmax, fabs(g1)); gsum += g1;
     g2 = deg * (ptk * PT[fa2 * N + fb0] - (ta2c * tb0d + ta2d * tb0c + sa2c * sb0d + sa2d * sb0c));
-    gmax = fmax(gmax, fabs(g2));
+    gmax = fmax(gmax, fabs(g2)); gsum += g2;
     g3 = deg * (ptk * PT[fa3 * N + fb0] - (ta3c * tb0d + ta3d * tb0c + sa3c * sb0d + sa3d * sb0c));
-    gmax = fmax(gmax, fabs(g3));
+    gmax = fmax(gmax, fabs(g3)); gsum += g3;
     g4 = deg * (ptk * PT[fa4 * N + fb0] - (ta4c * tb0d + ta4d * tb0c + sa4c * sb0d + sa4d * sb0c));
-    gmax = fmax(gmax, fabs(g4));
+    gmax = fmax(gmax, fabs(g4)); gsum += g4;
     g5 = deg * (ptk * PT[fa5 * N + fb0] - (ta5c * tb0d + ta5d * tb0c + sa5c * sb0d + sa5d * sb0c));
-    gmax = fmax(gmax, fabs(g5));
+    gmax = fmax(gmax, fabs(g5)); gsum += g5;
+    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -45,7 +45,7 @@ grad_PL_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   double g9 = 0.0;
   double g10 = 0.0;
   double g11 = 0.0;
-  double gmax = 0.0;
+  double gmax = 0.0, gsum = 0.0;
   if (ok) {
     const double ptk = 4.0 * PT[fc * N + fd];
     const double ta0c = PT[fa0 * N + fc], sa0c = PS[fa0 * N + fc];
@@ -63,29 +63,30 @@ grad_PL_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     const double tb3c = PT[fb3 * N + fc], sb3c = PS[fb3 * N + fc];
     const double tb3d = PT[fb3 * N + fd], sb3d = PS[fb3 * N + fd];
     g0 = deg * (ptk * PT[fa0 * N + fb0] - (ta0c * tb0d + ta0d * tb0c + sa0c * sb0d + sa0d * sb0c));
-    gmax = fmax(gmax, fabs(g0));
+    gmax = fmax(gmax, fabs(g0)); gsum += g0;
     g1 = deg * (ptk * PT[fa0 * N + fb1] - (ta0c * tb1d + ta0d * tb1c + sa0c * sb1d + sa0d * sb1c));
-    gmax = fmax(gmax, fabs(g1));
+    gmax = fmax(gmax, fabs(g1)); gsum += g1;
     g2 = deg * (ptk * PT[fa0 * N + fb2] - (ta0c * tb2d + ta0d * tb2c + sa0c * sb2d + sa0d * sb2c));
-    gmax = fmax(gmax, fabs(g2));
+    gmax = fmax(gmax, fabs(g2)); gsum += g2;
     g3 = deg * (ptk * PT[fa0 * N + fb3] - (ta0c * tb3d + ta0d * tb3c + sa0c * sb3d + sa0d * sb3c));
-    gmax = fmax(gmax, fabs(g3));
+    gmax = fmax(gmax, fabs(g3)); gsum += g3;
     g4 = deg * (ptk * PT[fa1 * N + fb0] - (ta1c * tb0d + ta1d * tb0c + sa1c * sb0d + sa1d * sb0c));
-    gmax = fmax(gmax, fabs(g4));
+    gmax = fmax(gmax, fabs(g4)); gsum += g4;
     g5 = deg * (ptk * PT[fa1 * N + fb1] - (ta1c * tb1d + ta1d * tb1c + sa1c * sb1d + sa1d * sb1c));
-    gmax = fmax(gmax, fabs(g5));
+    gmax = fmax(gmax, fabs(g5)); gsum += g5;
     g6 = deg * (ptk * PT[fa1 * N + fb2] - (ta1c * tb2d + ta1d * tb2c + sa1c * sb2d + sa1d * sb2c));
-    gmax = fmax(gmax, fabs(g6));
+    gmax = fmax(gmax, fabs(g6)); gsum += g6;
     g7 = deg * (ptk * PT[fa1 * N + fb3] - (ta1c * tb3d + ta1d * tb3c + sa1c * sb3d + sa1d * sb3c));
-    gmax = fmax(gmax, fabs(g7));
+    gmax = fmax(gmax, fabs(g7)); gsum += g7;
     g8 = deg * (ptk * PT[fa2 * N + fb0] - (ta2c * tb0d + ta2d * tb0c + sa2c * sb0d + sa2d * sb0c));
-    gmax = fmax(gmax, fabs(g8));
+    gmax = fmax(gmax, fabs(g8)); gsum += g8;
     g9 = deg * (ptk * PT[fa2 * N + fb1] - (ta2c * tb1d + ta2d * tb1c + sa2c * sb1d + sa2d * sb1c));
-    gmax = fmax(gmax, fabs(g9));
+    gmax = fmax(gmax, fabs(g9)); gsum += g9;
     g10 = deg * (ptk * PT[fa2 * N + fb2] - (ta2c * tb2d + ta2d * tb2c + sa2c * sb2d + sa2d * sb2c));
-    gmax = fmax(gmax, fabs(g10));
+    gmax = fmax(gmax, fabs(g10)); gsum += g10;
     g11 = deg * (ptk * PT[fa2 * N + fb3] - (ta2c * tb3d + ta2d * tb3c + sa2c * sb3d + sa2d * sb3c));
-    gmax = fmax(gmax, fabs(g11));
+    gmax = fmax(gmax, fabs(g11)); gsum += g11;
+    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -29,7 +29,7 @@ grad_SS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
   const int fa0 = bp.fP + 0;
   const int fb0 = bp.fQ + 0;
   double g0 = 0.0;
-  double gmax = 0.0;
+  double gmax = 0.0, gsum = 0.0;
   if (ok) {
     const double ptk = 4.0 * PT[fc * N + fd];
     const double ta0c = PT[fa0 * N + fc], sa0c = PS[fa0 * N + fc];
@@ -37,7 +37,8 @@ grad_SS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     const double tb0c = PT[fb0 * N + fc], sb0c = PS[fb0 * N + fc];
     const double tb0d = PT[fb0 * N + fd], sb0d = PS[fb0 * N + fd];
     g0 = deg * (ptk * PT[fa0 * N + fb0] - (ta0c * tb0d + ta0d * tb0c + sa0c * sb0d + sa0d * sb0c));
-    gmax = fmax(gmax, fabs(g0));
+    gmax = fmax(gmax, fabs(g0)); gsum += g0;
+    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

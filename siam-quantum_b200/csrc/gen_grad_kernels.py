@@ -187,7 +187,7 @@ def gen_grad(bra, ket, only=None):
             em("const int f%s%d = %s + %s;" % (x, k, base, func_perm(t, k)))
     for ab in range(na * nb):
         em("double g%d = 0.0;" % ab)
-    em("double gmax = 0.0;")
+    em("double gmax = 0.0, gsum = 0.0;")
     em("if (ok) {")
     em.ind += 1
     em("const double ptk = 4.0 * PT[fc * N + fd];")
@@ -199,7 +199,8 @@ def gen_grad(bra, ket, only=None):
         for j in range(nb):
             em("g%d = deg * (ptk * PT[fa%d * N + fb%d] - (ta%dc * tb%dd + ta%dd * tb%dc + sa%dc * sb%dd + sa%dd * sb%dc));" % (
                 i * nb + j, i, j, i, j, i, j, i, j, i, j))
-            em("gmax = fmax(gmax, fabs(g%d));" % (i * nb + j))
+            em("gmax = fmax(gmax, fabs(g%d)); gsum += g%d;" % (i * nb + j, i * nb + j))
+    em("if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing")
     em.ind -= 1
     em("}")
     # thresholds on |G|: screen times (shell degeneracy / function degeneracy) of the function quartet

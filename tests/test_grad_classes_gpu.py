@@ -46,3 +46,18 @@ def test_class_gradient_matches_run_time_kernel(shells, screen, restricted, monk
         eng.close()
     assert np.abs(G[0]).max() > 0
     assert np.abs(G[0] - G[1]).max() <= 1e-11 * np.abs(G[1]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_class_gradient_of_a_density_that_is_not_finite_is_not_finite(bad):
+    sqb = load_sqb200()
+    b = _basis(sqb, SHELLS, 7)
+    n = b.nbf
+    P = 0.2 * np.ones((n, n))
+    P[3, 2] = P[2, 3] = bad
+    eng = sqb.JKEngine(b)
+    G = eng.gradient(np.array([6.0, 8.0, 1.0]), np.array([[0.0, 0.0, 0.1], [0.0, 1.9, -0.4], [1.3, -0.7, 1.1]]), P, P, P,
+                     terms=8)
+    eng.close()
+    assert not np.isfinite(G).all()
