@@ -2858,8 +2858,9 @@ extern "C" int sqb200_syev_batched(int device, int n, int batch, double* A, doub
 // quartet whose density factor times prefactor and weights is below 1e-10 (both 1e-10 screens
 // follow SQB200_GRAD_SCREEN when it is set).  Derivatives of a primitive by its centre raise and lower
 // its angular momentum, d/dA_x g_a = 2 alpha g_{a+1x} - a_x g_{a-1x}; the fourth centre follows
-// from translational invariance.  The integrals are McMurchie-Davidson with runtime loops (one
-// thread per shell quartet or function pair): a correctness-first form, not tuned.
+// from translational invariance.  The kernels below are McMurchie-Davidson with run-time loops (one
+// thread per shell quartet, or per function pair and nucleus); the two-electron term of a basis of
+// s, sp, p and d shells runs in the generated class kernels (gen_grad_kernels.py) instead.
 
 namespace {
 

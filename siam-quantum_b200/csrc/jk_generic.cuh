@@ -1,8 +1,10 @@
 // The generic J/K path: shell quartets that involve a shell outside the generated class
 // kernels -- f shells (10 Cartesian functions, read by read_GAMESS_BasisSet, reference
 // src/basis.c:488-499) or any other shell layout genGTOShell accepts (src/matrix.c:2527-2535:
-// TYPEF for 10 functions, TYPEX otherwise) -- computed by one kernel with run-time angular
-// momenta (jk_generic.cu).  Internal to the library.
+// TYPEF for 10 functions, TYPEX otherwise).  Quartets whose generic bra is a canonical f shell with a
+// canonical s, sp, p, d or f shell run in the generated f-shell kernels (gen_fshell_kernels.py), the
+// others, and all of them in the multipole mode, in one kernel with run-time angular momenta
+// (jk_generic.cu).  Internal to the library.
 #pragma once
 #include <cuda_runtime.h>
 
