@@ -186,8 +186,9 @@ int sqb200_batch_destroy(sqb200_batch *batch);
 int sqb200_batch_offsets(sqb200_batch *batch, long long *off);
 
 /* Per-molecule spin and cutoffs of the next builds (arrays of nmol), with the meaning of
- * sqb200_jk_build's restricted / scf_cutoff / fixed_cutoff / dscreen_rmax.  Synchronises the
- * batch's streams and rebuilds the work list when a spin or Schwarz cutoff changed. */
+ * sqb200_jk_build's restricted / scf_cutoff / fixed_cutoff / dscreen_rmax.  Waits for the
+ * batch's last build (on any stream, a graph's replay included) and rebuilds the work list
+ * when a spin or Schwarz cutoff changed. */
 int sqb200_batch_set_step(sqb200_batch *batch, const int *restricted, const double *scf_cutoff,
                           const double *fixed_cutoff, const double *dscreen_rmax);
 

@@ -2399,6 +2399,7 @@ struct sqb200_batch {
   std::vector<cudaStream_t> side;
   cudaEvent_t ev_fork = nullptr;
   std::vector<cudaEvent_t> ev_join;
+  cudaEvent_t ev_done = nullptr;        // after the last build enqueued, or replayed from a graph
   cudaStream_t stream = nullptr;
 };
 
@@ -2447,6 +2448,7 @@ __global__ void k_finalize_batch(const double* __restrict__ J, const double* __r
 void free_batch(sqb200_batch* b) {
   for (size_t i = 0; i < b->side.size(); ++i) side_give(b->device, b->side[i], b->ev_join[i]);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+  if (b->ev_done) cudaEventDestroy(b->ev_done);
   if (b->stream) { cudaStreamSynchronize(b->stream); cudaStreamDestroy(b->stream); }
   for (auto& k : b->cls) { cudaFree(k.d_pairs); cudaFree(k.d_prims); cudaFree(k.d_primsf); }
   void* ptrs[] = {b->d_mols, b->d_shfirst, b->d_shn, b->d_PT, b->d_PM, b->d_J, b->d_KA, b->d_KB,
@@ -2531,6 +2533,7 @@ extern "C" int sqb200_batch_create(sqb200_batch** out, int nmol, sqb200_jk* cons
   e = h2d(b->d_shfirst, fst.data(), fst.size() * sizeof(int), b->stream);
   if (e == cudaSuccess) e = h2d(b->d_shn, nf.data(), nf.size() * sizeof(int), b->stream);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming);
   if (e != cudaSuccess) return bail(SQB200_ECUDA, cudaGetErrorString(e));
   b->form.assign(sqb::kNumClassKernels, -1);
   b->persistent = mols[0]->persistent;
@@ -2570,8 +2573,8 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
     b->rec[m].cut_fixed = fixed_cutoff[m];
     b->rec[m].dscreen_rmax = dscreen_rmax[m];
   }
-  CUDA_OK(cudaStreamSynchronize(b->stream));
-  for (cudaStream_t s : b->side) CUDA_OK(cudaStreamSynchronize(s));
+  // a build in flight, on whichever stream, reads the records and the items until its last kernel
+  CUDA_OK(cudaEventSynchronize(b->ev_done));
   CUDA_OK(h2d(b->d_mols, b->rec.data(), b->nmol * sizeof(sqb::MolRec), b->stream));
   if (same) return SQB200_OK;
   b->kernel.clear(); b->spin.clear(); b->first.clear(); b->count.clear(); b->cost.clear();
@@ -2751,6 +2754,11 @@ extern "C" int sqb200_batch_build_device(sqb200_batch* b, const double* dPA, con
   k_finalize_batch<<<dim3((b->max_nbf * b->max_nbf + 255) / 256, b->nmol), 256, 0, st>>>(
       b->d_J, b->d_KA, b->d_KB, dJT, dKA, dKB, b->d_mols);
   CUDA_OK(cudaGetLastError());
+  // for set_step; inside a caller's capture as a node, so that every replay records it
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CUDA_OK(cudaStreamIsCapturing(st, &cs));
+  CUDA_OK(cudaEventRecordWithFlags(b->ev_done, st,
+                                   cs == cudaStreamCaptureStatusNone ? cudaEventRecordDefault : cudaEventRecordExternal));
   b->last_launches = 3 + (int)b->kernel.size();
   return SQB200_OK;
 }

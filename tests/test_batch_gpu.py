@@ -108,6 +108,38 @@ def test_batch_graph_replay_and_autotune():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("captured", [False, True])
+def test_set_step_waits_for_the_build_in_flight(captured):
+    """A build waits on the caller's stream behind other work; set_step with other cutoffs and spins,
+    called at once, must not reach it: its records and work list are the build's until it ends."""
+    import torch
+    sqb, gs, engs, batch, PA, PB = _setup(["h2co_631gs", "water_321g"])
+    batch.set_step([True, True], 1e-10, 1e-10, 0.0)
+    st = torch.cuda.Stream()
+    out = _outs(batch)
+    build = lambda: batch.build_device(PA.data_ptr(), PB.data_ptr(), *(x.data_ptr() for x in out), stream=st.cuda_stream)
+    with torch.cuda.stream(st):
+        build()
+        st.synchronize()
+        ref = [x.clone() for x in out]
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                build()
+        for x in out:
+            x.fill_(float("nan"))
+        torch.cuda._sleep(50_000_000)           # some 25 ms
+        g.replay() if captured else build()
+        batch.set_step([False, False], 1e-2, 1e-2, float("inf"))
+        st.synchronize()
+    for x, y in zip(out, ref):
+        assert torch.abs(x - y).max().item() <= TOL_SAME
+    if captured:
+        del g
+    batch.close()
+
+
+@pytest.mark.gpu
 def test_single_context_autotune_keeps_results():
     import torch
     sqb = load_sqb200()
