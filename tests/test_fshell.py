@@ -216,6 +216,7 @@ def test_fshell_dropin_default_schedule_multipole_mode(maxmem):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not port.ref_available(), reason="oracle/_ref not built")
 def test_fshell_multipole_visits_match_reference():
     """Reference-parity multipole mode over SCF-like visits (a full density, then shrinking
     difference densities at tightening cutoffs) against the reference's own sequence."""

@@ -3,6 +3,7 @@ Boys function, screening and accumulation).  Errors are stated against the plain
 and, through the relinked reference program (which builds with difference densities each
 SCF iteration), against the reference's FP64 SCF energy: the bar is 1e-6 Eh."""
 import json
+import os
 
 import numpy as np
 import pytest
@@ -59,6 +60,7 @@ def test_mixed_error_shrinks_with_tau(case, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not os.path.exists(SQREF_GPU), reason="oracle/_ref/sqref_b200 not built")
 @pytest.mark.parametrize("tau", [1e-4, 1e-6])
 def test_mixed_scf_energy_within_1e6(tau, monkeypatch):
     """Whole SCF through the reference's own uhf() (1STEP), GPU Fock build in mixed precision."""

@@ -35,6 +35,7 @@ def _visits(n, P0, seed):
 
 
 @pytest.mark.gpu
+@pytest.mark.skipif(not port.ref_available(), reason="oracle/_ref not built")
 @pytest.mark.parametrize("case,max_mem", [("water_321g", 0), ("h2co_631gs", 0), ("h2co_631gs", 1)])
 def test_multipole_visits_match_reference(case, max_mem):
     sqb = load_sqb200()
