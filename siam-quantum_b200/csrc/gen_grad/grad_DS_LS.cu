@@ -68,7 +68,7 @@ grad_DS_LS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     gmax = fmax(gmax, fabs(g4)); gsum += g4;
     g5 = deg * (ptk * PT[fa5 * N + fb0] - (ta5c * tb0d + ta5d * tb0c + sa5c * sb0d + sa5d * sb0c));
     gmax = fmax(gmax, fabs(g5)); gsum += g5;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

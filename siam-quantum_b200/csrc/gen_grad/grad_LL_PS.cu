@@ -101,7 +101,7 @@ grad_LL_PS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     gmax = fmax(gmax, fabs(g14)); gsum += g14;
     g15 = deg * (ptk * PT[fa3 * N + fb3] - (ta3c * tb3d + ta3d * tb3c + sa3c * sb3d + sa3d * sb3c));
     gmax = fmax(gmax, fabs(g15)); gsum += g15;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

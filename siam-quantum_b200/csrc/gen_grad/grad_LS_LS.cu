@@ -56,7 +56,7 @@ grad_LS_LS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     gmax = fmax(gmax, fabs(g2)); gsum += g2;
     g3 = deg * (ptk * PT[fa3 * N + fb0] - (ta3c * tb0d + ta3d * tb0c + sa3c * sb0d + sa3d * sb0c));
     gmax = fmax(gmax, fabs(g3)); gsum += g3;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -86,7 +86,7 @@ grad_PL_LS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     gmax = fmax(gmax, fabs(g10)); gsum += g10;
     g11 = deg * (ptk * PT[fa2 * N + fb3] - (ta2c * tb3d + ta2d * tb3c + sa2c * sb3d + sa2d * sb3c));
     gmax = fmax(gmax, fabs(g11)); gsum += g11;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -74,7 +74,7 @@ grad_PP_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     gmax = fmax(gmax, fabs(g7)); gsum += g7;
     g8 = deg * (ptk * PT[fa2 * N + fb2] - (ta2c * tb2d + ta2d * tb2c + sa2c * sb2d + sa2d * sb2c));
     gmax = fmax(gmax, fabs(g8)); gsum += g8;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -38,7 +38,7 @@ grad_SS_SS(const sqb::GradArgs a, const sqb::WorkItem* __restrict__ items) {
     const double tb0d = PT[fb0 * N + fd], sb0d = PS[fb0 * N + fd];
     g0 = deg * (ptk * PT[fa0 * N + fb0] - (ta0c * tb0d + ta0d * tb0c + sa0c * sb0d + sa0d * sb0c));
     gmax = fmax(gmax, fabs(g0)); gsum += g0;
-    if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing
+    if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing
   }
   const double th = screen * (same_k && fc != fd ? 0.5 : 1.0), tho = same_b ? 0.5 * th : th;
   const double hp = same_pair ? 0.5 : 1.0;    // function pairs of one shell pair that differ

@@ -200,7 +200,7 @@ def gen_grad(bra, ket, only=None):
             em("g%d = deg * (ptk * PT[fa%d * N + fb%d] - (ta%dc * tb%dd + ta%dd * tb%dc + sa%dc * sb%dd + sa%dd * sb%dc));" % (
                 i * nb + j, i, j, i, j, i, j, i, j, i, j))
             em("gmax = fmax(gmax, fabs(g%d)); gsum += g%d;" % (i * nb + j, i * nb + j))
-    em("if (!(gsum - gsum == 0.0)) gmax = gsum;       // fmax drops a NaN: a density that is not finite skips nothing")
+    em("if (!(gsum - gsum == 0.0)) gmax = fabs(gsum); // fmax drops a NaN: a density that is not finite skips nothing")
     em.ind -= 1
     em("}")
     # thresholds on |G|: screen times (shell degeneracy / function degeneracy) of the function quartet

@@ -61,3 +61,21 @@ def test_class_gradient_of_a_density_that_is_not_finite_is_not_finite(bad):
                      terms=8)
     eng.close()
     assert not np.isfinite(G).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+def test_class_gradient_keeps_an_infinite_density_factor_of_either_sign(sign):
+    """Two H2 molecules 40 bohr apart; one density element of the first is infinite, the second
+    molecule's elements have one sign.  The only quartets that join the two are Coulomb ones, so
+    every density factor that reaches the second molecule is an infinity of that sign."""
+    sqb = load_sqb200()
+    xyz = np.array([[0.0, 0.0, z] for z in (0.0, 1.4, 40.0, 41.4)])
+    b = sqb.basis.build_basis([(1, *r) for r in xyz], "sto-3g")
+    P = np.zeros((2, 4, 4))
+    P[0, 0, 1] = P[0, 1, 0] = np.inf
+    P[0, 2:, 2:], P[1, 2:, 2:] = 0.3 * sign, 0.1 * sign
+    eng = sqb.JKEngine(b)
+    G = eng.gradient(np.ones(4), xyz, P[0], P[1], P[1], terms=8)
+    eng.close()
+    assert not np.isfinite(G[2:]).all(axis=1).any()
