@@ -1142,15 +1142,23 @@ double build_ops(const sqb200_jk* c, double outer, double fixed) {
 // 240; C60/6-31G (8e11) 68.2 / 57.4 / 56.0 / 56.2 at 10, 30 and 100 thousand and unsplit.
 double chain_ops(double ops) { return std::max({3000.0, std::min(4e-6 * ops, 2e4), 1.5e-7 * ops}); }
 
+// Kets of one FP32 item in the unit that f32_min_items counts in: items of 64 threads whose quartets
+// are split over their bra primitives alone, down to 32 primitive quartets a thread.
+int f32_item_kets(int nbp, int nkp) {
+  int split = 1;
+  while (split * 2 <= nbp && split * 2 <= 32 && (long)nbp * nkp / (split * 2) >= 32) split *= 2;
+  return 64 / split;
+}
+
 // Work items of class kernel ki for one molecule (context c): every surviving (bra pair, <=kper
 // ket pairs) unit, with pair indices shifted by bra_base/ket_base (the molecule's first pair in
 // a merged class array; 0 for a single-molecule build).  Kets whose Schwarz product is below the
-// context's fp32_below go to items32 (the FP32 form).  cost64/cost32 accumulate the emitted
-// operations, the launch-order and stream-balancing estimate.
+// context's fp32_below go to items32 (the FP32 form); n32 counts them in f32_item_kets' unit.
+// cost64/cost32 accumulate the emitted operations, the launch-order and stream-balancing estimate.
 void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra_base, int ket_base, int mol,
-                 double chain, int cta, std::vector<sqb::WorkItem>& items, std::vector<sqb::WorkItem>& items32, double& cost64,
-                 double& cost32, std::vector<int>* ers = nullptr, long long* er_run = nullptr,
-                 bool allow_f32 = true) {
+                 double chain, int cta, std::vector<sqb::WorkItem>& items, std::vector<sqb::WorkItem>& items32,
+                 size_t& n32, double& cost64, double& cost32, std::vector<int>* ers = nullptr,
+                 long long* er_run = nullptr, bool allow_f32 = true) {
   const sqb::ClassKernel& K = sqb::kClassKernels[ki];
   const PairClass& B = c->cls[K.bra_cls];
   const PairClass& T = c->cls[K.ket_cls];
@@ -1182,6 +1190,7 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
     const int split = run.split, kper = cta / ((split & 0xffff) * (split >> 16));
     const int b0 = B.sub[sx], b1 = B.sub[sx + 1], k0s = T.sub[sy], k1s = T.sub[sy + 1];
     const int nbp = B.pairs[b0].nprim, nkp = T.pairs[k0s].nprim;
+    const int kets32 = f32_item_kets(nbp, nkp);
     const double pq = (double)nbp * nkp;
     for (int b = b0; b < b1; ++b) {
       const double sb = B.pairs[b].schwarz;
@@ -1224,28 +1233,29 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
       }
       for (int k0 = std::max(start, mid); k0 < end; k0 += kper)
         items32.push_back({bra_base + b, ket_base + k0, std::min(kper, end - k0), split, mol});
+      n32 += (std::max(0, end - std::max(start, mid)) + kets32 - 1) / kets32;
       cost64 += std::max(0, mid - start) * (pq * K.flops_prim + K.flops_quartet);
       cost32 += std::max(0, end - std::max(start, mid)) * (pq * K.f32_flops_prim + K.f32_flops_quartet);
     }
   }
 }
 
-// A class whose FP32 work items would number fewer than this runs all its quartets in FP64: a
+// A class whose FP32 quartets would make fewer work items than this runs all its quartets in FP64: a
 // second launch of a few hundred CTAs costs more than its FP32 arithmetic saves, and splitting
 // the ket ranges at the FP32 threshold leaves the FP64 items shorter (SQB200_F32_MIN_ITEMS,
 // default 2400, read whenever a work list is made; measured on B200: benzene/6-31G* at tau 1e-5
 // 0.729 ms with 600, 0.725 with 1200, 0.716 with 2400, against 0.713-0.720 in FP64; C60/6-31G
-// 50.5 ms with each, against 63.1 in FP64).
+// 50.5 ms with each, against 63.1 in FP64).  Which quartets lose precision must not depend on the
+// shape of a build's items (their width and splits follow the build's size), so the count is
+// in items of one fixed shape, f32_item_kets, the one those figures were taken with.
 size_t f32_min_items() {
   const char* e = getenv("SQB200_F32_MIN_ITEMS");
   return e ? (size_t)std::max(0L, atol(e)) : (size_t)2400;
 }
 
-// True when a class's FP32 items are too few to launch: the class then runs all its quartets
-// in FP64, with the work items of a build without the FP32 split.
-bool too_few_f32(const std::vector<sqb::WorkItem>& items32) {
-  return !items32.empty() && items32.size() < f32_min_items();
-}
+// True when a class's FP32 quartets (n32 items) are too few to launch: the class then runs all its
+// quartets in FP64, with the work items of a build without the FP32 split.
+bool too_few_f32(size_t n32) { return n32 > 0 && n32 < f32_min_items(); }
 
 int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) {
   const int mpm = c->mp_on ? 1 : 0;
@@ -1265,14 +1275,15 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
   for (int ki = 0; ki < sqb::kNumClassKernels; ++ki) {
     const int first = (int)items.size();
     items32.clear();
+    size_t n32 = 0;
     double cost64 = 0.0, cost32 = 0.0;
-    class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, cost64, cost32, mpm ? &ers : nullptr,
+    class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, n32, cost64, cost32, mpm ? &ers : nullptr,
                 mpm ? &er_run : nullptr);
-    if (too_few_f32(items32)) {
+    if (too_few_f32(n32)) {
       items.resize(first);
       items32.clear();
       cost64 = cost32 = 0.0;
-      class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, cost64, cost32, nullptr, nullptr, false);
+      class_items(c, ki, outer, fixed, 0, 0, 0, chain, w.cta, items, items32, n32, cost64, cost32, nullptr, nullptr, false);
     }
     const int cnt = (int)items.size() - first;
     if (cnt > 0) {
@@ -2589,22 +2600,23 @@ extern "C" int sqb200_batch_set_step(sqb200_batch* b, const int* restricted, con
       const sqb::ClassKernel& K = sqb::kClassKernels[ki];
       const int f64 = (int)items.size();
       items32.clear();
+      size_t n32 = 0;
       double c64 = 0.0, c32 = 0.0;
       // (the items come longest loops first inside each molecule: across molecules that would
       // interleave their pair data and J/K blocks in L2, measured 4% slower on 256 molecules)
       for (int m = 0; m < b->nmol; ++m) {
         if (b->rec[m].uhf != sp) continue;
         class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
-                    b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32);
+                    b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, n32, c64, c32);
       }
-      if (too_few_f32(items32)) {
+      if (too_few_f32(n32)) {
         items.resize(f64);
         items32.clear();
         c64 = c32 = 0.0;
         for (int m = 0; m < b->nmol; ++m) {
           if (b->rec[m].uhf != sp) continue;
           class_items(b->mols[m], ki, scf_cutoff[m], fixed_cutoff[m], b->cls[K.bra_cls].pair_base[m],
-                      b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, c64, c32, nullptr, nullptr,
+                      b->cls[K.ket_cls].pair_base[m], m, chain, b->cta, items, items32, n32, c64, c32, nullptr, nullptr,
                       false);
         }
       }

@@ -71,3 +71,27 @@ def test_mixed_scf_energy_within_1e6(tau, monkeypatch):
     with open(results_path("mixed_scf_err_%g.json" % tau), "w") as f:
         json.dump({"tau": tau, "energy": e, "reference": float(g["energy"]), "abs_err": err}, f)
     assert err <= 1e-6, err
+
+
+# (heavy atoms, tau): the classes that launch their FP32 form for a 6-31G* organic
+F32_CLASSES = {(5, 1e-5): set(), (9, 1e-5): {"LS|SS"}, (9, 1e-3): {"LS|SS"},
+               (11, 1e-5): {"DS|LS", "DS|SS", "LS|LS", "LS|SS", "SS|SS"},
+               (13, 1e-5): {"DL|LS", "DL|SS", "DS|LS", "DS|SS", "LL|LS", "LL|SS", "LS|LS", "LS|SS", "SS|SS"}}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heavy,tau", sorted(F32_CLASSES))
+def test_fp32_classes_do_not_depend_on_the_item_shape(heavy, tau):
+    """A class runs quartets in FP32 from 2400 FP32 items of 64 threads on, counted in items of one
+    fixed shape: the items that a build is cut into get narrower and more with smaller builds,
+    which must not move quartets to FP32."""
+    sqb = load_sqb200()
+    atoms = sqb.molecules.to_bohr(sqb.molecules.random_organic(np.random.default_rng([3, heavy]), heavy))
+    b = sqb.basis.build_basis(atoms, "6-31g*")
+    eng = sqb.JKEngine(b)
+    eng.set_precision(tau)
+    eng.profile(True)
+    eng.build(np.eye(b.nbf), scf_cutoff=1e-10)
+    got = {r["class"] for r in eng.profile_read() if r["class"].endswith("f32")}
+    eng.close()
+    assert got == {c + " f32" for c in F32_CLASSES[heavy, tau]}
