@@ -171,9 +171,12 @@ __device__ __forceinline__ void boys(double T, const double* __restrict__ tab, d
     const double rt = rsqrt(T);
     F[0] = 0.88622692545275801365 * rt;          // sqrt(pi)/2 / sqrt(T)
     if (M > 0) {
-      // e^-T is below 1e-17 of every (2m+1) F_m, m < 8, for T >= 64
+      // e^-T is below 3e-18 of every (2m+1) F_m, m <= 8, for T >= 64
       const double e = T < 64.0 ? exp(-T) : 0.0;
-      const double h = 0.5 * rt * rt;
+      // 1/T = rt rt with one Newton step: the error of h enters every order anew (with rt rt
+      // alone F_8 has an rms error of 8.0 units of 2^-53 over T = 36..400, with the step 3.9,
+      // with a division 4.0)
+      const double q = rt * rt, h = 0.5 * fma(q, fma(-T, q, 1.0), q);
 #pragma unroll
       for (int m = 0; m < M; ++m) F[m + 1] = fma(2 * m + 1, F[m], -e) * h;
     }
@@ -202,7 +205,7 @@ __device__ __forceinline__ void boysf(float T, const float* __restrict__ tab, fl
     F[0] = 0.886226925f * rt;
     if (M > 0) {
       const float e = expf(-T);
-      const float h = 0.5f * rt * rt;
+      const float q = rt * rt, h = 0.5f * fmaf(q, fmaf(-T, q, 1.0f), q);   // as boys<M>
 #pragma unroll
       for (int m = 0; m < M; ++m) F[m + 1] = ((float)(2 * m + 1) * F[m] - e) * h;
     }

@@ -81,3 +81,20 @@ def test_boys_matches_exact_and_reference():
     with open(results_path("boys_vs_exact_and_fgamma_set.json"), "w") as f:
         json.dump({"max_rel_err_vs_exact": worst_exact, "max_rel_err_vs_reference_T_ge_5e-4": worst_ref,
                    "points": len(T)}, f)
+
+
+@pytest.mark.gpu
+def test_boys_upward_recursion_rounds_as_a_division_would():
+    """T >= 36: F_0 = sqrt(pi/T)/2 and F_{m+1} = ((2m+1) F_m - e^-T) h with h = 1/(2T).  A rounding
+    has an rms of about 0.42 units (2^-53 of the value).  With h correctly rounded F_m carries three
+    roundings of F_0, two of each of its m steps, and m times the one error of h:
+    0.42 sqrt(m^2 + 2m + 3) units; the bar is 1.4 times that, for every order."""
+    sqb = load_sqb200()
+    T = np.random.default_rng(7).uniform(36.1, 400.0, 200000)
+    x = T.astype(np.longdouble)
+    F = sqb.engine.boys_eval(8, T)
+    exact = np.sqrt(np.longdouble("3.14159265358979323846264338327950288") / x) / 2
+    for m in range(9):
+        rms = float(np.sqrt((((F[:, m] - exact) / exact) ** 2).mean())) * 2.0 ** 53
+        assert rms <= 1.4 * 0.42 * np.sqrt(m * m + 2 * m + 3), (m, rms)
+        exact = ((2 * m + 1) * exact - np.exp(-x)) / (2 * x)
