@@ -2,12 +2,13 @@
 #include "../jk_generic_dev.cuh"
 
 extern "C" __global__ void __launch_bounds__(128)
-jkf_FS_0(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {
+jkf_FS_0(const sqb::FArgs a, const sqb::FRun* __restrict__ runs, const long long* __restrict__ first, int nruns,
+   long long u0, long long nunits) {
   extern __shared__ double fsm[];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int ii = blockIdx.x * 4 + wp;
-  if (ii >= nitems) return;                     // whole warps leave
-  const sqb::FItem it = items[ii];
+  const long long unit = u0 + (long long)blockIdx.x * 4 + wp;
+  if (unit >= nunits) return;                   // whole warps leave
+  const sqb::FUnit it = sqb::f_unit(runs, first, nruns, unit);
   const int g = it.cg >> 16, s = lane / g, cc = lane - s * g, cd = (it.cg & 0xffff) + cc;
   const sqb::GenPairRec A = a.pairs[it.bra];
   const int kb = a.klist[it.k0 + min(s, it.cnt - 1)];   // idle lanes shadow the last ket
@@ -41,8 +42,8 @@ jkf_FS_0(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {
   double o7_0 = 0.0;
   double o8_0 = 0.0;
   double o9_0 = 0.0;
-  const int gi = it.split & 255, gj = (it.split >> 8) & 255, si = (it.split >> 16) & 255, sj = it.split >> 24;
-  for (int i = gi; i < A.nprim; i += si) {      // this item's part of the primitives
+  const int gi = it.gi, gj = it.gj, si = it.si, sj = it.sj;
+  for (int i = gi; i < A.nprim; i += si) {      // this unit's part of the primitives
     const double* pa = a.prims + (size_t)(A.poff + i) * sqb::kGenPrimStride;
     const double p = pa[0], Px = pa[1], Py = pa[2], Pz = pa[3], kpa = pa[4];
     double g000 = 0.0;

@@ -50,9 +50,9 @@ def gen_kernel(qt, blk):
     em = Emitter()
     em("extern __shared__ double fsm[];")
     em("const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;")
-    em("const int ii = blockIdx.x * %d + wp;" % WARPS)
-    em("if (ii >= nitems) return;                     // whole warps leave")
-    em("const sqb::FItem it = items[ii];")
+    em("const long long unit = u0 + (long long)blockIdx.x * %d + wp;" % WARPS)
+    em("if (unit >= nunits) return;                   // whole warps leave")
+    em("const sqb::FUnit it = sqb::f_unit(runs, first, nruns, unit);")
     em("const int g = it.cg >> 16, s = lane / g, cc = lane - s * g, cd = (it.cg & 0xffff) + cc;")
     em("const sqb::GenPairRec A = a.pairs[it.bra];")
     em("const int kb = a.klist[it.k0 + min(s, it.cnt - 1)];   // idle lanes shadow the last ket")
@@ -79,8 +79,8 @@ def gen_kernel(qt, blk):
     for a_ in fa:
         for b_ in range(nb):
             em("double o%d_%d = 0.0;" % (a_, b_))
-    em("const int gi = it.split & 255, gj = (it.split >> 8) & 255, si = (it.split >> 16) & 255, sj = it.split >> 24;")
-    em("for (int i = gi; i < A.nprim; i += si) {      // this item's part of the primitives")
+    em("const int gi = it.gi, gj = it.gj, si = it.si, sj = it.sj;")
+    em("for (int i = gi; i < A.nprim; i += si) {      // this unit's part of the primitives")
     em.ind += 1
     em("const double* pa = a.prims + (size_t)(A.poff + i) * sqb::kGenPrimStride;")
     em("const double p = pa[0], Px = pa[1], Py = pa[2], Pz = pa[3], kpa = pa[4];")
@@ -202,7 +202,8 @@ def gen_kernel(qt, blk):
     em("sqb::count_add(a.counters + 1, npq);")
     em("sqb::count_add(a.counters + 2, nfl);")
     out = ['extern "C" __global__ void __launch_bounds__(%d)' % (32 * WARPS),
-           "%s(const sqb::FArgs a, const sqb::FItem* __restrict__ items, int nitems) {" % name] + em.lines + ["}"]
+           "%s(const sqb::FArgs a, const sqb::FRun* __restrict__ runs, const long long* __restrict__ first, int nruns," % name,
+           "   long long u0, long long nunits) {"] + em.lines + ["}"]
     return name, "\n".join(out) + "\n"
 
 
@@ -217,7 +218,7 @@ def main():
             write_if_changed(os.path.join(outdir, name + ".cu"), head + src)
             files.append(name + ".cu")
             reg.append((qt, name))
-    text = head + "".join('extern "C" __global__ void %s(const sqb::FArgs, const sqb::FItem*, int);\n' % n for _, n in reg)
+    text = head + "".join('extern "C" __global__ void %s(const sqb::FArgs, const sqb::FRun*, const long long*, int, long long, long long);\n' % n for _, n in reg)
     text += "\nnamespace sqb {\nconst FKernel kFKernels[%d] = {\n" % len(reg)
     for qt, n in reg:
         text += "  {%d, (const void*)%s},\n" % ("SLPDF".index(qt), n)

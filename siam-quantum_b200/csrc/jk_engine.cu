@@ -416,8 +416,10 @@ struct sqb200_jk {
     int cta = 64;                 // threads per CTA of the class kernels
     sqb::GenItem* d_gitems = nullptr;   // the generic path's items (shells outside the classes)
     int gtotal = 0;
-    sqb::FItem* d_fitems = nullptr;     // the f-shell kernels' items, by class fseg[q] .. fseg[q + 1]
+    sqb::FRun* d_fruns = nullptr;       // the f-shell kernels' runs (FWork)
+    long long* d_ffirst = nullptr;
     int fseg[6] = {0, 0, 0, 0, 0, 0};
+    long long funits[5] = {0, 0, 0, 0, 0};
     double ops = 0.0;                   // emitted operations of a build (estimate)
     int launches = 0;                   // kernels of a build
     // captured launches per spin (build_graph); `seen`, `stamp`: the form_stamp of the last direct
@@ -1307,19 +1309,23 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
   }
   if (c->gen.on) {
     std::vector<sqb::GenItem> gi;
-    std::vector<sqb::FItem> fi;
-    sqb::gen_items(c->gen, outer, fixed, gi, fi, w.fseg, mpm ? &er_run : nullptr);
-    if (gi.size() > (size_t)INT_MAX || fi.size() > (size_t)INT_MAX)
+    sqb::FWork fw;
+    sqb::gen_items(c->gen, outer, fixed, gi, fw, mpm ? &er_run : nullptr);
+    if (gi.size() > (size_t)INT_MAX || fw.runs.size() > (size_t)INT_MAX)
       return fail(SQB200_EINVAL, "generic path: more than 2^31 work items");
     w.gtotal = (int)gi.size();
     if (!gi.empty()) {
       CUDA_OK(cudaMalloc(&w.d_gitems, gi.size() * sizeof(sqb::GenItem)));
       CUDA_OK(h2d(w.d_gitems, gi.data(), gi.size() * sizeof(sqb::GenItem), c->stream));
     }
-    if (!fi.empty()) {
-      CUDA_OK(cudaMalloc(&w.d_fitems, fi.size() * sizeof(sqb::FItem)));
-      CUDA_OK(h2d(w.d_fitems, fi.data(), fi.size() * sizeof(sqb::FItem), c->stream));
+    if (!fw.runs.empty()) {
+      CUDA_OK(cudaMalloc(&w.d_fruns, fw.runs.size() * sizeof(sqb::FRun)));
+      CUDA_OK(h2d(w.d_fruns, fw.runs.data(), fw.runs.size() * sizeof(sqb::FRun), c->stream));
+      CUDA_OK(cudaMalloc(&w.d_ffirst, fw.first.size() * sizeof(long long)));
+      CUDA_OK(h2d(w.d_ffirst, fw.first.data(), fw.first.size() * sizeof(long long), c->stream));
     }
+    std::copy(fw.seg, fw.seg + 6, w.fseg);
+    std::copy(fw.units, fw.units + 5, w.funits);
   }
   if (mpm) {
     if (er_run > INT_MAX) return fail(SQB200_EINVAL, "multipole mode: more than 2^31 quartets survive the outer cutoff");
@@ -1543,7 +1549,7 @@ int launch_classes(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double outer, doub
     }
     std::vector<cudaStream_t> lanes(1, st);
     lanes.insert(lanes.end(), c->side.begin(), c->side.begin() + (nlanes - 1));
-    rc = sqb::gen_launch(c->gen, w->d_gitems, w->gtotal, w->d_fitems, w->fseg, gb, lanes.data(), nlanes);
+    rc = sqb::gen_launch(c->gen, w->d_gitems, w->gtotal, w->d_fruns, w->d_ffirst, w->fseg, w->funits, gb, lanes.data(), nlanes);
     if (rc) return rc;
     if (ev.a) {
       CUDA_OK(cudaEventRecord(ev.b, st));
@@ -1846,7 +1852,7 @@ int sqb200_jk_destroy(sqb200_jk* c) {
   for (auto& kv : c->work)
     for (auto& g : kv.second.graph)
       if (g.exec) cudaGraphExecDestroy(g.exec);
-  for (auto& kv : c->work) { cudaFree(kv.second.d_items); cudaFree(kv.second.d_er); cudaFree(kv.second.d_gitems); cudaFree(kv.second.d_fitems); }
+  for (auto& kv : c->work) { cudaFree(kv.second.d_items); cudaFree(kv.second.d_er); cudaFree(kv.second.d_gitems); cudaFree(kv.second.d_fruns); cudaFree(kv.second.d_ffirst); }
   sqb::gen_free(c->gen);
   if (c->d_mpbase) cudaFree(c->d_mpbase);
   if (c->d_erbase) cudaFree(c->d_erbase);

@@ -681,14 +681,14 @@ static void f_chunks(int n, std::vector<std::pair<int, int>>& out) {
   if (n > c0) out.push_back({c0, n - c0});
 }
 
-void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, std::vector<FItem>& fitems,
-               int fseg[6], long long* er_run) {
+void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, FWork& fw,
+               long long* er_run) {
   const double cut = std::max(outer, fixed);
   const int np = (int)g.pairs.size();
   // kets with schwarz >= c / S(A) (less a relative 1e-12 that the kernel's exact test takes
-  // back): a prefix of the sorted list
-  auto prefix = [&](double c, double sa) {
-    const double thr = c / sa * (1.0 - 1e-12);
+  // back) are a prefix of the sorted pairs
+  auto prefix = [&](double c, double sA) {
+    const double thr = c / sA * (1.0 - 1e-12);
     int lo = 0, hi = np;
     while (lo < hi) {
       const int mid = (lo + hi) / 2;
@@ -696,58 +696,68 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
     }
     return lo;
   };
-  std::vector<FItem> seg[5];
-  std::vector<std::pair<int, int>> chunks;
+  struct Bra { int a, kets; };
+  std::map<int, std::vector<Bra>> bras[5];          // per class, by contraction length
   for (size_t x = 0; x < g.gen_idx.size(); ++x) {
     const int a = g.gen_idx[x];
     const GenPairRec& A = g.pairs[a];
     if (!(A.schwarz > 0.0)) continue;
     const int lo = prefix(cut, A.schwarz);
     int er = -1;
-    if (er_run) {   // slots for the outer cutoff's survivors, so the layout does not depend on `fixed`
+    if (er_run) {
       er = (int)*er_run;
       *er_run += prefix(outer, A.schwarz);
     }
-    if (er_run || g.fclass[x] < 0) {
+    if (er_run || g.fclass[x] < 0)
       for (int k0 = 0; k0 < lo; k0 += kGenKets) items.push_back({a, k0, std::min(kGenKets, lo - k0), er});
-      continue;
-    }
-    for (size_t k = 0; k + 1 < g.kgroup.size(); ++k) {
-      const int *b = g.klist.data() + g.kgroup[k], *e = g.klist.data() + g.kgroup[k + 1];
-      const GenPairRec& B = g.pairs[*b];
-      if (B.gen) b = std::lower_bound(b, e, a);   // two generic pairs: taken once, from the earlier position
-      e = std::lower_bound(b, e, lo);
-      if (b >= e) continue;
-      const int L = A.lP + A.lQ + B.lP + B.lQ;
-      f_chunks(B.nfP * B.nfQ, chunks);
-      // contracted quartets in parts of at most kFSteps primitive quartets, which digest their own
-      // partial blocks: one bra primitive each, then runs of ket primitives
-      unsigned si = 1, sj = 1;
-      if (A.nprim * B.nprim > kFSteps) {
-        si = std::min(A.nprim, 255);
-        sj = std::min((B.nprim + kFSteps - 1) / kFSteps, 255);
-      }
-      for (const auto& c : chunks) {
-        const int ng = std::max(1, std::min(32 / c.second, kFWarpDoubles / f_slot(L)));
-        for (const int* q = b; q < e; q += ng)
-          for (unsigned gi = 0; gi < si; ++gi)
-            for (unsigned gj = 0; gj < sj; ++gj)
-              seg[g.fclass[x]].push_back({a, (int)(q - g.klist.data()), (int)std::min<long>(ng, e - q),
-                                          c.first | c.second << 16, gi | gj << 8 | si << 16 | sj << 24});
-      }
-    }
+    else
+      bras[g.fclass[x]][A.nprim].push_back({a, lo});
   }
-  // heaviest primitive loops and largest kets first
-  fseg[0] = 0;
+  // The runs of a class by (contraction length of the bra, ket group), heaviest primitive loops and
+  // largest kets first: what the order goes by is one value per such pair.  (A record per unit, sorted
+  // one by one, took 1.3 s and 155 MB for benzene/QZP's 7.7 million units.)
+  std::vector<std::pair<int, int>> chunks;
   for (int q = 0; q < 5; ++q) {
-    auto key = [&](const FItem& it) {
-      const GenPairRec &A = g.pairs[it.bra], &B = g.pairs[g.klist[it.k0]];
-      const int si = (it.split >> 16) & 255, sj = it.split >> 24;
-      return (long long)((A.nprim + si - 1) / si) * ((B.nprim + sj - 1) / sj) * (20 + B.nfP * B.nfQ);
-    };
-    std::stable_sort(seg[q].begin(), seg[q].end(), [&](const FItem& x, const FItem& y) { return key(x) > key(y); });
-    fitems.insert(fitems.end(), seg[q].begin(), seg[q].end());
-    fseg[q + 1] = (int)fitems.size();
+    struct Block { long long key; const std::vector<Bra>* bras; size_t group; int si, sj; };
+    std::vector<Block> blocks;
+    for (const auto& kv : bras[q])
+      for (size_t k = 0; k + 1 < g.kgroup.size(); ++k) {
+        const GenPairRec& B = g.pairs[g.klist[g.kgroup[k]]];
+        const int na = kv.first;
+        // contracted quartets in parts of at most kFSteps primitive quartets, which digest their own
+        // partial blocks: one bra primitive each, then runs of ket primitives
+        int si = 1, sj = 1;
+        if (na * B.nprim > kFSteps) {
+          si = std::min(na, 255);
+          sj = std::min((B.nprim + kFSteps - 1) / kFSteps, 255);
+        }
+        const long long key = (long long)((na + si - 1) / si) * ((B.nprim + sj - 1) / sj) * (20 + B.nfP * B.nfQ);
+        blocks.push_back({key, &kv.second, k, si, sj});
+      }
+    std::stable_sort(blocks.begin(), blocks.end(), [](const Block& x, const Block& y) { return x.key > y.key; });
+    long long unit = 0;
+    for (const Block& bl : blocks) {
+      const int *g0 = g.klist.data() + g.kgroup[bl.group], *g1 = g.klist.data() + g.kgroup[bl.group + 1];
+      const GenPairRec& B = g.pairs[*g0];
+      f_chunks(B.nfP * B.nfQ, chunks);
+      for (const Bra& x : *bl.bras) {
+        const GenPairRec& A = g.pairs[x.a];
+        // two generic pairs: taken once, from the earlier position
+        const int* b = B.gen ? std::lower_bound(g0, g1, x.a) : g0;
+        const int cnt = (int)(std::lower_bound(b, g1, x.kets) - b);
+        if (cnt <= 0) continue;
+        const int L = A.lP + A.lQ + B.lP + B.lQ;
+        for (const auto& c : chunks) {
+          const int ng = std::max(1, std::min(32 / c.second, kFWarpDoubles / f_slot(L)));
+          fw.runs.push_back({x.a, (int)(b - g.klist.data()), cnt, c.first | c.second << 16,
+                             (unsigned)(bl.si | bl.sj << 8 | ng << 16)});
+          fw.first.push_back(unit);
+          unit += (long long)((cnt + ng - 1) / ng) * bl.si * bl.sj;
+        }
+      }
+    }
+    fw.units[q] = unit;
+    fw.seg[q + 1] = (int)fw.runs.size();
   }
 }
 
@@ -756,8 +766,8 @@ int gen_zero(const GenPath& g, cudaStream_t st) {
   return e == cudaSuccess ? SQB200_OK : set_error(SQB200_ECUDA, std::string("generic counters: ") + cudaGetErrorString(e));
 }
 
-int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FItem* d_fitems, const int fseg[6],
-               const GenBuild& b, const cudaStream_t* lanes, int nlanes) {
+int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FRun* d_fruns, const long long* d_ffirst,
+               const int fseg[6], const long long funits[5], const GenBuild& b, const cudaStream_t* lanes, int nlanes) {
   cudaError_t e = cudaSuccess;
   if (nitems > 0) {
     GenArgs a = make_args(g);
@@ -771,12 +781,19 @@ int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FItem
   for (int k = kNumFKernels - 1; k >= 0; --k) {      // the largest bras first
     const int q = kFKernels[k].q;
     int n = fseg[q + 1] - fseg[q];
-    if (n <= 0) continue;
-    const FItem* items = d_fitems + fseg[q];
-    void* args[] = {&f, &items, &n};
-    e = cudaLaunchKernel(kFKernels[k].fn, dim3((n + kFWarps - 1) / kFWarps), dim3(32 * kFWarps), args,
-                         kFWarps * kFWarpDoubles * sizeof(double), lanes[lane++ % nlanes]);
-    if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("f-shell kernel: ") + cudaGetErrorString(e));
+    const FRun* runs = d_fruns + fseg[q];
+    const long long* first = d_ffirst + fseg[q];
+    const cudaStream_t st = lanes[lane % nlanes];
+    if (n > 0) ++lane;
+    // (a grid holds 2^31 - 1 CTAs)
+    const long long most = (1ll << 30) * kFWarps;
+    long long nunits = funits[q];
+    for (long long u0 = 0; u0 < nunits; u0 += most) {
+      void* args[] = {&f, &runs, &first, &n, &u0, &nunits};
+      const unsigned grid = (unsigned)((std::min(most, nunits - u0) + kFWarps - 1) / kFWarps);
+      e = cudaLaunchKernel(kFKernels[k].fn, dim3(grid), dim3(32 * kFWarps), args, kFWarps * kFWarpDoubles * sizeof(double), st);
+      if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("f-shell kernel: ") + cudaGetErrorString(e));
+    }
   }
   return SQB200_OK;
 }

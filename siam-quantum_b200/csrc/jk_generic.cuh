@@ -48,13 +48,24 @@ struct GenItem {
   int bra, k0, cnt, er;
 };
 
-// A warp's unit of the f-shell kernels (gen_fshell_kernels.py): one bra pair and the cnt ket pairs
-// klist[k0 ..], g function pairs from c0 of each (cg = c0 | g << 16), one lane per function pair; of
-// the primitives the bra's gi, gi + si, ... and the ket's gj, gj + sj, ... (split = gi | gj << 8 |
-// si << 16 | sj << 24).
-struct FItem {
+// A run of the f-shell kernels' work (gen_fshell_kernels.py): one bra pair and the cnt ket pairs
+// klist[k0 ..] of one group, g function pairs from c0 of each (cg = c0 | g << 16).  A warp's unit is ng
+// of the kets, one lane per function pair, and one part of the primitives: the bra's gi, gi + si, ...
+// and the ket's gj, gj + sj, ... (split = si | sj << 8 | ng << 16).  The units of a run lie side by
+// side, kets outermost, then gi; the list holds each run's first unit beside it, and a warp finds
+// its run by its unit's number.
+struct FRun {
   int bra, k0, cnt, cg;
   unsigned split;
+};
+
+// The run list of one build: the runs of class q (0 s .. 4 f) are seg[q] .. seg[q + 1], their units
+// 0 .. units[q] - 1.
+struct FWork {
+  std::vector<FRun> runs;
+  std::vector<long long> first;     // per run, its first unit within its class
+  int seg[6] = {0, 0, 0, 0, 0, 0};
+  long long units[5] = {0, 0, 0, 0, 0};
 };
 
 // Shared memory of one warp of the f-shell kernels (doubles), and of one quartet of total order L:
@@ -128,17 +139,16 @@ void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* 
 int gen_upload(GenPath& g, cudaStream_t st);
 // Schwarz entries sqrt|(pq|pq)| of the generic pairs' functions into S (nbf x nbf, device).
 int gen_schwarz(const GenPath& g, int nbf, double* S, cudaStream_t st);
-// Work items of one build at these cutoffs: bras of the f-shell kernels to fitems (grouped by class,
-// fseg[q] .. fseg[q + 1]), the others to items.
+// Work of one build at these cutoffs: bras of the f-shell kernels to fw, the others to items.
 // er_run != nullptr (multipole mode): every bra to items; it takes error-bank slots for its kets
 // that pass the outer cutoff, numbered on from *er_run.
-void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, std::vector<FItem>& fitems,
-               int fseg[6], long long* er_run = nullptr);
+void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem>& items, FWork& fw,
+               long long* er_run = nullptr);
 // The launches over the items (counters zeroed first on lanes[0], which the other lanes must wait
 // for): the run-time kernel on lanes[0], the f-shell kernels over all lanes.
 int gen_zero(const GenPath& g, cudaStream_t st);
-int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FItem* d_fitems, const int fseg[6],
-               const GenBuild& b, const cudaStream_t* lanes, int nlanes);
+int gen_launch(const GenPath& g, const GenItem* d_items, int nitems, const FRun* d_fruns, const long long* d_ffirst,
+               const int fseg[6], const long long funits[5], const GenBuild& b, const cudaStream_t* lanes, int nlanes);
 void gen_free(GenPath& g);
 
 }  // namespace sqb

@@ -62,6 +62,32 @@ static __device__ double gen_boys(int n, double T, const double* __restrict__ ta
   return F;
 }
 
+// The unit of a warp: its bra, its kets klist[k0 .. k0 + cnt), its function pairs and its part of the
+// primitives.
+struct FUnit {
+  int bra, k0, cnt, cg, gi, gj, si, sj;
+};
+
+// Unit u of a class's runs (first[r] <= u < first[r + 1]; the last run ends with the class).  The
+// warp looks for the run together, 32 starts at a time: three rounds of loads for the 2e4 runs of
+// water/QZP.
+static __device__ __forceinline__ FUnit f_unit(const FRun* __restrict__ runs, const long long* __restrict__ first,
+                                               int nruns, long long u) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0;
+  for (int n = nruns; n > 1;) {            // the run is one of lo .. lo + n - 1
+    const int step = (n + 31) / 32, x = lane * step;
+    const int k = __popc(__ballot_sync(0xffffffffu, x < n && first[lo + x] <= u)) - 1;   // lane 0's start is not above u
+    lo += k * step;
+    n = min(step, n - k * step);
+  }
+  const FRun r = runs[lo];
+  const int si = r.split & 255, sj = (r.split >> 8) & 255, ng = r.split >> 16, parts = si * sj;
+  const long long at = u - first[lo];
+  const int kb = (int)(at / parts), part = (int)(at - (long long)kb * parts), gi = part / sj;
+  return {r.bra, r.k0 + kb * ng, min(ng, r.cnt - kb * ng), r.cg, gi, part - gi * sj, si, sj};
+}
+
 // The f-shell kernels' seeds base[n] = 2 pi^(5/2)/sqrt(p+q) (-2 alpha)^n F_n(T), n <= L, by the g
 // lanes of a quartet (cc = 0 .. g-1), each its own orders.
 static __device__ __forceinline__ void f_seeds(int L, double alpha, double rs, double X, double Y, double Z,

@@ -41,3 +41,27 @@ def test_f_kernels_match_oracle(name, restricted):
                 assert np.abs(KB - KB0).max() <= 1e-10 * scale
     finally:
         eng.close()
+
+
+@pytest.mark.gpu
+def test_first_build_with_f_shells_takes_little_longer_than_the_next():
+    """The first build of a context makes its work list: for benzene/QZP 7.7 million units of the f-shell
+    kernels, which the list must not hold or sort one by one (that took three builds' time)."""
+    import time
+    sqb = load_sqb200()
+
+    def times(atoms, builds):
+        b = sqb.basis.build_basis(sqb.molecules.to_bohr(atoms), "qzp")
+        P = 0.5 * np.eye(b.nbf)
+        eng = sqb.JKEngine(b)
+        out = []
+        for _ in range(builds):
+            t = time.perf_counter()
+            eng.build(P, scf_cutoff=1e-10)
+            out.append(time.perf_counter() - t)
+        eng.close()
+        return out
+
+    times(sqb.molecules.water(), 2)                     # the kernels' code is loaded
+    t = times(sqb.molecules.benzene(), 3)
+    assert t[0] <= 2.0 * min(t[1:]), t
