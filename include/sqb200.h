@@ -99,6 +99,11 @@ int sqb200_jk_build_noalloc(sqb200_jk *ctx, const double *dPA, const double *dPB
  * once that stream has finished.  (No reference counterpart: instrumentation.) */
 int sqb200_jk_stats(sqb200_jk *ctx, long long *out, int n);
 
+/* Builds of the context that replayed a graph the library captured of its own launches (small
+ * builds of a work list that was built before), of all its builds so far.  (Instrumentation,
+ * no reference counterpart.) */
+int sqb200_jk_replays(sqb200_jk *ctx, long long *n);
+
 /* Per-class timing: enable (1) or disable (0) CUDA-event timing of every class kernel
  * launch on the build's stream, clearing the accumulators.  (Instrumentation, no
  * reference counterpart.) */

@@ -436,6 +436,7 @@ struct sqb200_jk {
   std::vector<long long> last_counts;
   long long last_flops = 0;
   int last_launches = 0;        // kernels enqueued by the last build
+  long long replays = 0;        // builds that replayed a captured graph
   // side streams for concurrent class launches: the build forks them off its stream after the
   // prologue and joins them before k_finalize (SQB200_STREAMS, default 8; 0 = one stream)
   int nside = -1;
@@ -1645,6 +1646,7 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   if (graph) {
     c->last_launches = w->launches;
     CUDA_OK(cudaGraphLaunch(graph, st));
+    ++c->replays;
   } else {
     rc = launch_classes(c, w, uhf, outer, fixed, dscreen, st);
     if (rc) return rc;
@@ -1910,6 +1912,12 @@ int sqb200_jk_tiles(sqb200_jk* c, int* form, int n) {
     form[k] = (K.fn_rw || K.fn_rs) ? c->form[k] : -1;
   }
   return std::min(n, sqb::kNumClassKernels);
+}
+
+int sqb200_jk_replays(sqb200_jk* c, long long* n) {
+  if (!c || !n) return fail(SQB200_EINVAL, "null argument");
+  *n = c->replays;
+  return SQB200_OK;
 }
 
 int sqb200_jk_set_tiles(sqb200_jk* c, const int* form, int n) {

@@ -30,7 +30,7 @@ EXPORTS = ["sqb200_jk_create", "sqb200_jk_destroy", "sqb200_jk_build", "sqb200_j
            "sqb200_syev_batched", "sqb200_gradient", "sqb200_gradient_terms",
            "sqb200_segdots_create", "sqb200_segdots_run", "sqb200_segdots_destroy",
            "sqb200_jk_set_multipole", "sqb200_jk_set_persistent", "sqb200_batch_set_persistent",
-           "sqb200_boys_eval", "sqb200_last_error"]
+           "sqb200_boys_eval", "sqb200_jk_replays", "sqb200_last_error"]
 
 
 class SQB200Error(RuntimeError):
@@ -76,6 +76,7 @@ def load_library(path=LIB_PATH):
     L.sqb200_batch_autotune.argtypes = [vp, vp, vp, vp]
     L.sqb200_jk_autotune.argtypes = [vp, vp, vp, ctypes.c_int, ctypes.c_double, ctypes.c_double,
                                      ctypes.c_double, vp]
+    L.sqb200_jk_replays.argtypes = [vp, ctypes.POINTER(ctypes.c_longlong)]
     L.sqb200_jk_tiles.argtypes = [vp, _i32p, ctypes.c_int]
     L.sqb200_syev_batched.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, vp, vp, vp]
     L.sqb200_gradient.argtypes = [vp, ctypes.c_int, _f64p, _f64p, _f64p, _f64p, _f64p, _f64p]
@@ -203,6 +204,12 @@ class JKEngine:
         _check(_lib.sqb200_jk_stats(self._ctx, out, 6))
         return {"quartets": out[0], "prim_quartets": out[1], "flops": out[2], "shells": out[3],
                 "pairs": out[4], "launches": out[5]}
+
+    def replays(self):
+        """Builds so far that replayed the library's own captured graph of the build."""
+        n = ctypes.c_longlong()
+        _check(_lib.sqb200_jk_replays(self._ctx, ctypes.byref(n)))
+        return n.value
 
     def profile(self, enable=True):
         """Start (or stop) per-class CUDA-event timing of the class kernels."""

@@ -60,3 +60,89 @@ def test_replayed_builds_match_direct(case):
     ref, _ = _fresh(sqb, g, [d[0].cpu().numpy()] * 2, **kw)
     assert np.abs(out[0].cpu().numpy() - ref[0]).max() <= 1e-11 * max(1.0, np.abs(ref[0]).max())
     eng.close()
+
+
+class _Calls:
+    """Builds of one context on one stream, each against a fresh context's first build."""
+
+    def __init__(self, sqb, g, seed):
+        import torch
+        self.torch, self.sqb, self.g = torch, sqb, g
+        self.n = golden_basis(g).nbf
+        self.eng = sqb.JKEngine(golden_basis(g), schwarz=g["schwarz"])
+        self.st = torch.cuda.Stream()
+        rng = np.random.default_rng(seed)
+        self.P = [A + A.T for A in rng.standard_normal((2, self.n, self.n))]
+        self.d = [torch.tensor(p, dtype=torch.float64, device="cuda") for p in self.P]
+        self.out = [torch.empty((self.n, self.n), dtype=torch.float64, device="cuda") for _ in range(3)]
+        torch.cuda.synchronize()
+
+    def build(self, **kw):
+        self.eng.build_tensors(*self.d, *self.out, stream=self.st, scf_cutoff=1e-10, **kw)
+
+    def check(self, **kw):
+        self.st.synchronize()
+        ref, _ = _fresh(self.sqb, self.g, self.P, scf_cutoff=1e-10, **kw)
+        for x, y in zip(self.out, ref):
+            assert np.abs(x.cpu().numpy() - y).max() <= 1e-11 * max(1.0, np.abs(y).max())
+
+    def until_replayed(self, **kw):
+        """Builds until one is a replay; how many were direct."""
+        n0 = self.eng.replays()
+        for k in range(100):
+            self.build(**kw)
+            if self.eng.replays() > n0:
+                return k
+        raise AssertionError("no build of this work list was replayed")
+
+
+@pytest.mark.gpu
+def test_which_builds_are_replays():
+    import torch
+    sqb = load_sqb200()
+    c = _Calls(sqb, golden("h2co_631gs"), 9)
+    kw = dict(restricted=False)
+    assert c.until_replayed(**kw) >= 1          # a work list's first build launches directly
+    c.check(**kw)
+    for _ in range(3):                          # from then on every build is a replay
+        n = c.eng.replays()
+        c.build(**kw)
+        assert c.eng.replays() == n + 1
+    c.build(dscreen_rmax=0.0, **kw)             # the density screen is no part of the graph
+    assert c.eng.replays() == n + 2
+    c.check(dscreen_rmax=0.0, **kw)
+
+    def direct(**k):
+        n = c.eng.replays()
+        c.build(**k)
+        assert c.eng.replays() == n
+        c.check(**k)
+
+    direct(restricted=False, fixed_cutoff=1e-9)   # another work list
+    c.eng.set_tiles(np.full(256, 2, np.int32))    # other forms
+    direct(**kw)
+    c.until_replayed(**kw)
+    c.check(**kw)
+    c.eng.profile(True)
+    direct(**kw)
+    c.eng.profile(False)
+    c.eng.set_persistent(True)
+    direct(**kw)
+    c.eng.set_persistent(False)
+    n = c.eng.replays()
+    graph = torch.cuda.CUDAGraph()
+    c.st.synchronize()
+    with torch.cuda.graph(graph, stream=c.st):
+        c.build(**kw)
+    assert c.eng.replays() == n
+    for x in c.out:
+        x.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    c.check(**kw)
+    c.build(**kw)
+    assert c.eng.replays() == n + 1
+    c.check(**kw)
+    del graph
+    c.eng.close()
