@@ -100,7 +100,7 @@ int sqb200_jk_build_noalloc(sqb200_jk *ctx, const double *dPA, const double *dPB
 int sqb200_jk_stats(sqb200_jk *ctx, long long *out, int n);
 
 /* Builds of the context that replayed a graph the library captured of its own launches (small
- * builds of a work list that was built before), of all its builds so far.  (Instrumentation,
+ * builds of a work list that was built some twenty times before), of all its builds so far.  (Instrumentation,
  * no reference counterpart.) */
 int sqb200_jk_replays(sqb200_jk *ctx, long long *n);
 

@@ -423,8 +423,8 @@ struct sqb200_jk {
     double ops = 0.0;                   // emitted operations of a build (estimate)
     int launches = 0;                   // kernels of a build
     // captured launches per spin (build_graph); `seen`, `stamp`: the form_stamp of the last direct
-    // build and of the capture
-    struct Graph { cudaGraphExec_t exec = nullptr; int stamp = -1, seen = -1; bool failed = false; } graph[2];
+    // build and of the capture; `direct`: direct builds with these forms so far
+    struct Graph { cudaGraphExec_t exec = nullptr; int stamp = -1, seen = -1, direct = 0; bool failed = false; } graph[2];
   };
   // key: outer cutoff, fixed cutoff, FP32 threshold, multipole mode
   std::map<std::tuple<double, double, double, int>, Work> work;
@@ -1355,8 +1355,17 @@ int build_work(sqb200_jk* c, double outer, double fixed, sqb200_jk::Work** out) 
   return SQB200_OK;
 }
 
-// Builds of at most this many emitted operations replay a captured graph from their third pass on.
+// Builds of at most this many emitted operations replay a captured graph once a work list has been
+// built kGraphAfter times.  Capture, instantiation and the first launch of a graph take 0.39 ms (water
+// RHF/3-21G) to 0.65 ms (benzene/6-31G*) on B200, what 17 to 30 replays save: an SCF of a dozen builds
+// must not pay for it (captured on the second build, that build took 0.43 instead of 0.07 ms for
+// water, 0.82 instead of 0.24 for a radical of 3 heavy atoms, 1.2 instead of 0.60 for benzene), and a long
+// run of builds gives away about what the capture costs.  us per build replayed / direct, each waited
+// for: water 45 / 68, the radical 201 / 232, benzene 569 / 590, an organic of 4 heavy atoms in DZP 607 / 645;
+// many in a row: 35 / 57, 187 / 209, 555 / 562, 594 / 614, of 9 heavy atoms in 6-31G* 1138 / 1146, of 11
+// (4e10 operations) 2171 / 2156.
 constexpr double kGraphOps = 2e10;
+constexpr int kGraphAfter = 24;
 
 // Profile and class-name index of the generic path's kernel (after the FP64 and FP32 forms).
 const int kGenericKernel = 2 * sqb::kNumClassKernels;
@@ -1589,11 +1598,10 @@ int launch_classes(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double outer, doub
 }
 
 // The captured graph of launch_classes for this work list and spin, or null.  A small molecule's
-// build is a few microseconds of kernels behind some forty stream calls; they are captured once, on
-// the second build of a work list, and replayed as one launch (water RHF/3-21G on B200: 43 us per
-// build with single launches, 32.5 with the graph; a radical of 3 heavy atoms 211 and 183).  Everything the captured
-// launches are given is the context's own and stays for its life: density copies, accumulators, the
-// molecule record that carries the cutoffs, the work list.  The graph is made anew when a form
+// build is a few microseconds of kernels behind some forty stream calls; they are captured once, after
+// kGraphAfter builds of a work list, and replayed as one launch.  Everything the captured launches are
+// given is the context's own and stays for its life: density copies, accumulators, the molecule
+// record that carries the cutoffs, the work list.  The graph is made anew when a form
 // was tuned or set since; profiled, persistent and multipole builds, builds with the generic path
 // (whose launches carry cutoffs) and builds inside a caller's capture launch directly.
 cudaGraphExec_t build_graph(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double outer, double fixed, double dscreen,
@@ -1603,8 +1611,12 @@ cudaGraphExec_t build_graph(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double ou
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
   if (g.exec && g.stamp == c->form_stamp) return g.exec;
-  if (g.seen != c->form_stamp) {             // the first build with these forms launches directly
+  if (g.seen != c->form_stamp) {
     g.seen = c->form_stamp;
+    g.direct = 0;
+  }
+  if (g.direct < kGraphAfter) {
+    ++g.direct;
     return nullptr;
   }
   if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
