@@ -390,6 +390,10 @@ struct sqb200_jk {
   void* d_pairbase = nullptr;   // one allocation holding the pair classes' device arrays
   void* d_grad = nullptr;       // workspace of the gradient, as large as its largest call so far
   size_t grad_bytes = 0;
+  // Gradients of one context may be asked for by several threads, and beside a build: the workspace
+  // is one call's at a time (grad_mu, over the whole call), the side streams and their events one
+  // enqueue's (lanes_mu; taken after grad_mu).
+  std::mutex grad_mu, lanes_mu;
   size_t pairbase_bytes = 0;
   double* d_boys = nullptr;   // plain Boys table (gradient)
   double* d_boysr = nullptr;  // row table of boys<M>
@@ -1620,13 +1624,19 @@ cudaGraphExec_t build_graph(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double ou
     return nullptr;
   }
   if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+  // on a stream of its own: other threads' calls on this context enqueue on c->stream
   cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+  cudaStream_t cap = nullptr;
+  cudaEvent_t cap_ev = nullptr;
+  cudaError_t e = side_take(c->device, &cap, &cap_ev);
+  const bool have = e == cudaSuccess;
+  if (have) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    const int rc = launch_classes(c, w, uhf, outer, fixed, dscreen, c->stream);
-    e = cudaStreamEndCapture(c->stream, &graph);
+    const int rc = launch_classes(c, w, uhf, outer, fixed, dscreen, cap);
+    e = cudaStreamEndCapture(cap, &graph);
     if (rc && e == cudaSuccess) e = cudaErrorUnknown;
   }
+  if (have) side_give(c->device, cap, cap_ev);
   if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   if (e != cudaSuccess) {                    // the direct launches serve
@@ -1645,6 +1655,7 @@ int launch_build(sqb200_jk* c, const double* dPA, const double* dPB, int restric
   const int uhf = restricted ? 0 : 1;
   if (!restricted && dPB == nullptr) return fail(SQB200_EINVAL, "unrestricted build needs PB");
   if (dPB == nullptr) dPB = dPA;
+  std::lock_guard<std::mutex> lock(c->lanes_mu);
   sqb200_jk::Work* w = nullptr;
   int rc = build_work(c, outer, fixed, &w);
   if (rc) return rc;
@@ -3464,6 +3475,7 @@ void grad_work(const sqb200_jk* c, const int* fat, const double* PT, double scre
 // The class kernels on the context's streams (forked off c->stream and joined to it, as a
 // build's), each with its CTAs' bra records in at most 32 KB of shared memory at a time.
 int grad_launch(sqb200_jk* c, const GradWork& w, sqb::GradArgs a) {
+  std::lock_guard<std::mutex> lock(c->lanes_mu);
   int rc = ensure_side_streams(c, w.segs.size());
   if (rc) return rc;
   const int nl = lanes_for(c, w.segs.size());
@@ -3636,6 +3648,7 @@ extern "C" int sqb200_gradient_terms(sqb200_jk* c, int natom, const double* Z, c
   up.put(&gw.d_items, gw.items.size() * sizeof(sqb::WorkItem), gw.items.data());
   up.put(&dg, 3 * natom * sizeof(double), nullptr);
   up.put(&dcopies, (size_t)kGradCopies * gstride * sizeof(double), nullptr);
+  std::lock_guard<std::mutex> lock(c->grad_mu);
   // the workspace stays with the context: a cudaMalloc and a cudaFree of some megabytes in every call
   // took 0.4 ms, and the free synchronised the device
   cudaError_t e = up.upload_kept(&c->d_grad, &c->grad_bytes, c->stream);

@@ -79,3 +79,57 @@ def test_class_gradient_keeps_an_infinite_density_factor_of_either_sign(sign):
     G = eng.gradient(np.ones(4), xyz, P[0], P[1], P[1], terms=8)
     eng.close()
     assert not np.isfinite(G[2:]).all(axis=1).any()
+
+
+@pytest.mark.gpu
+def test_gradients_of_one_context_from_several_threads_beside_its_builds():
+    """Two threads ask one context for gradients of densities of their own (one with a quarter of the
+    pairs screened out, so that the calls' sizes differ) while a third builds with it, past the
+    number of builds that makes a replay graph; each against its own call alone."""
+    import threading
+
+    import torch
+    sqb = load_sqb200()
+    atoms = sqb.molecules.to_bohr(sqb.molecules.random_organic(np.random.default_rng(3), 4))
+    b = sqb.basis.build_basis(atoms, "6-31g*")
+    n = b.nbf
+    Z = np.array([a[0] for a in atoms], dtype=np.float64)
+    xyz = np.array([a[1:] for a in atoms])
+    rng = np.random.default_rng(4)
+    P = [0.1 * (A + A.T) for A in rng.standard_normal((3, n, n))]
+    P[1][:n // 2, :n // 2] = 0.0
+    eng = sqb.JKEngine(b)
+    ref = [eng.gradient(Z, xyz, p, p, P[2]) for p in P[:2]]
+    st = torch.cuda.Stream()
+    d = torch.tensor(P[2], device="cuda")
+    out = [torch.empty((n, n), dtype=torch.float64, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    eng.build_tensors(d, d, *out, scf_cutoff=1e-10, stream=st)
+    st.synchronize()
+    J, K = out[0].clone(), out[1].clone()
+    torch.cuda.synchronize()
+    bad = []
+
+    def gradients(k):
+        for _ in range(25):
+            err = np.abs(eng.gradient(Z, xyz, P[k], P[k], P[2]) - ref[k]).max()
+            if not err <= 1e-11 * np.abs(ref[k]).max():
+                bad.append(("gradient", k, err))
+
+    def builds():
+        for k in range(60):
+            eng.build_tensors(d, d, *out, scf_cutoff=1e-10, stream=st)
+            if k % 10 == 9:
+                st.synchronize()
+                err = max((out[0] - J).abs().max().item(), (out[1] - K).abs().max().item())
+                if not err <= 1e-11 * J.abs().max().item():
+                    bad.append(("build", k, err))
+
+    ts = [threading.Thread(target=gradients, args=(k,)) for k in (0, 1)] + [threading.Thread(target=builds)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad
+    assert eng.replays() > 0
+    eng.close()
