@@ -195,31 +195,58 @@ const BoysTables& boys_tables() {
 
 // The tables on the device: static arrays of about 0.6 MB, filled when the first context of a device
 // is created and read by all of them (a copy in every context's own allocation took a small
-// molecule's context past the size the driver carves from a pool: 1.6 -> 3.8 ms to create).
+// molecule's context past the size the driver carves from a pool: 1.6 -> 3.8 ms to create).  A
+// cudaDeviceReset of the host program takes them, and every stream, event and function attribute,
+// with the CUDA context: g_boys_ready lies beside the tables, so it goes with them.
 constexpr int kBoysPlain = BOYS_NGRID * BOYS_NCOL;
 constexpr int kBoysRows = (BOYS_MMAX + 2) * BOYS_NGRID * BOYS_ROW;
 constexpr int kBoysRowsF = (BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF;
 __device__ __align__(128) double g_boys_plain[kBoysPlain];
 __device__ __align__(128) double g_boys_rows[kBoysRows];
 __device__ __align__(128) float g_boys_rowsf[kBoysRowsF];
+__device__ int g_boys_ready;
 
-// Addresses of the tables on the current device, filled on first use.
+// Per device, the number of times its tables were filled (device_epoch).
+struct Epochs {
+  std::mutex mu;
+  std::map<int, int> at;
+};
+Epochs& epochs() {
+  static Epochs* e = new Epochs;          // never destroyed: contexts may outlive static objects
+  return *e;
+}
+
+}  // namespace
+
+int sqb::device_epoch(int dev) {
+  Epochs& e = epochs();
+  std::lock_guard<std::mutex> lock(e.mu);
+  return e.at[dev];
+}
+
+namespace {
+
+// Addresses of the tables on the current device, filled on first use and after a reset.
 cudaError_t boys_device(double** plain, double** rows, float** rowsf, cudaStream_t st) {
-  static std::mutex mu;
-  static std::set<int> filled;
-  int dev = 0;
+  int dev = 0, ready = 0, *d_ready = nullptr;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)plain, g_boys_plain);
   if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)rows, g_boys_rows);
   if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)rowsf, g_boys_rowsf);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress((void**)&d_ready, g_boys_ready);
   if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lock(mu);
-  if (filled.count(dev)) return cudaSuccess;
+  Epochs& ep = epochs();
+  std::lock_guard<std::mutex> lock(ep.mu);
+  e = cudaMemcpyAsync(&ready, d_ready, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess || ready) return e;
+  ++ep.at[dev];
   const BoysTables& bt = boys_tables();
   e = h2d(*plain, bt.plain.data(), bt.plain.size() * sizeof(double), st);
   if (e == cudaSuccess) e = h2d(*rows, bt.rows.data(), bt.rows.size() * sizeof(double), st);
   if (e == cudaSuccess) e = h2d(*rowsf, bt.rowsf.data(), bt.rowsf.size() * sizeof(float), st);
-  if (e == cudaSuccess) filled.insert(dev);
+  ready = 1;
+  if (e == cudaSuccess) e = h2d(d_ready, &ready, sizeof(int), st);
   return e;
 }
 
@@ -380,7 +407,7 @@ int set_error(int code, const std::string& msg) { return fail(code, msg); }
 }  // namespace sqb
 
 struct sqb200_jk {
-  int device = 0;
+  int device = 0, epoch = 0;     // epoch: the device's device_epoch at creation
   int nbf = 0, ns = 0;
   std::vector<Shell> shells;
   std::vector<double> schwarz;   // basis level, nbf*nbf
@@ -1011,12 +1038,12 @@ int cta_threads(double ops) {
 // kernels side by side on an SM share its instruction cache).
 constexpr int kSideStreams = 8;
 
-// Side streams and their join events, per device.  A context or batch takes the ones it needs and gives
-// them back, idle, when it is destroyed; at most kSidePool stay for the next (creating and destroying
-// eight takes over a millisecond of a short SCF job's set-up and end).
+// Side streams and their join events, per device and device epoch.  A context or batch takes the ones
+// it needs and gives them back, idle, when it is destroyed; at most kSidePool stay for the next
+// (creating and destroying eight takes over a millisecond of a short SCF job's set-up and end).
 struct SidePool {
   std::mutex mu;
-  std::map<int, std::vector<std::pair<cudaStream_t, cudaEvent_t>>> idle;
+  std::map<std::pair<int, int>, std::vector<std::pair<cudaStream_t, cudaEvent_t>>> idle;
 };
 constexpr size_t kSidePool = 64;
 SidePool& side_pool() {
@@ -1024,11 +1051,11 @@ SidePool& side_pool() {
   return *p;
 }
 
-cudaError_t side_take(int device, cudaStream_t* s, cudaEvent_t* ev) {
+cudaError_t side_take(int device, int epoch, cudaStream_t* s, cudaEvent_t* ev) {
   SidePool& p = side_pool();
   {
     std::lock_guard<std::mutex> lock(p.mu);
-    auto& v = p.idle[device];
+    auto& v = p.idle[{device, epoch}];
     if (!v.empty()) {
       *s = v.back().first;
       *ev = v.back().second;
@@ -1044,11 +1071,11 @@ cudaError_t side_take(int device, cudaStream_t* s, cudaEvent_t* ev) {
 }
 
 // The stream's work is waited for; a stream in error is destroyed.
-void side_give(int device, cudaStream_t s, cudaEvent_t ev) {
+void side_give(int device, int epoch, cudaStream_t s, cudaEvent_t ev) {
   SidePool& p = side_pool();
   if (cudaStreamSynchronize(s) == cudaSuccess) {
     std::lock_guard<std::mutex> lock(p.mu);
-    auto& v = p.idle[device];
+    auto& v = p.idle[{device, epoch}];
     if (v.size() < kSidePool) {
       v.push_back({s, ev});
       return;
@@ -1068,7 +1095,7 @@ int ensure_side_streams(sqb200_jk* c, size_t launches) {
   while (c->side.size() < (size_t)c->nside && c->side.size() + 1 < launches) {
     cudaStream_t s;
     cudaEvent_t e;
-    CUDA_OK(side_take(c->device, &s, &e));
+    CUDA_OK(side_take(c->device, c->epoch, &s, &e));
     c->side.push_back(s);
     c->ev_join.push_back(e);
   }
@@ -1410,11 +1437,12 @@ int pick_form(const sqb::ClassKernel& K, bool f32, int uhf, int form, const void
 int ensure_smem(const void* fn, size_t smem) {
   if (smem <= 48 * 1024) return SQB200_OK;
   static std::mutex mu;
-  static std::map<std::pair<int, const void*>, size_t> done;
+  static std::map<std::tuple<int, int, const void*>, size_t> done;
   int dev = 0;
   CUDA_OK(cudaGetDevice(&dev));
+  const int epoch = sqb::device_epoch(dev);
   std::lock_guard<std::mutex> lock(mu);
-  size_t& have = done[{dev, fn}];
+  size_t& have = done[{dev, epoch, fn}];
   if (have >= smem) return SQB200_OK;
   CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   have = smem;
@@ -1628,7 +1656,7 @@ cudaGraphExec_t build_graph(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double ou
   cudaGraph_t graph = nullptr;
   cudaStream_t cap = nullptr;
   cudaEvent_t cap_ev = nullptr;
-  cudaError_t e = side_take(c->device, &cap, &cap_ev);
+  cudaError_t e = side_take(c->device, c->epoch, &cap, &cap_ev);
   const bool have = e == cudaSuccess;
   if (have) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
@@ -1636,7 +1664,7 @@ cudaGraphExec_t build_graph(sqb200_jk* c, sqb200_jk::Work* w, int uhf, double ou
     e = cudaStreamEndCapture(cap, &graph);
     if (rc && e == cudaSuccess) e = cudaErrorUnknown;
   }
-  if (have) side_give(c->device, cap, cap_ev);
+  if (have) side_give(c->device, c->epoch, cap, cap_ev);
   if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   if (e != cudaSuccess) {                    // the direct launches serve
@@ -1822,6 +1850,10 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   int rc = build_shells(nbf, nprim, lmn, xyz, exps, ncoefs, c->shells);
   if (rc) { delete c; return rc; }
   c->ns = (int)c->shells.size();
+  cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = boys_device(&c->d_boys, &c->d_boysr, &c->d_boysf, c->stream);
+  if (e != cudaSuccess) { sqb200_jk_destroy(c); return fail(SQB200_ECUDA, cudaGetErrorString(e)); }
+  c->epoch = sqb::device_epoch(device);
   if (schwarz) c->schwarz.assign(schwarz, schwarz + (size_t)nbf * nbf);
   else c->schwarz.assign((size_t)nbf * nbf, 1.0);   // placeholder until the device pass below
   build_pairs(c);
@@ -1840,14 +1872,12 @@ int sqb200_jk_create(sqb200_jk** out, int nbf, const int* nprim, const int* lmn,
   cv.add(&c->d_counters, 8 * sqb::kNumClassKernels * sizeof(unsigned long long));
   cv.add(&c->d_queue, 2 * sqb::kNumClassKernels * sizeof(unsigned long long));
   cv.add(&c->d_mol, sizeof(sqb::MolRec));
-  cudaError_t e = cv.alloc(&c->d_base);
+  e = cv.alloc(&c->d_base);
   if (e != cudaSuccess) {
     sqb200_jk_destroy(c);
     return fail(SQB200_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
-  e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = boys_device(&c->d_boys, &c->d_boysr, &c->d_boysf, c->stream);
-  if (e == cudaSuccess) e = h2d(c->d_shfirst, fst.data(), c->ns * sizeof(int), c->stream);
+  e = h2d(c->d_shfirst, fst.data(), c->ns * sizeof(int), c->stream);
   if (e == cudaSuccess) e = h2d(c->d_shn, nf.data(), c->ns * sizeof(int), c->stream);
   if (e != cudaSuccess) { sqb200_jk_destroy(c); return fail(SQB200_ECUDA, cudaGetErrorString(e)); }
   if (!schwarz) {
@@ -1872,7 +1902,7 @@ int sqb200_jk_destroy(sqb200_jk* c) {
   if (!c) return SQB200_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (size_t i = 0; i < c->side.size(); ++i) side_give(c->device, c->side[i], c->ev_join[i]);
+  for (size_t i = 0; i < c->side.size(); ++i) side_give(c->device, c->epoch, c->side[i], c->ev_join[i]);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   for (auto& kv : c->work)
     for (auto& g : kv.second.graph)
@@ -2414,7 +2444,7 @@ extern "C" int sqb200_oneint(sqb200_jk* c, int natom, const double* Z, const dou
 // each work item names its molecule, whose MolRec gives the matrix offsets and cutoffs.
 
 struct sqb200_batch {
-  int device = 0, nmol = 0;
+  int device = 0, epoch = 0, nmol = 0;
   std::vector<sqb200_jk*> mols;
   std::vector<long long> moff, pmoff;   // nmol + 1 entries
   std::vector<int> shoff;               // nmol + 1 entries
@@ -2494,7 +2524,7 @@ __global__ void k_finalize_batch(const double* __restrict__ J, const double* __r
 }
 
 void free_batch(sqb200_batch* b) {
-  for (size_t i = 0; i < b->side.size(); ++i) side_give(b->device, b->side[i], b->ev_join[i]);
+  for (size_t i = 0; i < b->side.size(); ++i) side_give(b->device, b->epoch, b->side[i], b->ev_join[i]);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
   if (b->stream) { cudaStreamSynchronize(b->stream); cudaStreamDestroy(b->stream); }
@@ -2518,6 +2548,7 @@ extern "C" int sqb200_batch_create(sqb200_batch** out, int nmol, sqb200_jk* cons
   }
   sqb200_batch* b = new sqb200_batch();
   b->device = mols[0]->device;
+  b->epoch = mols[0]->epoch;
   b->nmol = nmol;
   b->mols.assign(mols, mols + nmol);
   b->moff.assign(nmol + 1, 0);
@@ -2774,7 +2805,7 @@ extern "C" int sqb200_batch_build_device(sqb200_batch* b, const double* dPA, con
     for (int i = 0; i < n; ++i) {
       cudaStream_t s;
       cudaEvent_t e;
-      CUDA_OK(side_take(b->device, &s, &e));
+      CUDA_OK(side_take(b->device, b->epoch, &s, &e));
       b->side.push_back(s);
       b->ev_join.push_back(e);
     }

@@ -594,18 +594,19 @@ void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* 
 }
 
 int gen_upload(GenPath& g, cudaStream_t st) {
-  // the f-shell kernels' shared memory is above the default limit: raised once per device
+  // the f-shell kernels' shared memory is above the default limit: raised once per device context
   {
     static std::mutex mu;
-    static std::set<int> done;
+    static std::set<std::pair<int, int>> done;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
+    const std::pair<int, int> at{dev, device_epoch(dev)};
     std::lock_guard<std::mutex> lock(mu);
-    if (e == cudaSuccess && !done.count(dev)) {
+    if (e == cudaSuccess && !done.count(at)) {
       for (int k = 0; k < kNumFKernels && e == cudaSuccess; ++k)
         e = cudaFuncSetAttribute(kFKernels[k].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kFWarps * kFWarpDoubles * (int)sizeof(double));
-      if (e == cudaSuccess) done.insert(dev);
+      if (e == cudaSuccess) done.insert(at);
     }
     if (e != cudaSuccess) return set_error(SQB200_ECUDA, std::string("f-shell kernels: ") + cudaGetErrorString(e));
   }

@@ -133,6 +133,11 @@ struct FKernel {
 extern const FKernel kFKernels[];
 extern const int kNumFKernels;
 
+// The number of CUDA contexts that the library has met on the device in this process, as of the
+// last sqb200_jk_create: it grows when the host program has reset the device, which ends streams,
+// events and function attributes (jk_engine.cu).
+int device_epoch(int dev);
+
 // Pair records and primitive data for every shell pair; `schwarz` is the basis-level matrix.
 void gen_build_pairs(GenPath& g, const std::vector<GenShell>& sh, const double* schwarz, int nbf);
 // Device copies of the pair data and the generic Boys table.
