@@ -2783,7 +2783,9 @@ extern "C" int sqb200_batch_autotune(sqb200_batch* b, const double* dPA, const d
     }
     for (int f = 0; f < 3; ++f) tf[3 * v + f] += ts[f];
   }
-  for (int k = 0; k < sqb::kNumClassKernels; ++k) b->form[k] = (signed char)pick_tuned(sqb::kClassKernels[k], &tf[3 * k]);
+  // (classes without work in this step keep what they have: a later step may bring them in)
+  for (int v : b->kernel)
+    if (v < sqb::kNumClassKernels) b->form[v] = (signed char)pick_tuned(sqb::kClassKernels[v], &tf[3 * v]);
   CUDA_OK(cudaStreamSynchronize(st));
   return SQB200_OK;
 }

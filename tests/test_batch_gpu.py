@@ -140,6 +140,26 @@ def test_set_step_waits_for_the_build_in_flight(captured):
 
 
 @pytest.mark.gpu
+def test_autotune_leaves_classes_without_work_at_their_default():
+    """The operations a batch counts follow its classes' forms: after an autotune of a step in which
+    no quartet survives, a full step runs the forms of a batch that was never tuned."""
+    import torch
+    flops = []
+    for tune in (False, True):
+        sqb, gs, engs, batch, PA, PB = _setup(["benzene_631gs", "h2co_631gs"])
+        if tune:
+            batch.set_step([True, True], 1e6, 1e6, float("inf"))
+            batch.autotune(PA.data_ptr(), PB.data_ptr())
+        batch.set_step([True, True], 1e-10, 1e-10, float("inf"))
+        out = _outs(batch)
+        batch.build_device(PA.data_ptr(), PB.data_ptr(), *(x.data_ptr() for x in out))
+        torch.cuda.synchronize()
+        flops.append(batch.stats()["flops"])
+        batch.close()
+    assert flops[0] == flops[1] > 0
+
+
+@pytest.mark.gpu
 def test_single_context_autotune_keeps_results():
     import torch
     sqb = load_sqb200()
