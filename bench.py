@@ -682,6 +682,7 @@ def run_ours(args, sqb):
         step()
     torch.cuda.synchronize(dev)
     prof = eng.profile_read()
+    ran = eng.ran_tiles()
     eng.profile(False)
     # keep the clock sampler on the same load for at least ~1 s
     tail_end = time.perf_counter() + (0.0 if args.profile_run else max(0.0, 1.0 - t_dev))
@@ -719,7 +720,7 @@ def run_ours(args, sqb):
     peak = fp32_peak if dom32 else fp64_peak
     # (the f-shell kernels, one row for all of them, count the operations they execute)
     dom_name = "jkf_F*" if dom["class"].startswith("generic") else "jk_" + dom["class"].replace(" f32", "").replace("|", "_") + (
-        "_R_f32" if dom32 else {1: "_R_w", 2: "_R_s"}.get(int(tiles[dom["index"]]) if dom["index"] < len(tiles) else 0, "_R"))
+        "_R_f32" if dom32 else {1: "_R_w", 2: "_R_s"}.get(int(ran[dom["index"]]) if dom["index"] < len(ran) else 0, "_R"))
     roof = {"bound": "fp32" if dom32 else "fp64",
             "kernel": dom_name,
             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,

@@ -166,6 +166,11 @@ int sqb200_jk_autotune(sqb200_jk *ctx, const double *dPA, const double *dPB, int
 int sqb200_jk_tiles(sqb200_jk *ctx, int *form, int n);
 int sqb200_jk_set_tiles(sqb200_jk *ctx, const int *form, int n);
 
+/* The FP64 form (0, 1 or 2) each class ran in the context's last build that launched it, its
+ * default resolved; 0 for a class no build has launched.  Returns the number of entries written
+ * (at most n). */
+int sqb200_jk_ran_tiles(sqb200_jk *ctx, int *form, int n);
+
 /* One-electron integrals of the context's basis on its device: overlap S, kinetic T and
  * nuclear attraction V = -sum_C Z_C <p|1/|r-C||q> for natom point charges Z at axyz (bohr),
  * each written to a host nbf*nbf array (the matrices the reference's uhf() builds with

@@ -1967,6 +1967,12 @@ int sqb200_jk_tiles(sqb200_jk* c, int* form, int n) {
   return std::min(n, sqb::kNumClassKernels);
 }
 
+int sqb200_jk_ran_tiles(sqb200_jk* c, int* form, int n) {
+  if (!c || !form) return fail(SQB200_EINVAL, "null argument");
+  for (int k = 0; k < n && k < sqb::kNumClassKernels; ++k) form[k] = c->ran_form[k];
+  return std::min(n, sqb::kNumClassKernels);
+}
+
 int sqb200_jk_replays(sqb200_jk* c, long long* n) {
   if (!c || !n) return fail(SQB200_EINVAL, "null argument");
   *n = c->replays;

@@ -30,7 +30,8 @@ EXPORTS = ["sqb200_jk_create", "sqb200_jk_destroy", "sqb200_jk_build", "sqb200_j
            "sqb200_syev_batched", "sqb200_gradient", "sqb200_gradient_terms",
            "sqb200_segdots_create", "sqb200_segdots_run", "sqb200_segdots_destroy",
            "sqb200_jk_set_multipole", "sqb200_jk_set_persistent", "sqb200_batch_set_persistent",
-           "sqb200_boys_eval", "sqb200_jk_replays", "sqb200_last_error"]
+           "sqb200_boys_eval", "sqb200_jk_replays", "sqb200_jk_ran_tiles",
+           "sqb200_last_error"]
 
 
 class SQB200Error(RuntimeError):
@@ -76,6 +77,7 @@ def load_library(path=LIB_PATH):
     L.sqb200_batch_autotune.argtypes = [vp, vp, vp, vp]
     L.sqb200_jk_autotune.argtypes = [vp, vp, vp, ctypes.c_int, ctypes.c_double, ctypes.c_double,
                                      ctypes.c_double, vp]
+    L.sqb200_jk_ran_tiles.argtypes = [vp, _i32p, ctypes.c_int]
     L.sqb200_jk_replays.argtypes = [vp, ctypes.POINTER(ctypes.c_longlong)]
     L.sqb200_jk_tiles.argtypes = [vp, _i32p, ctypes.c_int]
     L.sqb200_syev_batched.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, vp, vp, vp]
@@ -190,6 +192,14 @@ class JKEngine:
         (-1: its default form, neither tuned nor set; also a class with one form)."""
         out = np.zeros(256, np.int32)
         n = _lib.sqb200_jk_tiles(self._ctx, out, len(out))
+        if n < 0:
+            _check(n)
+        return out[:n].copy()
+
+    def ran_tiles(self):
+        """Per class kernel: the FP64 form (0, 1 or 2) it ran last, its default resolved."""
+        out = np.zeros(256, np.int32)
+        n = _lib.sqb200_jk_ran_tiles(self._ctx, out, len(out))
         if n < 0:
             _check(n)
         return out[:n].copy()

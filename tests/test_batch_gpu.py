@@ -186,6 +186,20 @@ def test_single_context_autotune_keeps_results():
 
 
 @pytest.mark.gpu
+def test_ran_tiles_resolve_the_default():
+    sqb = load_sqb200()
+    g = golden("h2co_631gs")
+    eng = sqb.JKEngine(golden_basis(g), schwarz=g["schwarz"])
+    eng.build(g["PA"])
+    ran = eng.ran_tiles()
+    assert (eng.tiles() == -1).all() and ran.min() >= 0 and (ran > 0).any()
+    eng.set_tiles(np.zeros(len(ran), np.int32))
+    eng.build(g["PA"])
+    assert (eng.ran_tiles() == 0).all()
+    eng.close()
+
+
+@pytest.mark.gpu
 def test_batched_scf_reaches_reference_energies():
     sqb = load_sqb200()
     gs = [golden(c) for c in GOLDEN_CASES]
