@@ -463,7 +463,7 @@ const ClassKernel kClassKernels[55] = {
    594,
    1, (const void*)jk_PP_DS_R_w, (const void*)jk_PP_DS_U_w, 594, 396, 702,
    2, (const void*)jk_PP_DS_R_s, (const void*)jk_PP_DS_U_s, 945, 378, 728,
-   0},
+   1},
   {5, 5, 9, 9, 33, 33, 4, 3, (const void*)jk_PP_PP_R, (const void*)jk_PP_PP_U, 1120, 594, 1062,
    2, (const void*)jk_PP_PP_R_f32, (const void*)jk_PP_PP_U_f32, 977, 594, 1044,
    834,

@@ -81,22 +81,27 @@ REG_CAP = {"jk_LL_LS_R_w": 128, "jk_LS_LS_R_s": 128}
 
 
 # The FP64 form a class runs without autotuning: 0 narrow, 1 wide, 2 swapped.  Measured on B200
-# (us per launch, narrow / wide / swapped):
-#   an organic of 14 heavy atoms, 6-31G*: DL|LL 538 / 345 / 354, LL|LL 268 / 225 / 215, DL|DL 290 / 203 / 290,
-#   DL|LS 254 / 190 / 236, LL|LS 244 / 212 / 179, LS|SS 159 / 160 / 127, LS|LS 170 / 171 / 124, SS|SS 142 / 142 /
-#   102, DS|LS 144 / 144 / 104, DL|DS 165 / 117 / 179, LL|DS 147 / 122 / 147, DD|LS 90 / 91 / 133;
-#   of 10 heavy atoms, DZP: DP|PP 471 / 305 / 359, DP|PS 363 / 238 / 293, DP|DP 220 / 167 / 196, DP|DS 226 / 142 /
-#   216, PP|PS 352 / 352 / 315, PS|SS 374 / 377 / 323, DP|SS 143 / 143 / 215; C60/6-31G LL|LL 60 / 39 / 45 ms.
-# So: bras of at least 18 functions wide (narrow where they have no wide form), the others swapped
-# on s-type kets, wide otherwise.
+# (us per launch, narrow / wide / swapped, equal where a class has no wide form):
+#   an organic of 14 heavy atoms, 6-31G*: DL|LL 471 / 312 / 346, LL|LL 228 / 175 / 184, DL|DL 248 / 186 / 247,
+#   DL|LS 241 / 173 / 222, LL|LS 227 / 182 / 188, LS|SS 111 / 111 / 81, LS|LS 111 / 112 / 94, SS|SS 68 / 67 / 51,
+#   DS|LS 93 / 93 / 86, LL|SS 100 / 101 / 82, DS|SS 70 / 70 / 52, DL|DS 144 / 105 / 170, LL|DS 123 / 108 / 141,
+#   DL|SS 82 / 83 / 72, DS|DS 57 / 67 / 54, DD|LS 81 / 83 / 138, DD|SS 58 / 58 / 82;
+#   of 10 heavy atoms, DZP: DP|PP 397 / 238 / 281, DP|PS 318 / 213 / 291, DP|DP 203 / 175 / 206, DP|DS 197 / 133 /
+#   221, PP|PS 352 / 352 / 321, PS|SS 367 / 367 / 308, PS|PS 362 / 362 / 280, PP|SS 161 / 162 / 145, DP|SS 101 /
+#   101 / 104, PP|PP 200 / 156 / 173, PP|DS 174 / 164 / 226, DS|DS 74 / 73 / 71; C60/6-31G LL|LL 60 / 39 / 45 ms,
+#   LL|LS with its register cap 16 ms wide.
+# So: bras of at least 18 functions (DL, DP, DD) take the wide form, narrow where they have none
+# (their swapped flush is large), but for DL|SS, swapped; smaller bras take the swapped form on SS, PS
+# and LS kets (LL|LS: within 3% of wide), and on the others the wide one, narrow where they have
+# none; but for DS|DS, whose second pass gains nothing, narrow.
 def default_form(bra, ket, has_wide, has_swap):
     if bra in ("DL", "DP", "DD"):
         if (bra, ket) == ("DL", "SS"):
             return 2
         return 1 if has_wide else 0
-    if ket[1] == "S" and ket != "DS" and has_swap:
+    if ket in ("SS", "PS", "LS") and has_swap:
         return 2
-    if (bra, ket) in (("DS", "DS"), ("PP", "DS")):
+    if (bra, ket) == ("DS", "DS"):
         return 0
     return 1 if has_wide else 0
 
