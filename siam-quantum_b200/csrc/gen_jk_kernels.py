@@ -727,6 +727,11 @@ def emit_multipole(em, blk, nab, nb_, nd):
     em("}")
 
 
+def grouped(nab, ncd):
+    """True where the digestion sums the lanes of a quartet before its atomics (group_add)."""
+    return nab * ncd <= GROUP_MAX
+
+
 def emit_digest(em, spin, blk, nab, na, nb_, nd, ncd_all, ablk=None):
     """Digest the contracted block o<ab>_<cd> (cd in blk, ab in ablk -- all bra functions by
     default) into the J/K accumulators.  Expects PA, PB (unrestricted), PT, N, bp, kp, deg and
@@ -736,7 +741,7 @@ def emit_digest(em, spin, blk, nab, na, nb_, nd, ncd_all, ablk=None):
     # small blocks, whose long contractions are split over many lanes, sum those lanes' values before
     # the atomic; larger blocks have too many targets: the inlined sums grow the code past what the
     # instruction cache holds (every class with them: benzene/6-31G* 0.68 -> 0.75 ms per build)
-    group = nab * ncd_all <= GROUP_MAX
+    group = grouped(nab, ncd_all)
     add = lambda p, v: em("sqb::group_add(%s, %s, isplit, gmask, grp == 0);" % (p, v) if group else "atomicAdd(%s, %s);" % (p, v))
     cset = sorted({cd // nd for cd in blk})
     dset = sorted({cd % nd for cd in blk})
@@ -884,7 +889,7 @@ def main():
                 sr["flops"]["quartet"]))
         else:
             reg.append('   0, nullptr, nullptr, 0, 0, 0,')
-        reg.append('   %d},' % default_form(r["bra"], r["ket"], bool(wr), bool(sr)))
+        reg.append('   %d, %d},' % (default_form(r["bra"], r["ket"], bool(wr), bool(sr)), grouped(r["nab"], r["ncd"])))
     reg.append("};")
     reg.append("const int kNumClassKernels = %d;" % (len(metas) // 2))
     reg.append("}  // namespace sqb")

@@ -1117,7 +1117,7 @@ double step_ops(const sqb::ClassKernel& K) { return 150.0 + (double)K.flops_prim
 // when 32 do not reach that, the split with the shortest loop).  Every thread digests its own
 // partial block, so a split costs a digestion per thread; among splits of one size the one over
 // the bra primitives comes first (a thread flushes once per bra primitive).  pow2: aligned lanes
-// (classes of at most 16 function quartets, whose lanes' sums meet in shuffles before the atomics).
+// (classes whose lanes' sums meet in shuffles before the atomics).
 int pick_split(int nbp, int nkp, double steps, bool pow2) {
   int best = 1 | 1 << 16;
   long best_loop = (long)nbp * nkp, best_n = 1;
@@ -1214,7 +1214,7 @@ void class_items(const sqb200_jk* c, int ki, double outer, double fixed, int bra
     for (size_t sy = same ? sx : 0; sy + 1 < T.sub.size(); ++sy) {
       const int nbp = B.pairs[B.sub[sx]].nprim, nkp = T.pairs[T.sub[sy]].nprim;
       // multipole mode needs each quartet's whole block in one thread
-      const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K), K.nab * K.ncd <= 16);
+      const int split = mpm ? (1 | 1 << 16) : pick_split(nbp, nkp, chain / step_ops(K), K.grouped != 0);
       const int si = split & 0xffff, sj = split >> 16;
       runs.push_back({(long)((nbp + si - 1) / si) * ((nkp + sj - 1) / sj), sx, sy, split});
     }

@@ -41,6 +41,8 @@ struct ClassKernel {
   const void* fn_us;
   int s_flops_prim, s_flops_flush, s_flops_quartet;
   int dflt;               // FP64 form without autotuning: 0 narrow, 1 wide, 2 swapped
+  int grouped;            // the digestion sums a quartet's lanes in shuffles (group_add): a quartet's
+                          // threads must be a power of two
 };
 
 extern const ClassKernel kClassKernels[];
