@@ -169,9 +169,9 @@ struct BoysTables {
   std::vector<double> plain, rows;
   std::vector<float> rowsf;
   BoysTables() : plain(sqb::boys_table(BOYS_NCOL)) {
-    rows.assign((size_t)(BOYS_MMAX + 2) * BOYS_NGRID * BOYS_ROW, 0.0);   // one order more: the gradient
+    rows.assign((size_t)BOYS_MROWS * BOYS_NGRID * BOYS_ROW, 0.0);
     rowsf.assign((size_t)(BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF, 0.0f);
-    for (int M = 0; M <= BOYS_MMAX + 1; ++M)
+    for (int M = 0; M < BOYS_MROWS; ++M)
       for (int g = 0; g < BOYS_NGRID; ++g) {
         const size_t r = (size_t)M * BOYS_NGRID + g;
         double f = 1.0;
@@ -199,7 +199,7 @@ const BoysTables& boys_tables() {
 // cudaDeviceReset of the host program takes them, and every stream, event and function attribute,
 // with the CUDA context: g_boys_ready lies beside the tables, so it goes with them.
 constexpr int kBoysPlain = BOYS_NGRID * BOYS_NCOL;
-constexpr int kBoysRows = (BOYS_MMAX + 2) * BOYS_NGRID * BOYS_ROW;
+constexpr int kBoysRows = BOYS_MROWS * BOYS_NGRID * BOYS_ROW;
 constexpr int kBoysRowsF = (BOYS_MMAX + 1) * BOYS_NGRID * BOYS_ROWF;
 __device__ __align__(128) double g_boys_plain[kBoysPlain];
 __device__ __align__(128) double g_boys_rows[kBoysRows];
