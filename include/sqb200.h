@@ -119,8 +119,8 @@ int sqb200_jk_profile_read(sqb200_jk *ctx, double *rows, int max_rows, int *nrow
 const char *sqb200_jk_class_name(int k);
 
 /* Mixed precision: shell quartets whose Schwarz product Sch(PQ)*Sch(IJ) is below fp32_below
- * evaluate their Hermite integrals and contractions in FP32 (setup, Boys function, screening
- * and every J/K accumulation stay FP64); quartets above it, and the classes of highest angular
+ * are evaluated in FP32 up to their contracted integrals (screening and every J/K accumulation
+ * stay FP64); quartets above it, and the classes of highest angular
  * momentum (total L >= 7), stay FP64.  0 (the default) = plain FP64.  Applies to the
  * following builds of the context (not to sqb200_jk_build_noalloc).  No reference
  * counterpart: the reference computes every quartet in FP64. */

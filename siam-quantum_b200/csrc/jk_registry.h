@@ -18,7 +18,7 @@ struct ClassKernel {
   int flops_prim;         // FP64 ops per primitive quartet as emitted (all passes, repeats included)
   int flops_flush;        // FP64 ops per bra primitive and ket pair (all passes)
   int flops_quartet;      // FP64 ops of one digestion (all passes) of a (partial) quartet block
-  // mixed form (FP32 Hermite integrals and contraction, FP64 Boys/setup/accumulation); null
+  // mixed form (FP32 up to the contracted block, FP64 J/K accumulation); null
   // for the classes of highest angular momentum, whose small quartets stay in FP64
   int passes32;
   const void* fn_r32;

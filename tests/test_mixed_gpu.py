@@ -1,5 +1,5 @@
 """Mixed precision: quartets whose Schwarz bound is below tau use the FP32 kernel form (FP64
-Boys function, screening and accumulation).  Errors are stated against the plain-FP64 build
+screening and accumulation).  Errors are stated against the plain-FP64 build
 and, through the relinked reference program (which builds with difference densities each
 SCF iteration), against the reference's FP64 SCF energy: the bar is 1e-6 Eh."""
 import json
