@@ -25,7 +25,6 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <set>
 #include <tuple>
 #include <string>
 #include <vector>

@@ -716,7 +716,8 @@ void gen_items(const GenPath& g, double outer, double fixed, std::vector<GenItem
   }
   // The runs of a class by (contraction length of the bra, ket group), heaviest primitive loops and
   // largest kets first: what the order goes by is one value per such pair.  (A record per unit, sorted
-  // one by one, took 1.3 s and 155 MB for benzene/QZP's 7.7 million units.)
+  // one by one, took 1.3 s and 155 MB for benzene/QZP's 7.7 million units; its 72,606 runs take 4 ms and
+  // 2 MB.)
   std::vector<std::pair<int, int>> chunks;
   for (int q = 0; q < 5; ++q) {
     struct Block { long long key; const std::vector<Bra>* bras; size_t group; int si, sj; };
